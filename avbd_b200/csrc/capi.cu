@@ -10,6 +10,7 @@
 //   * one CUDA graph holds a whole fixed-iteration step.
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -449,6 +450,134 @@ void build_neighbors(avbd_ctx* c, const std::vector<unsigned>& inc_off, const st
     }
 }
 
+// Runs work(first, last) over [0, n) on the host's threads.
+template <typename F>
+void parallel_vertices(unsigned n, F work) {
+    const unsigned nt = n < 20000 ? 1 : std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
+    if (nt == 1) return work(0u, n);
+    std::vector<std::thread> th;
+    for (unsigned t = 0; t < nt; t++)
+        th.emplace_back(work, (unsigned)((uint64_t)n * t / nt), (unsigned)((uint64_t)n * (t + 1) / nt));
+    for (auto& t : th) t.join();
+}
+
+// The four rows of D = [Q; -1^T Q] of a tet.
+void tet_rows(const HostNH& h, double D[4][3]) {
+    for (int j = 0; j < 3; j++) {
+        D[0][j] = h.Q[j];
+        D[1][j] = h.Q[3 + j];
+        D[2][j] = h.Q[6 + j];
+        D[3][j] = -(h.Q[j] + h.Q[3 + j] + h.Q[6 + j]);
+    }
+}
+
+// Star form of every solved vertex (engine.h, StarNb), in internal order.
+template <typename RS>
+struct HostStar {
+    std::vector<uint2> off;
+    std::vector<StarNb<RS>> nb;
+    std::vector<StarTet<RS>> tet;
+    std::vector<uint32_t> loc;
+    std::vector<RS> hd;
+    std::vector<float> mol;
+    unsigned max_nb = 0;
+};
+
+// False when the context needs the records: a vertex with more than
+// STAR_MAX_NB neighbours, or element constants outside RS's comfortable range
+// (rest volumes far from any mesh's, or values that are not finite).
+template <typename RS>
+bool build_star(const avbd_ctx* c, const std::vector<uint32_t>& begin, const std::vector<unsigned>& inc_off,
+                const std::vector<uint32_t>& inc_tet, const std::vector<uint16_t>& inc_local, HostStar<RS>& S) {
+    const unsigned n = (unsigned)c->mass.size();
+    S.off.assign(n + 1, make_uint2(0, 0));
+    std::atomic<bool> ok{true};
+    // neighbours of vertex i (external ids, ascending) into v
+    auto neighbours = [&](unsigned i, std::vector<unsigned>& v) {
+        const unsigned e = c->perm[i];
+        v.clear();
+        for (unsigned k = inc_off[e]; k < inc_off[e + 1]; k++)
+            for (unsigned j = 0; j < 4; j++)
+                if (j != inc_local[k]) v.push_back(c->nh[inc_tet[k]].idx[j]);
+        std::sort(v.begin(), v.end());
+        v.erase(std::unique(v.begin(), v.end()), v.end());
+    };
+    parallel_vertices(n, [&](unsigned b, unsigned en) {
+        std::vector<unsigned> v;
+        for (unsigned i = b; i < en; i++) {
+            if (begin[i + 1] == begin[i]) continue;
+            neighbours(i, v);
+            if (v.size() > STAR_MAX_NB) ok = false;
+            S.off[i + 1].x = (unsigned)v.size();
+        }
+    });
+    if (!ok) return false;
+    for (unsigned i = 0; i < n; i++) {
+        S.max_nb = std::max(S.max_nb, S.off[i + 1].x);
+        S.off[i + 1].x += S.off[i].x;
+        S.off[i + 1].y = begin[i + 1];
+    }
+    S.nb.resize(S.off[n].x);
+    S.tet.resize(begin[n]);
+    S.loc.resize(begin[n]);
+    S.hd.assign(n, RS(0));
+    S.mol.assign(n, 0.f);
+    const bool single = sizeof(RS) == 4;
+    const double lo = single ? 1e-30 : 1e-280, hi = single ? 1e30 : 1e280;
+    auto fits = [&](double x) { return x == 0 || (std::fabs(x) >= lo && std::fabs(x) <= hi); };
+    auto bounded = [&](double x) { return std::fabs(x) <= hi; };
+    parallel_vertices(n, [&](unsigned b, unsigned en) {
+        std::vector<unsigned> v;
+        std::vector<double> w;
+        for (unsigned i = b; i < en; i++) {
+            if (begin[i + 1] == begin[i]) continue;
+            neighbours(i, v);
+            w.assign(v.size(), 0.0);
+            const unsigned e = c->perm[i];
+            double hd = 0, mol = 0;
+            size_t t = begin[i];
+            for (unsigned k = inc_off[e]; k < inc_off[e + 1]; k++, t++) {
+                const HostNH& h = c->nh[inc_tet[k]];
+                const unsigned me = inc_local[k];
+                double D[4][3];
+                tet_rows(h, D);
+                const double* d[3];
+                unsigned slot[3], o = 0;
+                for (unsigned j = 0; j < 4; j++) {
+                    if (j == me) continue;
+                    d[o] = D[j];
+                    slot[o] = (unsigned)(std::lower_bound(v.begin(), v.end(), h.idx[j]) - v.begin());
+                    w[slot[o]] += h.V * h.mu * (D[me][0] * D[j][0] + D[me][1] * D[j][1] + D[me][2] * D[j][2]);
+                    o++;
+                }
+                hd += h.V * h.mu * (D[me][0] * D[me][0] + D[me][1] * D[me][1] + D[me][2] * D[me][2]);
+                mol += h.mu / h.lambda;
+                // |det D| from the tet's own rows 0..2, the same number for its
+                // four vertices; only the sign depends on which row is left out
+                const double* q = h.Q;
+                const double det = q[0] * (q[4] * q[8] - q[5] * q[7]) - q[1] * (q[3] * q[8] - q[5] * q[6]) +
+                                   q[2] * (q[3] * q[7] - q[4] * q[6]);
+                const double s = (me & 1u) ? det : -det;
+                const double a = h.V * h.lambda * s * s, r = s != 0 ? (1 + h.mu / h.lambda) / s : 0.0;
+                if (!fits(a) || !fits(r)) ok = false;
+                S.tet[t] = StarTet<RS>{(RS)a, (RS)r};
+                S.loc[t] = slot[0] | slot[1] << 8 | slot[2] << 16;
+            }
+            for (size_t j = 0; j < v.size(); j++) {
+                if (!bounded(w[j])) ok = false;
+                StarNb<RS>& q = S.nb[S.off[i].x + j];
+                q = StarNb<RS>{};
+                q.idx = c->inv[v[j]];
+                q.w = (RS)w[j];
+            }
+            if (!bounded(hd)) ok = false;
+            S.hd[i] = (RS)hd;
+            S.mol[i] = (float)mol;
+        }
+    });
+    return ok;
+}
+
 template <typename R, typename RS>
 int upload_state(avbd_ctx* c, DevState<R>& s, const std::vector<unsigned>& inc_off,
                  const std::vector<uint32_t>& inc_tet, const std::vector<uint16_t>& inc_local,
@@ -471,7 +600,7 @@ int upload_state(avbd_ctx* c, DevState<R>& s, const std::vector<unsigned>& inc_o
         if (ground_of[e] >= 0) f |= VF_GROUND;
         flags[i] = f;
     }
-    // incidence records in internal order; only solved positional vertices get records
+    // element data in internal order; only solved positional vertices have any
     std::vector<uint32_t> begin(n + 1, 0);
     for (unsigned i = 0; i < n; i++) {
         unsigned e = c->perm[i];
@@ -479,11 +608,13 @@ int upload_state(avbd_ctx* c, DevState<R>& s, const std::vector<unsigned>& inc_o
         begin[i + 1] = begin[i] + (solved ? inc_off[e + 1] - inc_off[e] : 0);
     }
     const size_t nrec = begin[n];
+    HostStar<RS> star;
+    const bool use_star = !c->damping && build_star<RS>(c, begin, inc_off, inc_tet, inc_local, star);
     // algorithmic bytes of each color's solve launch, and of each scene's
     // part of it (the pieces a run-to-tolerance sweep launches per scene)
     c->color_bytes.assign(c->num_colors, 0.0);
     {
-        const double V4B = sizeof(V4), RECB = sizeof(IncRec<RS>);
+        const double V4B = sizeof(V4);
         const double ground_b = c->ground.empty() ? 0.0 : 3 * V4B + 1;
         std::vector<unsigned> sb = c->scene_begin;
         if (sb.back() != n) sb.push_back(n);
@@ -492,7 +623,13 @@ int upload_state(avbd_ctx* c, DevState<R>& s, const std::vector<unsigned>& inc_o
         for (unsigned col = 0; col < c->num_colors; col++) {
             double b = 0;
             for (unsigned i = c->color_begin[col]; i < c->color_begin[col] + c->color_solve[col]; i++) {
-                double bi = 3 * V4B + 2 * sizeof(uint32_t) + 1 + RECB * (begin[i + 1] - begin[i]);
+                const unsigned nt = begin[i + 1] - begin[i];
+                double bi = 3 * V4B + 2 * sizeof(uint32_t) + 1;
+                if (use_star)
+                    bi += 2 * sizeof(uint32_t) + sizeof(RS) + sizeof(StarNb<RS>) * (star.off[i + 1].x - star.off[i].x) +
+                          (sizeof(StarTet<RS>) + sizeof(uint32_t)) * nt;
+                else
+                    bi += sizeof(IncRec<RS>) * nt;
                 if (flags[i] & VF_GROUND) bi += ground_b;
                 b += bi;
                 const unsigned sc = (unsigned)(std::upper_bound(sb.begin(), sb.end(), c->perm[i]) - sb.begin()) - 1;
@@ -501,12 +638,9 @@ int upload_state(avbd_ctx* c, DevState<R>& s, const std::vector<unsigned>& inc_o
             c->color_bytes[col] = b;
         }
     }
-    std::vector<IncRec<RS>> rec(nrec);
-    {
-        unsigned nt = std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
-        if (n < 20000) nt = 1;
-        auto work = [&](unsigned t) {
-            unsigned b = (unsigned)((uint64_t)n * t / nt), en = (unsigned)((uint64_t)n * (t + 1) / nt);
+    std::vector<IncRec<RS>> rec(use_star ? 0 : nrec);
+    if (!use_star)
+        parallel_vertices(n, [&](unsigned b, unsigned en) {
             for (unsigned i = b; i < en; i++) {
                 unsigned e = c->perm[i];
                 if (begin[i + 1] == begin[i]) continue;
@@ -515,12 +649,7 @@ int upload_state(avbd_ctx* c, DevState<R>& s, const std::vector<unsigned>& inc_o
                     const HostNH& h = c->nh[inc_tet[k]];
                     unsigned loc = inc_local[k];
                     double D[4][3];
-                    for (int j = 0; j < 3; j++) {
-                        D[0][j] = h.Q[0 * 3 + j];
-                        D[1][j] = h.Q[1 * 3 + j];
-                        D[2][j] = h.Q[2 * 3 + j];
-                        D[3][j] = -(h.Q[j] + h.Q[3 + j] + h.Q[6 + j]);
-                    }
+                    tet_rows(h, D);
                     IncRec<RS>& r = rec[w];
                     int o = 0;
                     for (int j = 0; j < 4; j++) {
@@ -537,24 +666,33 @@ int upload_state(avbd_ctx* c, DevState<R>& s, const std::vector<unsigned>& inc_o
                     r.mol = (RS)(h.mu / h.lambda);
                 }
             }
-        };
-        if (nt == 1) work(0);
-        else {
-            std::vector<std::thread> th;
-            for (unsigned t = 0; t < nt; t++) th.emplace_back(work, t);
-            for (auto& t : th) t.join();
-        }
-    }
+        });
     int rc;
     if ((rc = dalloc(c, &s.x, n)) || (rc = dalloc(c, &s.y, n)) || (rc = dalloc(c, &s.xp, n)) ||
         (rc = dalloc(c, &s.xl, n)) || (rc = dalloc(c, &s.xll, n)) || (rc = dalloc(c, &s.v, n)) ||
-        (rc = dalloc(c, &s.vp, n)) || (rc = dalloc(c, &s.flags, n)) || (rc = dalloc(c, &s.inc_begin, n + 1)))
+        (rc = dalloc(c, &s.vp, n)) || (rc = dalloc(c, &s.flags, n)))
         return rc;
-    IncRec<RS>* d_rec = nullptr;
-    if ((rc = dalloc(c, &d_rec, nrec))) return rc;
-    if constexpr (std::is_same<R, RS>::value) s.inc = d_rec;
-    else s.inc32 = d_rec;
     cudaStream_t st = c->stream;
+    TetElems<RS> el;
+    auto put = [&](auto** d, const auto& h) -> int {  // device copy of a host vector
+        using T = std::remove_const_t<std::remove_pointer_t<std::remove_pointer_t<decltype(d)>>>;
+        T* p = nullptr;
+        if (int r = dalloc(c, &p, h.size())) return r;
+        *d = p;
+        if (!h.empty()) CUDA_OR_FAIL(cudaMemcpyAsync(p, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice, st));
+        return AVBD_OK;
+    };
+    if (use_star) {
+        if ((rc = put(&el.star, star.off)) || (rc = put(&el.nb, star.nb)) || (rc = put(&el.tet, star.tet)) ||
+            (rc = put(&el.loc, star.loc)) || (rc = put(&el.hd, star.hd)) || (rc = put(&el.mol, star.mol)))
+            return rc;
+        el.max_nb = star.max_nb;
+    } else if ((rc = put(&el.inc, rec)) || (rc = put(&el.inc_begin, begin))) {
+        return rc;
+    }
+    if constexpr (std::is_same<R, RS>::value) s.el = el;
+    else s.el32 = el;
+    c->star_nb = el.max_nb;
     CUDA_OR_FAIL(cudaMemcpyAsync(s.x, x.data(), sizeof(V4) * n, cudaMemcpyHostToDevice, st));
     CUDA_OR_FAIL(cudaMemcpyAsync(s.y, y.data(), sizeof(V4) * n, cudaMemcpyHostToDevice, st));
     CUDA_OR_FAIL(cudaMemcpyAsync(s.xp, x.data(), sizeof(V4) * n, cudaMemcpyHostToDevice, st));
@@ -563,8 +701,6 @@ int upload_state(avbd_ctx* c, DevState<R>& s, const std::vector<unsigned>& inc_o
     CUDA_OR_FAIL(cudaMemcpyAsync(s.v, v.data(), sizeof(V4) * n, cudaMemcpyHostToDevice, st));
     CUDA_OR_FAIL(cudaMemcpyAsync(s.vp, vp.data(), sizeof(V4) * n, cudaMemcpyHostToDevice, st));
     CUDA_OR_FAIL(cudaMemcpyAsync(s.flags, flags.data(), n, cudaMemcpyHostToDevice, st));
-    if (nrec) CUDA_OR_FAIL(cudaMemcpyAsync(d_rec, rec.data(), sizeof(IncRec<RS>) * nrec, cudaMemcpyHostToDevice, st));
-    CUDA_OR_FAIL(cudaMemcpyAsync(s.inc_begin, begin.data(), sizeof(uint32_t) * (n + 1), cudaMemcpyHostToDevice, st));
 
     // ground contact, one record per particle (internal order)
     if (!c->ground.empty()) {
@@ -1162,7 +1298,8 @@ int autotune_impl(avbd_ctx* c, DevState<R>& s) {
     const char* env = getenv("AVBD_LANES");
     if (env) {
         int l = atoi(env);
-        if (l == 1 || l == 2 || l == 4 || l == 8 || l == 16 || l == 32) c->lanes = l;
+        if (l == 1 || l == 2 || l == 4 || l == 8 || l == 16 || l == 32) c->lanes = std::min(std::max(l, 2), 16);
+        if (!c->star_nb && c->lanes != 2) c->lanes = 8;
         return AVBD_OK;
     }
     unsigned long long solved = 0;
@@ -1181,7 +1318,8 @@ int autotune_impl(avbd_ctx* c, DevState<R>& s) {
     const unsigned long long launches0 = c->stats.kernel_launches;
     int best = 8;
     float best_ms = 1e30f;
-    for (int l : {1, 2, 4, 8, 16}) {
+    for (int l : {2, 4, 8, 16}) {
+        if (!c->star_nb && l != 2 && l != 8) continue;
         c->lanes = l;
         for (int rep = 0; rep < 2; rep++) {  // rep 0 warms up, rep 1 is timed
             if (rep == 1) CUDA_OR_FAIL(cudaEventRecord(a, st));

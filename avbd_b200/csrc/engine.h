@@ -38,6 +38,42 @@ template <> struct alignas(16) IncRec<double> {
 static_assert(sizeof(IncRec<float>) == 64, "FP32 incidence record must be 64 B");
 static_assert(sizeof(IncRec<double>) == 112, "FP64 incidence record must be 112 B");
 
+// The undamped incidence restated about the solved vertex i (star form).  With
+// e_k = x_k - x_i the edges to the three other vertices of a tet, F = E D for
+// the matrix D of the rows d_k, so det F = s e_1.N with s = det D and
+// N = (e_2 - e_1) x (e_3 - e_1), cof(F) d_i = -s N, and F d_i is a combination
+// of the edges with constant weights.  The block of the vertex is then
+//   gradient  sum_k W_k e_k - sum_t a (e_1.N - r) N
+//   Hessian   hd I + sum_t a N N^T
+// with a = V lambda s^2, r = (1 + mu/lambda)/s per tet, W_k = sum V mu d_i.d_k
+// per distinct neighbour and hd = sum V mu |d_i|^2 per vertex: 12 bytes a tet
+// and 8 a neighbour instead of 64 a tet (FP32 records), and a quarter of the
+// arithmetic of forming F.  W and a, r are the same numbers in the lists of
+// all four vertices of a tet, so the element forces balance exactly.
+template <typename R> struct StarNb;
+template <> struct alignas(8) StarNb<float> { uint32_t idx; float w; };
+template <> struct alignas(16) StarNb<double> { uint32_t idx, pad; double w; };
+template <typename R> struct alignas(2 * sizeof(R)) StarTet { R a, r; };
+// distinct neighbours a vertex may have for its context to take the star form
+// (their edges are staged in shared memory); beyond it, and with damping,
+// which needs F itself, the records serve
+constexpr unsigned STAR_MAX_NB = 64;
+
+// Element data of the tet solve in record precision RS: the star form when
+// `star` is set, else the records.
+template <typename RS>
+struct TetElems {
+    const IncRec<RS>* inc = nullptr;
+    const uint32_t* inc_begin = nullptr;
+    const uint2* star = nullptr;          // n + 1: first neighbour, first tet of each vertex
+    const StarNb<RS>* nb = nullptr;
+    const StarTet<RS>* tet = nullptr;
+    const uint32_t* loc = nullptr;        // the tet's three others as positions in the neighbour list, 8 bits each
+    const RS* hd = nullptr;               // per vertex
+    const float* mol = nullptr;           // per vertex: sum of mu/lambda over its tets (warm-start feature)
+    unsigned max_nb = 0;                  // largest neighbour count of the context
+};
+
 enum VertexFlags : uint8_t { VF_FIXED = 1, VF_ORIENTED = 2, VF_GROUND = 4 };
 enum GroundFlags : uint8_t { GF_USE_STATIC = 1, GF_UNCLAMPED = 2 };
 
@@ -71,9 +107,8 @@ struct DevState {
     // before iteration 0.
     V4 *x = nullptr, *y = nullptr, *xp = nullptr, *xl = nullptr, *xll = nullptr, *v = nullptr, *vp = nullptr;
     uint8_t* flags = nullptr;
-    IncRec<R>* inc = nullptr;
-    IncRec<float>* inc32 = nullptr;   // FP32 records of the mixed mode (double state)
-    uint32_t* inc_begin = nullptr;
+    TetElems<R> el;
+    TetElems<float> el32;             // FP32 element data of the mixed mode (double state)
     // per-tet data (damping path only)
     unsigned ntets = 0;
     uint4* tet_idx = nullptr;
@@ -304,6 +339,7 @@ struct avbd_ctx {
     bool graph_tol = false;
     bool use_graph = true;
     int lanes = 8;                      // threads per vertex in the tet solve
+    unsigned star_nb = 0;               // largest neighbour count of the star form, 0: records
     int block = 256;
 
     // learned warm start (mlp.cu): 0 off, 1 record features/targets, 2 apply

@@ -252,6 +252,111 @@ AVBD_D void accumulate_tet(const DevState<P>& s, const IncRec<RS>& r, V3<P> xi, 
     accumulate_tet_e<P, RS, HT, DAMP>(s, r, r.tet, e1, e2, e3, dt, B);
 }
 
+// Loads of the star form: read once per launch, so kept out of L1, where the
+// neighbour gathers live.
+AVBD_D uint2 ld_once(const uint2* p) {
+    uint2 v;
+    asm("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+AVBD_D uint32_t ld_once(const uint32_t* p) {
+    uint32_t v;
+    asm("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+AVBD_D StarNb<float> ld_once(const StarNb<float>* p) {
+    const uint2 v = ld_once(reinterpret_cast<const uint2*>(p));
+    return {v.x, __uint_as_float(v.y)};
+}
+AVBD_D StarTet<float> ld_once(const StarTet<float>* p) {
+    const uint2 v = ld_once(reinterpret_cast<const uint2*>(p));
+    return {__uint_as_float(v.x), __uint_as_float(v.y)};
+}
+AVBD_D StarNb<double> ld_once(const StarNb<double>* p) {
+    StarNb<double> v;
+    asm("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(v.idx), "=r"(v.pad) : "l"(p));
+    asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v.w) : "l"(&p->w));
+    return v;
+}
+AVBD_D StarTet<double> ld_once(const StarTet<double>* p) {
+    StarTet<double> v;
+    asm("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.a), "=d"(v.r) : "l"(p));
+    return v;
+}
+
+// Shared-memory staging of the neighbour edges: component c of edge j of the
+// block's vertex slot g lies at [(c max_nb + j) stride + g].  Lanes of one
+// vertex read different j and neighbouring vertices mostly the same j, so the
+// stride is skewed by a half-warp's (FP64) or a warp's (FP32) width over
+// LANES to spread both over the banks.
+template <typename P, int LANES>
+struct StarStage {
+    static constexpr unsigned GROUPS = 256 / LANES;
+    static constexpr unsigned STRIDE = GROUPS + (sizeof(P) == 8 ? 16 : 32) / LANES;
+    static unsigned bytes(unsigned max_nb) { return 3 * max_nb * STRIDE * (unsigned)sizeof(P); }
+};
+
+// The block of a vertex from its star form (StarNb): the edges to the distinct
+// neighbours are gathered once (14 instead of 61 positions on the split hex
+// grids) and staged in shared memory, the deviatoric part summed over them;
+// then each tet takes its three edges from there.  es: this vertex's slot.
+template <typename P, typename RS, typename HT, int LANES, bool COH>
+AVBD_D void accumulate_star(const DevState<P>& s, const TetElems<RS>& el, uint2 o0, uint2 o1, unsigned lane, V3<P> xi,
+                            P* es, Block3<P, HT>& B) {
+    constexpr unsigned ST = StarStage<P, LANES>::STRIDE;
+    constexpr unsigned U = LANES <= 2 ? 4 : 2;  // neighbour gathers in flight per lane
+    const unsigned K = el.max_nb;
+    for (unsigned j = o0.x + lane; j < o1.x; j += U * LANES) {
+        StarNb<RS> q[U];
+        V3<P> e[U];
+#pragma unroll
+        for (unsigned u = 0; u < U; u++)
+            if (j + u * LANES < o1.x) q[u] = ld_once(el.nb + j + u * LANES);
+#pragma unroll
+        for (unsigned u = 0; u < U; u++)
+            if (j + u * LANES < o1.x) e[u] = xyz(COH ? s.x[q[u].idx] : ld_ro(s.x + q[u].idx));
+#pragma unroll
+        for (unsigned u = 0; u < U; u++)
+            if (j + u * LANES < o1.x) {
+                e[u] = e[u] - xi;
+                P* d = es + (j + u * LANES - o0.x) * ST;
+                d[0] = e[u].x;
+                d[K * ST] = e[u].y;
+                d[2 * K * ST] = e[u].z;
+                const P w = (P)q[u].w;
+                B.g0 += w * e[u].x;
+                B.g1 += w * e[u].y;
+                B.g2 += w * e[u].z;
+            }
+    }
+    __syncwarp();
+#pragma unroll 2
+    for (unsigned t = o0.y + lane; t < o1.y; t += LANES) {
+        const StarTet<RS> q = ld_once(el.tet + t);
+        const uint32_t l = ld_once(el.loc + t);
+        const P* p1 = es + (l & 255u) * ST;
+        const P* p2 = es + (l >> 8 & 255u) * ST;
+        const P* p3 = es + (l >> 16) * ST;
+        const V3<P> e1 = mk3(p1[0], p1[K * ST], p1[2 * K * ST]);
+        const V3<P> f2 = mk3(p2[0], p2[K * ST], p2[2 * K * ST]) - e1;
+        const V3<P> f3 = mk3(p3[0], p3[K * ST], p3[2 * K * ST]) - e1;
+        const V3<P> N = cross3(f2, f3);
+        const P h = (P)q.a * ((P)q.r - dot3(e1, N));
+        B.g0 += h * N.x;
+        B.g1 += h * N.y;
+        B.g2 += h * N.z;
+        const HT nx = (HT)N.x, ny = (HT)N.y, nz = (HT)N.z, a = (HT)q.a;
+        const HT ax = a * nx, ay = a * ny, az = a * nz;
+        B.h00 += ax * nx;
+        B.h11 += ay * ny;
+        B.h22 += az * nz;
+        B.h01 += ax * ny;
+        B.h02 += ax * nz;
+        B.h12 += ay * nz;
+    }
+    __syncwarp();  // the slot is refilled for the lane group's next vertex
+}
+
 // Ground contact term of the block (CollisionConstraintEnergySolver::accumulate<3>
 // with GroundCollisionConstraintSolver): the Hessian k grad C grad C^T is always
 // added, the gradient is gated by the clamped multipliers.
@@ -310,16 +415,20 @@ enum { MODE_SOLVE = 0, MODE_RESIDUAL = 1, MODE_DEBUG = 2, MODE_FEATURES = 3 };
 // at 3 blocks (80 registers, ~100 bytes of spill) its vertex solve ran 15 %
 // faster over a whole run-to-tolerance step of the 1024-cube batch.  FP32
 // fits 4 blocks (64 registers) without spills; FP64 keeps the default.
-template <typename P, typename RS>
+template <typename P, typename RS, int FORM>
 struct SolveMinBlocks {
-    static constexpr int value = sizeof(P) == 4 ? 4 : (sizeof(RS) == 4 ? 3 : 1);
+    static constexpr int value = FORM == 0 ? (sizeof(P) == 4 ? 4 : 3) : sizeof(P) == 4 ? 4 : (sizeof(RS) == 4 ? 3 : 1);
 };
 
 // DYN: the instantiation for vertices with dynamic contact energies or a
 // color changed by the recoloring, launched over per-color lists; the slab
 // launches (DYN false) skip those vertices and carry no dynamic code.
-template <typename P, typename RS, typename HT, int LANES, bool DAMP, bool GROUND, int MODE, bool DYN, bool COH = false>
-__device__ __forceinline__ void tet_vertex(const DevState<P>& s, const IncRec<RS>* __restrict__ inc, unsigned begin,
+// FORM: the element data the context holds -- the star form, or the records
+// without or with damping.
+enum ElemForm { FORM_STAR = 0, FORM_REC = 1, FORM_DAMP = 2 };
+
+template <typename P, typename RS, typename HT, int LANES, int FORM, bool GROUND, int MODE, bool DYN, bool COH = false>
+__device__ __forceinline__ void tet_vertex(const DevState<P>& s, const TetElems<RS>& el, unsigned begin,
                                            unsigned count, unsigned gi, unsigned lane, const Consts<P>& c,
                                            unsigned long long* counters, double* out, const SceneTol& T,
                                            const float4* __restrict__ aux, const uint32_t* __restrict__ list,
@@ -338,9 +447,40 @@ __device__ __forceinline__ void tet_vertex(const DevState<P>& s, const IncRec<RS
     V3<P> xi = mk3<P>(0, 0, 0);
     // MODE_FEATURES: sum of the other vertices' velocities and of mu/lambda over the incident tets
     float fv0 = 0.f, fv1 = 0.f, fv2 = 0.f, fmol = 0.f, fcnt = 0.f;
-    if (active) {
+    if constexpr (FORM == FORM_STAR) {
+        extern __shared__ __align__(16) unsigned char stage[];
+        P* es = reinterpret_cast<P*>(stage) + threadIdx.x / LANES;
+        uint2 o0 = make_uint2(0, 0), o1 = o0;
+        if (active) {
+            xi = xyz(s.x[p]);
+            o0 = el.star[p];
+            o1 = el.star[p + 1];
+        }
+        accumulate_star<P, RS, HT, LANES, COH>(s, el, o0, o1, lane, xi, es, B);
+        if (active && lane == 0) {
+            const HT hd = (HT)el.hd[p];
+            B.h00 += hd;
+            B.h11 += hd;
+            B.h22 += hd;
+        }
+        if constexpr (MODE == MODE_FEATURES) {
+            for (unsigned t = o0.y + lane; t < o1.y; t += LANES) {
+                const uint32_t l = el.loc[t];
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    typename Vec4Of<P>::T vo = s.v[el.nb[o0.x + (l >> 8 * j & 255u)].idx];
+                    fv0 += (float)vo.x;
+                    fv1 += (float)vo.y;
+                    fv2 += (float)vo.z;
+                }
+                fcnt += 1.f;
+            }
+            if (active && lane == 0) fmol = el.mol[p];
+        }
+    } else if (active) {
         xi = xyz(s.x[p]);
-        unsigned b = s.inc_begin[p], e = s.inc_begin[p + 1];
+        const IncRec<RS>* __restrict__ inc = el.inc;
+        unsigned b = el.inc_begin[p], e = el.inc_begin[p + 1];
         // the next record is fetched into L1 while this one is processed (a
         // register copy of it, as a software pipeline, spilled: 192 B of
         // spill in the mixed mode at 3 blocks per SM, 3 % slower), and the
@@ -351,7 +491,7 @@ __device__ __forceinline__ void tet_vertex(const DevState<P>& s, const IncRec<RS
             if (kn < e) prefetch_l1(inc + kn);
             IncRec<RS> r = load_rec<RS>(inc + k);
             if (kn + 3 * LANES < e) prefetch_l2(inc + kn + 3 * LANES);
-            accumulate_tet<P, RS, HT, DAMP, COH>(s, r, xi, c.dt, B);
+            accumulate_tet<P, RS, HT, FORM == FORM_DAMP, COH>(s, r, xi, c.dt, B);
             if constexpr (MODE == MODE_FEATURES) {
 #pragma unroll
                 for (int j = 0; j < 3; j++) {
@@ -521,8 +661,8 @@ __device__ __forceinline__ void tet_vertex(const DevState<P>& s, const IncRec<RS
 // One piece (at most 512 consecutive solved vertices of one scene in one
 // color slab) solved by one block; its residual terms are summed over the
 // block.  rg = (first vertex, count, scene).
-template <typename P, typename RS, typename HT, int LANES, bool DAMP, bool GROUND, int MODE, bool DYN, bool COH>
-__device__ __forceinline__ void solve_piece(const DevState<P>& s, const IncRec<RS>* __restrict__ inc, const uint4 rg,
+template <typename P, typename RS, typename HT, int LANES, int FORM, bool GROUND, int MODE, bool DYN, bool COH>
+__device__ __forceinline__ void solve_piece(const DevState<P>& s, const TetElems<RS>& el, const uint4 rg,
                                             const Consts<P>& c, unsigned long long* counters, double* out,
                                             const SceneTol& T, const float4* __restrict__ aux,
                                             const uint32_t* __restrict__ list) {
@@ -535,17 +675,25 @@ __device__ __forceinline__ void solve_piece(const DevState<P>& s, const IncRec<R
     TB.cand = nullptr;
     double acc = 0.0;
     for (unsigned base = 0; base < rg.y; base += blockDim.x / LANES) {
-        // the first records of this thread group's next vertex are fetched
-        // into L2 while this one is solved (its first loads are then not
-        // DRAM misses)
+        // this thread group's next vertex is fetched into L2 while this one is
+        // solved (its first loads are then not DRAM misses): its whole star
+        // form, or the first records
         const unsigned gn = base + blockDim.x / LANES + threadIdx.x / LANES;
         if (gn < rg.y) {
-            const unsigned bn = s.inc_begin[rg.x + gn], en = s.inc_begin[rg.x + gn + 1];
+            if constexpr (FORM == FORM_STAR) {
+                const uint2 a = el.star[rg.x + gn], b = el.star[rg.x + gn + 1];
+                constexpr unsigned SN = 32 / sizeof(StarNb<RS>), ST = 32 / sizeof(StarTet<RS>);
+                for (unsigned j = a.x + SN * lane; j < b.x; j += SN * LANES) prefetch_l2(el.nb + j);
+                for (unsigned j = a.y + ST * lane; j < b.y; j += ST * LANES) prefetch_l2(el.tet + j);
+                for (unsigned j = a.y + 8 * lane; j < b.y; j += 8 * LANES) prefetch_l2(el.loc + j);
+            } else {
+                const unsigned bn = el.inc_begin[rg.x + gn], en = el.inc_begin[rg.x + gn + 1];
 #pragma unroll
-            for (unsigned j = 0; j < 4; j++)
-                if (bn + lane + j * LANES < en) prefetch_l2(inc + bn + lane + j * LANES);
+                for (unsigned j = 0; j < 4; j++)
+                    if (bn + lane + j * LANES < en) prefetch_l2(el.inc + bn + lane + j * LANES);
+            }
         }
-        tet_vertex<P, RS, HT, LANES, DAMP, GROUND, MODE, DYN, COH>(s, inc, rg.x, rg.y, base + threadIdx.x / LANES,
+        tet_vertex<P, RS, HT, LANES, FORM, GROUND, MODE, DYN, COH>(s, el, rg.x, rg.y, base + threadIdx.x / LANES,
                                                                    lane, c, counters, out, TB, aux, list,
                                                                    sum ? &acc : nullptr);
     }
@@ -563,19 +711,19 @@ __device__ __forceinline__ void solve_piece(const DevState<P>& s, const IncRec<R
     }
 }
 
-template <typename P, typename RS, typename HT, int LANES, bool DAMP, bool GROUND, int MODE, bool DYN>
-__global__ void __launch_bounds__(256, SolveMinBlocks<P, RS>::value) k_solve_tet(DevState<P> s, const IncRec<RS>* __restrict__ inc,
+template <typename P, typename RS, typename HT, int LANES, int FORM, bool GROUND, int MODE, bool DYN>
+__global__ void __launch_bounds__(256, (SolveMinBlocks<P, RS, FORM>::value)) k_solve_tet(DevState<P> s, TetElems<RS> el,
                                                    unsigned begin, unsigned count, Consts<P> c,
                                                    unsigned long long* counters, double* out, SceneTol T,
                                                    const float4* __restrict__ aux, const uint32_t* __restrict__ list,
                                                    const uint4* __restrict__ ranges) {
     if (ranges) {
-        solve_piece<P, RS, HT, LANES, DAMP, GROUND, MODE, DYN, false>(s, inc, ranges[blockIdx.x], c, counters, out, T,
+        solve_piece<P, RS, HT, LANES, FORM, GROUND, MODE, DYN, false>(s, el, ranges[blockIdx.x], c, counters, out, T,
                                                                       aux, list);
         return;
     }
     const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x;
-    tet_vertex<P, RS, HT, LANES, DAMP, GROUND, MODE, DYN>(s, inc, begin, count, tid / LANES, tid % LANES, c, counters,
+    tet_vertex<P, RS, HT, LANES, FORM, GROUND, MODE, DYN>(s, el, begin, count, tid / LANES, tid % LANES, c, counters,
                                                           out, T, aux, list);
 }
 
@@ -594,9 +742,9 @@ AVBD_D bool grid_barrier(unsigned* sync, int* err) {
 // block draws exactly one ticket past the color's pieces, so color k's tickets
 // start at sum over earlier colors of (pieces + blocks).  sync: [ticket,
 // arrivals, generation], zeroed before each launch.
-template <typename P, typename RS, typename HT, int LANES, bool GROUND>
-__global__ void __launch_bounds__(256, SolveMinBlocks<P, RS>::value)
-    k_sweep_persistent(DevState<P> s, const IncRec<RS>* __restrict__ inc, Consts<P> c, unsigned long long* counters,
+template <typename P, typename RS, typename HT, int LANES, int FORM, bool GROUND>
+__global__ void __launch_bounds__(256, (SolveMinBlocks<P, RS, FORM>::value))
+    k_sweep_persistent(DevState<P> s, TetElems<RS> el, Consts<P> c, unsigned long long* counters,
                        SceneTol T, const uint4* __restrict__ ranges, const unsigned* __restrict__ color_off,
                        unsigned ncolors, unsigned* sync) {
     __shared__ unsigned ticket;
@@ -609,8 +757,8 @@ __global__ void __launch_bounds__(256, SolveMinBlocks<P, RS>::value)
             __syncthreads();
             const unsigned t = ticket;
             if (t >= np) break;
-            solve_piece<P, RS, HT, LANES, false, GROUND, MODE_SOLVE, false, true>(s, inc, ranges[r0 + t], c,
-                                                                                  counters, nullptr, T, nullptr,
+            solve_piece<P, RS, HT, LANES, FORM, GROUND, MODE_SOLVE, false, true>(s, el, ranges[r0 + t], c,
+                                                                                 counters, nullptr, T, nullptr,
                                                                                   nullptr);
         }
         base += np + gridDim.x;
@@ -753,34 +901,51 @@ void launch_tet_eprev(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaStre
     count_launch(c);
 }
 
+// Dynamic shared memory of a kernel's neighbour staging; above 48 KB the
+// kernel has to opt in.
+template <typename K>
+static bool stage_smem(K kern, unsigned bytes) {
+    return bytes <= 48 * 1024 ||
+           cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+}
+
+template <typename P, typename RS, typename HT, int LANES, int FORM, int MODE, bool DYN>
+static void solve_dispatch_form(avbd_ctx* c, DevState<P>& s, const TetElems<RS>& el, const StepConsts& k,
+                                unsigned begin, unsigned count, cudaStream_t st, double* out, const SceneTol& T,
+                                const uint32_t* list, const uint4* ranges, unsigned nranges) {
+    const unsigned blocks = ranges ? nranges : nblocks(count * LANES, 256);
+    if (blocks == 0) return;
+    const unsigned smem = FORM == FORM_STAR ? StarStage<P, LANES>::bytes(el.max_nb) : 0;
+    auto kern = c->ground.empty() ? k_solve_tet<P, RS, HT, LANES, FORM, false, MODE, DYN>
+                                  : k_solve_tet<P, RS, HT, LANES, FORM, true, MODE, DYN>;
+    // a kernel that cannot have its shared memory fails at the launch, which the step checks
+    stage_smem(kern, smem);
+    kern<<<blocks, 256, smem, st>>>(s, el, begin, count, mkc<P>(k), c->d_counters, out, T,
+                                    reinterpret_cast<const float4*>(c->ws_prev_arg), list, ranges);
+    count_launch(c);
+}
+
 template <typename P, typename RS, typename HT, int LANES, int MODE, bool DYN = false>
-static void solve_dispatch(avbd_ctx* c, DevState<P>& s, const IncRec<RS>* inc, const StepConsts& k, unsigned begin,
+static void solve_dispatch(avbd_ctx* c, DevState<P>& s, const TetElems<RS>& el, const StepConsts& k, unsigned begin,
                            unsigned count, cudaStream_t st, double* out, const SceneTol& T, const uint32_t* list,
                            const uint4* ranges = nullptr, unsigned nranges = 0) {
-    unsigned threads = count * LANES;
-    unsigned blocks = ranges ? nranges : nblocks(threads, 256);
-    if (blocks == 0) return;
-    bool damp = c->damping, ground = !c->ground.empty();
-    auto kc = mkc<P>(k);
-    auto* ctr = c->d_counters;
-    const float4* aux = reinterpret_cast<const float4*>(c->ws_prev_arg);
-    if (damp && ground)
-        k_solve_tet<P, RS, HT, LANES, true, true, MODE, DYN><<<blocks, 256, 0, st>>>(s, inc, begin, count, kc, ctr, out, T, aux, list, ranges);
-    else if (damp)
-        k_solve_tet<P, RS, HT, LANES, true, false, MODE, DYN><<<blocks, 256, 0, st>>>(s, inc, begin, count, kc, ctr, out, T, aux, list, ranges);
-    else if (ground)
-        k_solve_tet<P, RS, HT, LANES, false, true, MODE, DYN><<<blocks, 256, 0, st>>>(s, inc, begin, count, kc, ctr, out, T, aux, list, ranges);
-    else
-        k_solve_tet<P, RS, HT, LANES, false, false, MODE, DYN><<<blocks, 256, 0, st>>>(s, inc, begin, count, kc, ctr, out, T, aux, list, ranges);
-    count_launch(c);
+    if (el.star)
+        solve_dispatch_form<P, RS, HT, LANES, FORM_STAR, MODE, DYN>(c, s, el, k, begin, count, st, out, T, list, ranges, nranges);
+    else if constexpr (LANES == 2 || LANES == 8) {
+        if (c->damping)
+            solve_dispatch_form<P, RS, HT, LANES, FORM_DAMP, MODE, DYN>(c, s, el, k, begin, count, st, out, T, list, ranges, nranges);
+        else
+            solve_dispatch_form<P, RS, HT, LANES, FORM_REC, MODE, DYN>(c, s, el, k, begin, count, st, out, T, list, ranges, nranges);
+    }
 }
 
 // The solve, residual and features passes run with the context's lane count
 // (the residual pass spans every vertex every iteration, so its thread count
 // matters even when few scenes are candidates); the one-vertex debug pass
 // uses 8.
+// Lane counts: 2, 4, 8 and 16 with the star form, 2 and 8 with the records.
 template <typename P, typename RS, typename HT, int MODE>
-static void solve_lanes_t(avbd_ctx* c, DevState<P>& s, const IncRec<RS>* inc, const StepConsts& k, unsigned begin,
+static void solve_lanes_t(avbd_ctx* c, DevState<P>& s, const TetElems<RS>& el, const StepConsts& k, unsigned begin,
                           unsigned count, cudaStream_t st, double* out, const SceneTol& T, const uint32_t* list,
                           const uint4* ranges = nullptr, unsigned nranges = 0) {
     if constexpr (MODE == MODE_RESIDUAL) {  // tolerance residual: the sweeps' per-scene pieces, all colors
@@ -789,35 +954,18 @@ static void solve_lanes_t(avbd_ctx* c, DevState<P>& s, const IncRec<RS>* inc, co
             nranges = c->solve_range_off.back();
         }
     }
-    if constexpr (MODE == MODE_SOLVE || MODE == MODE_RESIDUAL) {
-        if (ranges) {
-            const uint4* rg = ranges;
-            const unsigned nr = nranges;
-            switch (c->lanes) {
-                case 1: solve_dispatch<P, RS, HT, 1, MODE>(c, s, inc, k, 0, 0, st, out, T, nullptr, rg, nr); break;
-                case 2: solve_dispatch<P, RS, HT, 2, MODE>(c, s, inc, k, 0, 0, st, out, T, nullptr, rg, nr); break;
-                case 4: solve_dispatch<P, RS, HT, 4, MODE>(c, s, inc, k, 0, 0, st, out, T, nullptr, rg, nr); break;
-                case 16: solve_dispatch<P, RS, HT, 16, MODE>(c, s, inc, k, 0, 0, st, out, T, nullptr, rg, nr); break;
-                case 32: solve_dispatch<P, RS, HT, 32, MODE>(c, s, inc, k, 0, 0, st, out, T, nullptr, rg, nr); break;
-                default: solve_dispatch<P, RS, HT, 8, MODE>(c, s, inc, k, 0, 0, st, out, T, nullptr, rg, nr); break;
-            }
-            return;
-        }
-    }
     if constexpr (MODE == MODE_DEBUG) {
-        if (c->dyn) solve_dispatch<P, RS, HT, 8, MODE, true>(c, s, inc, k, begin, count, st, out, T, list);
-        else solve_dispatch<P, RS, HT, 8, MODE>(c, s, inc, k, begin, count, st, out, T, list);
+        if (c->dyn) solve_dispatch<P, RS, HT, 8, MODE, true>(c, s, el, k, begin, count, st, out, T, list);
+        else solve_dispatch<P, RS, HT, 8, MODE>(c, s, el, k, begin, count, st, out, T, list);
     } else if (list) {
         if constexpr (MODE == MODE_SOLVE || MODE == MODE_RESIDUAL)
-            solve_dispatch<P, RS, HT, 8, MODE, true>(c, s, inc, k, begin, count, st, out, T, list);
+            solve_dispatch<P, RS, HT, 8, MODE, true>(c, s, el, k, begin, count, st, out, T, list);
     } else {
         switch (c->lanes) {
-            case 1: solve_dispatch<P, RS, HT, 1, MODE>(c, s, inc, k, begin, count, st, out, T, list); break;
-            case 2: solve_dispatch<P, RS, HT, 2, MODE>(c, s, inc, k, begin, count, st, out, T, list); break;
-            case 4: solve_dispatch<P, RS, HT, 4, MODE>(c, s, inc, k, begin, count, st, out, T, list); break;
-            case 16: solve_dispatch<P, RS, HT, 16, MODE>(c, s, inc, k, begin, count, st, out, T, list); break;
-            case 32: solve_dispatch<P, RS, HT, 32, MODE>(c, s, inc, k, begin, count, st, out, T, list); break;
-            default: solve_dispatch<P, RS, HT, 8, MODE>(c, s, inc, k, begin, count, st, out, T, list); break;
+            case 2: solve_dispatch<P, RS, HT, 2, MODE>(c, s, el, k, begin, count, st, out, T, list, ranges, nranges); break;
+            case 4: solve_dispatch<P, RS, HT, 4, MODE>(c, s, el, k, begin, count, st, out, T, list, ranges, nranges); break;
+            case 16: solve_dispatch<P, RS, HT, 16, MODE>(c, s, el, k, begin, count, st, out, T, list, ranges, nranges); break;
+            default: solve_dispatch<P, RS, HT, 8, MODE>(c, s, el, k, begin, count, st, out, T, list, ranges, nranges); break;
         }
     }
 }
@@ -828,16 +976,16 @@ template <int MODE>
 static void solve_lanes(avbd_ctx* c, DevState<float>& s, const StepConsts& k, unsigned begin, unsigned count,
                         cudaStream_t st, double* out, const SceneTol& T, const uint32_t* list = nullptr,
                         const uint4* ranges = nullptr, unsigned nranges = 0) {
-    solve_lanes_t<float, float, float, MODE>(c, s, s.inc, k, begin, count, st, out, T, list, ranges, nranges);
+    solve_lanes_t<float, float, float, MODE>(c, s, s.el, k, begin, count, st, out, T, list, ranges, nranges);
 }
 template <int MODE>
 static void solve_lanes(avbd_ctx* c, DevState<double>& s, const StepConsts& k, unsigned begin, unsigned count,
                         cudaStream_t st, double* out, const SceneTol& T, const uint32_t* list = nullptr,
                         const uint4* ranges = nullptr, unsigned nranges = 0) {
     if (c->solver.precision == AVBD_PRECISION_MIXED)
-        solve_lanes_t<double, float, float, MODE>(c, s, s.inc32, k, begin, count, st, out, T, list, ranges, nranges);
+        solve_lanes_t<double, float, float, MODE>(c, s, s.el32, k, begin, count, st, out, T, list, ranges, nranges);
     else
-        solve_lanes_t<double, double, double, MODE>(c, s, s.inc, k, begin, count, st, out, T, list, ranges, nranges);
+        solve_lanes_t<double, double, double, MODE>(c, s, s.el, k, begin, count, st, out, T, list, ranges, nranges);
 }
 
 // The persistent sweep (default; AVBD_PERSISTENT=0 at context creation turns
@@ -846,20 +994,25 @@ static void solve_lanes(avbd_ctx* c, DevState<double>& s, const StepConsts& k, u
 // no oriented particles and no dynamic contacts (the caller checks the last
 // two); returns false, having launched nothing, otherwise.
 template <typename P, typename RS, typename HT>
-static bool sweep_persistent_t(avbd_ctx* c, DevState<P>& s, const IncRec<RS>* inc, const StepConsts& k,
+static bool sweep_persistent_t(avbd_ctx* c, DevState<P>& s, const TetElems<RS>& el, const StepConsts& k,
                                cudaStream_t st, const SceneTol& T) {
     if (!c->persistent || c->lanes != 2 || c->damping || !c->d_solve_ranges || !c->d_solve_range_off ||
         !c->d_sweep_sync || c->num_sms == 0)
         return false;
     const bool ground = !c->ground.empty();
-    auto kern = ground ? k_sweep_persistent<P, RS, HT, 2, true> : k_sweep_persistent<P, RS, HT, 2, false>;
+    auto kern = el.star ? (ground ? k_sweep_persistent<P, RS, HT, 2, FORM_STAR, true>
+                                  : k_sweep_persistent<P, RS, HT, 2, FORM_STAR, false>)
+                        : (ground ? k_sweep_persistent<P, RS, HT, 2, FORM_REC, true>
+                                  : k_sweep_persistent<P, RS, HT, 2, FORM_REC, false>);
+    const unsigned smem = el.star ? StarStage<P, 2>::bytes(el.max_nb) : 0;
+    if (!stage_smem(kern, smem)) return false;
     // resident blocks per SM of this context's instantiation, queried once
     // (-1 where the device cannot launch cooperative kernels: per-color
     // launches then)
     if (c->sweep_blocks_per_sm == 0) {
         int per_sm = 0, coop = 0;
         if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device) != cudaSuccess || !coop ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0) != cudaSuccess || per_sm < 1) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem) != cudaSuccess || per_sm < 1) {
             cudaGetLastError();
             c->sweep_blocks_per_sm = -1;
         } else {
@@ -871,6 +1024,7 @@ static bool sweep_persistent_t(avbd_ctx* c, DevState<P>& s, const IncRec<RS>* in
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)per_sm * c->num_sms);
     cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -879,20 +1033,20 @@ static bool sweep_persistent_t(avbd_ctx* c, DevState<P>& s, const IncRec<RS>* in
     cfg.numAttrs = 1;
     cudaMemsetAsync(c->d_sweep_sync, 0, 3 * sizeof(unsigned), st);
     // a failed launch is left in the runtime's last error, which the step checks
-    cudaLaunchKernelEx(&cfg, kern, s, inc, mkc<P>(k), c->d_counters, T, (const uint4*)c->d_solve_ranges,
+    cudaLaunchKernelEx(&cfg, kern, s, el, mkc<P>(k), c->d_counters, T, (const uint4*)c->d_solve_ranges,
                        (const unsigned*)c->d_solve_range_off, c->num_colors, c->d_sweep_sync);
     count_launch(c);
     return true;
 }
 static bool sweep_persistent(avbd_ctx* c, DevState<float>& s, const StepConsts& k, cudaStream_t st,
                              const SceneTol& T) {
-    return sweep_persistent_t<float, float, float>(c, s, s.inc, k, st, T);
+    return sweep_persistent_t<float, float, float>(c, s, s.el, k, st, T);
 }
 static bool sweep_persistent(avbd_ctx* c, DevState<double>& s, const StepConsts& k, cudaStream_t st,
                              const SceneTol& T) {
     if (c->solver.precision == AVBD_PRECISION_MIXED)
-        return sweep_persistent_t<double, float, float>(c, s, s.inc32, k, st, T);
-    return sweep_persistent_t<double, double, double>(c, s, s.inc, k, st, T);
+        return sweep_persistent_t<double, float, float>(c, s, s.el32, k, st, T);
+    return sweep_persistent_t<double, double, double>(c, s, s.el, k, st, T);
 }
 
 template <typename R>
