@@ -71,6 +71,8 @@ static void free_device(avbd_ctx* c) {
     }
     for (void* p : c->allocations) cudaFree(p);
     c->allocations.clear();
+    for (void* p : c->piece_alloc) cudaFree(p);
+    c->piece_alloc.clear();
     dyn_destroy(c);
     c->f = DevState<float>();
     c->d = DevState<double>();
@@ -98,6 +100,9 @@ static void free_device(avbd_ctx* c) {
     c->graph_tol = false;
     c->d_solve_ranges = nullptr;
     c->solve_range_off.clear();
+    c->d_slabs = nullptr;
+    c->d_sweep_sync = nullptr;
+    std::memset(c->iterate_fits, 0, sizeof(c->iterate_fits));
     mlp_device_free(c->ws_mlp);
     c->ws_mlp = nullptr;
     c->d_ws_feat = c->d_ws_x0 = nullptr;
@@ -488,30 +493,18 @@ struct HostStar {
 // (rest volumes far from any mesh's, or values that are not finite).
 template <typename RS>
 bool build_star(const avbd_ctx* c, const std::vector<uint32_t>& begin, const std::vector<unsigned>& inc_off,
-                const std::vector<uint32_t>& inc_tet, const std::vector<uint16_t>& inc_local, HostStar<RS>& S) {
+                const std::vector<uint32_t>& inc_tet, const std::vector<uint16_t>& inc_local,
+                const std::vector<unsigned>& p_off, const std::vector<unsigned>& p_nbr, HostStar<RS>& S) {
     const unsigned n = (unsigned)c->mass.size();
     S.off.assign(n + 1, make_uint2(0, 0));
     std::atomic<bool> ok{true};
-    // neighbours of vertex i (external ids, ascending) into v
-    auto neighbours = [&](unsigned i, std::vector<unsigned>& v) {
-        const unsigned e = c->perm[i];
-        v.clear();
-        for (unsigned k = inc_off[e]; k < inc_off[e + 1]; k++)
-            for (unsigned j = 0; j < 4; j++)
-                if (j != inc_local[k]) v.push_back(c->nh[inc_tet[k]].idx[j]);
-        std::sort(v.begin(), v.end());
-        v.erase(std::unique(v.begin(), v.end()), v.end());
-    };
-    parallel_vertices(n, [&](unsigned b, unsigned en) {
-        std::vector<unsigned> v;
-        for (unsigned i = b; i < en; i++) {
-            if (begin[i + 1] == begin[i]) continue;
-            neighbours(i, v);
-            if (v.size() > STAR_MAX_NB) ok = false;
-            S.off[i + 1].x = (unsigned)v.size();
-        }
-    });
-    if (!ok) return false;
+    // a positional vertex's neighbours (external ids, ascending) are those of its tets
+    for (unsigned i = 0; i < n; i++) {
+        if (begin[i + 1] == begin[i]) continue;
+        const unsigned e = c->perm[i], m = p_off[e + 1] - p_off[e];
+        if (m > STAR_MAX_NB) return false;
+        S.off[i + 1].x = m;
+    }
     for (unsigned i = 0; i < n; i++) {
         S.max_nb = std::max(S.max_nb, S.off[i + 1].x);
         S.off[i + 1].x += S.off[i].x;
@@ -527,13 +520,13 @@ bool build_star(const avbd_ctx* c, const std::vector<uint32_t>& begin, const std
     auto fits = [&](double x) { return x == 0 || (std::fabs(x) >= lo && std::fabs(x) <= hi); };
     auto bounded = [&](double x) { return std::fabs(x) <= hi; };
     parallel_vertices(n, [&](unsigned b, unsigned en) {
-        std::vector<unsigned> v;
         std::vector<double> w;
         for (unsigned i = b; i < en; i++) {
             if (begin[i + 1] == begin[i]) continue;
-            neighbours(i, v);
-            w.assign(v.size(), 0.0);
             const unsigned e = c->perm[i];
+            const unsigned* v = p_nbr.data() + p_off[e];
+            const unsigned m = p_off[e + 1] - p_off[e];
+            w.assign(m, 0.0);
             double hd = 0, mol = 0;
             size_t t = begin[i];
             for (unsigned k = inc_off[e]; k < inc_off[e + 1]; k++, t++) {
@@ -546,7 +539,7 @@ bool build_star(const avbd_ctx* c, const std::vector<uint32_t>& begin, const std
                 for (unsigned j = 0; j < 4; j++) {
                     if (j == me) continue;
                     d[o] = D[j];
-                    slot[o] = (unsigned)(std::lower_bound(v.begin(), v.end(), h.idx[j]) - v.begin());
+                    slot[o] = (unsigned)(std::lower_bound(v, v + m, h.idx[j]) - v);
                     w[slot[o]] += h.V * h.mu * (D[me][0] * D[j][0] + D[me][1] * D[j][1] + D[me][2] * D[j][2]);
                     o++;
                 }
@@ -563,11 +556,12 @@ bool build_star(const avbd_ctx* c, const std::vector<uint32_t>& begin, const std
                 S.tet[t] = StarTet<RS>{(RS)a, (RS)r};
                 S.loc[t] = slot[0] | slot[1] << 8 | slot[2] << 16;
             }
-            for (size_t j = 0; j < v.size(); j++) {
+            for (unsigned j = 0; j < m; j++) {
                 if (!bounded(w[j])) ok = false;
                 StarNb<RS>& q = S.nb[S.off[i].x + j];
                 q = StarNb<RS>{};
                 q.idx = c->inv[v[j]];
+                if (!c->fixed[v[j]] && c->color[v[j]] < c->color[e]) q.idx += n;
                 q.w = (RS)w[j];
             }
             if (!bounded(hd)) ok = false;
@@ -581,7 +575,8 @@ bool build_star(const avbd_ctx* c, const std::vector<uint32_t>& begin, const std
 template <typename R, typename RS>
 int upload_state(avbd_ctx* c, DevState<R>& s, const std::vector<unsigned>& inc_off,
                  const std::vector<uint32_t>& inc_tet, const std::vector<uint16_t>& inc_local,
-                 const std::vector<int>& ground_of) {
+                 const std::vector<int>& ground_of, const std::vector<unsigned>& p_off,
+                 const std::vector<unsigned>& p_nbr) {
     using V4 = typename Vec4Of<R>::T;
     const unsigned n = (unsigned)c->mass.size();
     s.n = n;
@@ -609,7 +604,7 @@ int upload_state(avbd_ctx* c, DevState<R>& s, const std::vector<unsigned>& inc_o
     }
     const size_t nrec = begin[n];
     HostStar<RS> star;
-    const bool use_star = !c->damping && build_star<RS>(c, begin, inc_off, inc_tet, inc_local, star);
+    const bool use_star = !c->damping && build_star<RS>(c, begin, inc_off, inc_tet, inc_local, p_off, p_nbr, star);
     // algorithmic bytes of each color's solve launch, and of each scene's
     // part of it (the pieces a run-to-tolerance sweep launches per scene)
     c->color_bytes.assign(c->num_colors, 0.0);
@@ -668,7 +663,7 @@ int upload_state(avbd_ctx* c, DevState<R>& s, const std::vector<unsigned>& inc_o
             }
         });
     int rc;
-    if ((rc = dalloc(c, &s.x, n)) || (rc = dalloc(c, &s.y, n)) || (rc = dalloc(c, &s.xp, n)) ||
+    if ((rc = dalloc(c, &s.x, 2ull * n)) || (rc = dalloc(c, &s.y, n)) || (rc = dalloc(c, &s.xp, n)) ||
         (rc = dalloc(c, &s.xl, n)) || (rc = dalloc(c, &s.xll, n)) || (rc = dalloc(c, &s.v, n)) ||
         (rc = dalloc(c, &s.vp, n)) || (rc = dalloc(c, &s.flags, n)))
         return rc;
@@ -693,6 +688,7 @@ int upload_state(avbd_ctx* c, DevState<R>& s, const std::vector<unsigned>& inc_o
     if constexpr (std::is_same<R, RS>::value) s.el = el;
     else s.el32 = el;
     c->star_nb = el.max_nb;
+    c->star_off.swap(star.off);
     CUDA_OR_FAIL(cudaMemcpyAsync(s.x, x.data(), sizeof(V4) * n, cudaMemcpyHostToDevice, st));
     CUDA_OR_FAIL(cudaMemcpyAsync(s.y, y.data(), sizeof(V4) * n, cudaMemcpyHostToDevice, st));
     CUDA_OR_FAIL(cudaMemcpyAsync(s.xp, x.data(), sizeof(V4) * n, cudaMemcpyHostToDevice, st));
@@ -1039,11 +1035,11 @@ extern "C" int avbd_finalize(avbd_ctx* c) {
     CUDA_OR_FAIL(cudaMemcpyAsync(c->d_perm, c->perm.data(), sizeof(unsigned) * n, cudaMemcpyHostToDevice, c->stream));
     CUDA_OR_FAIL(cudaMemcpyAsync(c->d_inv, c->inv.data(), sizeof(unsigned) * n, cudaMemcpyHostToDevice, c->stream));
     if (c->solver.precision == AVBD_PRECISION_MIXED)
-        rc = upload_state<double, float>(c, c->d, inc_off, inc_tet, inc_local, ground_of);
+        rc = upload_state<double, float>(c, c->d, inc_off, inc_tet, inc_local, ground_of, p_off, p_nbr);
     else if (use64(c))
-        rc = upload_state<double, double>(c, c->d, inc_off, inc_tet, inc_local, ground_of);
+        rc = upload_state<double, double>(c, c->d, inc_off, inc_tet, inc_local, ground_of, p_off, p_nbr);
     else
-        rc = upload_state<float, float>(c, c->f, inc_off, inc_tet, inc_local, ground_of);
+        rc = upload_state<float, float>(c, c->f, inc_off, inc_tet, inc_local, ground_of, p_off, p_nbr);
     if (rc) return rc;
     // per-scene run-to-tolerance state
     {
@@ -1057,8 +1053,8 @@ extern "C" int avbd_finalize(avbd_ctx* c) {
                 mg2[scene_of[e]] += c->mass[e] * c->mass[e];  // sum of m^2; g^2 is applied per step
             }
         if ((rc = dalloc(c, &c->d_scene, n)) || (rc = dalloc(c, &c->d_scene_active, S)) ||
-            (rc = dalloc(c, &c->d_scene_cand, S)) || (rc = dalloc(c, &c->d_scene_r2, S)) ||
-            (rc = dalloc(c, &c->d_scene_ex, S)) || (rc = dalloc(c, &c->d_scene_rin, S)) || (rc = dalloc(c, &c->d_scene_mg2, S)) ||
+            (rc = dalloc(c, &c->d_scene_cand, S)) || (rc = dalloc(c, &c->d_scene_r2, 3ull * S)) ||
+            (rc = dalloc(c, &c->d_scene_ex, 2ull * S)) || (rc = dalloc(c, &c->d_scene_rin, S)) || (rc = dalloc(c, &c->d_scene_mg2, S)) ||
             (rc = dalloc(c, &c->d_scene_iters, S)) || (rc = dalloc(c, &c->d_tol_count, 1)) ||
             (rc = dalloc(c, &c->d_tol_it, 1)) || (rc = dalloc(c, &c->d_tol_omega, 1)))
             return rc;
@@ -1075,11 +1071,9 @@ extern "C" int avbd_finalize(avbd_ctx* c) {
                 b = q;
             }
         }
-        // pieces of at most solve_chunk vertices for the sweeps (AVBD_SOLVE_CHUNK
-        // overrides; 0 launches whole slabs): 256 for the persistent sweep,
-        // whose blocks draw pieces by ticket (a finer grain shortens each
-        // color's tail at its grid barrier), 512 for one block per piece
-        c->solve_chunk = c->persistent ? 256 : 512;
+        // pieces of at most solve_chunk vertices for sweeps of one launch per
+        // color (AVBD_SOLVE_CHUNK overrides; 0 launches whole slabs)
+        c->solve_chunk = 512;
         if (const char* env = getenv("AVBD_SOLVE_CHUNK")) c->solve_chunk = (unsigned)atoi(env);
         c->solve_range_off.assign(nc + 1, 0);
         std::vector<uint4> pieces;
@@ -1098,13 +1092,11 @@ extern "C" int avbd_finalize(avbd_ctx* c) {
             if ((rc = dalloc(c, &c->d_solve_ranges, pieces.size()))) return rc;
             CUDA_OR_FAIL(cudaMemcpyAsync(c->d_solve_ranges, pieces.data(), sizeof(uint4) * pieces.size(),
                                          cudaMemcpyHostToDevice, c->stream));
-            if (c->persistent) {
-                if ((rc = dalloc(c, &c->d_solve_range_off, nc + 1)) || (rc = dalloc(c, &c->d_sweep_sync, 3)))
-                    return rc;
-                CUDA_OR_FAIL(cudaMemcpyAsync(c->d_solve_range_off, c->solve_range_off.data(),
-                                             sizeof(uint32_t) * (nc + 1), cudaMemcpyHostToDevice, c->stream));
-            }
         }
+        std::vector<uint4> slabs(nc);
+        for (unsigned k = 0; k < nc; k++) slabs[k] = make_uint4(c->color_begin[k], c->color_solve[k], 0, 0);
+        if ((rc = dalloc(c, &c->d_slabs, nc)) || (rc = dalloc(c, &c->d_sweep_sync, 4))) return rc;
+        CUDA_OR_FAIL(cudaMemcpyAsync(c->d_slabs, slabs.data(), sizeof(uint4) * nc, cudaMemcpyHostToDevice, c->stream));
         CUDA_OR_FAIL(cudaMemcpyAsync(c->d_scene_mg2, mg2.data(), sizeof(double) * S, cudaMemcpyHostToDevice, c->stream));
         CUDA_OR_FAIL(cudaStreamSynchronize(c->stream));
     }
@@ -1119,6 +1111,7 @@ extern "C" int avbd_finalize(avbd_ctx* c) {
     c->stats.num_scenes = (unsigned)sb.size() - 1;
     trace("finalize: autotune");
     if (int r3 = autotune(c)) return r3;
+    std::vector<uint2>().swap(c->star_off);
     c->finalized = true;
     c->graph_dirty = true;
     return AVBD_OK;
@@ -1174,8 +1167,6 @@ void enqueue_sweep(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaStream_
         for (unsigned col = 0; col < nc; col++) dyn_solve_color<R>(c, s, k, col, st, T);
         return;
     }
-    // the persistent sweep covers tet-only contexts (no 6-DOF slabs between the colors)
-    if (T.active && c->persistent && s.no == 0 && launch_sweep_persistent<R>(c, s, k, st, T)) return;
     for (unsigned col = 0; col < c->num_colors; col++) {
         if (c->color_solve[col] && T.active && c->d_solve_ranges) {  // run-to-tolerance: per-scene pieces
             const unsigned r0 = c->solve_range_off[col], r1 = c->solve_range_off[col + 1];
@@ -1223,10 +1214,14 @@ void enqueue_iteration(avbd_ctx* c, DevState<R>& s, const StepConsts& k, double 
 template <typename R>
 int enqueue_step_fixed(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaStream_t st) {
     if (int r = enqueue_begin<R>(c, s, k, st)) return r;
-    double omega = 1;
-    for (unsigned i = 0; i < c->solver.solver_iters; i++) {
-        omega = omega_at(i, c->solver.iter_acceleration, omega);
-        enqueue_iteration<R>(c, s, k, omega, i, st);
+    IterLaunch L;
+    L.n = c->solver.solver_iters;
+    if (L.n == 0 || !launch_iterate<R>(c, s, k, st, L)) {
+        double omega = 1;
+        for (unsigned i = 0; i < c->solver.solver_iters; i++) {
+            omega = omega_at(i, c->solver.iter_acceleration, omega);
+            enqueue_iteration<R>(c, s, k, omega, i, st);
+        }
     }
     enqueue_velocity<R>(c, s, k, st);
     return AVBD_OK;
@@ -1289,27 +1284,37 @@ int step_fixed_dyn_graph(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaS
 
 StepConsts consts(avbd_ctx* c) { return StepConsts{c->params.dt, c->params.g_accel, c->kappa_max}; }
 
-// Picks the threads-per-vertex of the tet solve (1, 2, 4, 8, 16 or 32) by timing one
-// sweep of every color slab with each choice on the context's own data.
-// Positions are snapshotted and restored, so the state is untouched.
-// AVBD_LANES=<n> in the environment forces a choice.
+// Picks the threads-per-vertex of the tet solve (1, 2, 4, 8 or 16; 2 or 8 with
+// the records) by timing sweeps with each choice on the context's own data,
+// in the launches a step will use.  Positions are snapshotted and restored,
+// so the state is untouched.  AVBD_LANES=<n> in the environment forces a
+// choice.
 template <typename R>
 int autotune_impl(avbd_ctx* c, DevState<R>& s) {
+    cudaStream_t st = c->stream;
     const char* env = getenv("AVBD_LANES");
     if (env) {
         int l = atoi(env);
-        if (l == 1 || l == 2 || l == 4 || l == 8 || l == 16 || l == 32) c->lanes = std::min(std::max(l, 2), 16);
-        if (!c->star_nb && c->lanes != 2) c->lanes = 8;
-        return AVBD_OK;
+        if (l == 1 || l == 2 || l == 4 || l == 8 || l == 16 || l == 32) c->lanes = std::min(l, 16);
+        if (!c->star_nb && c->lanes > 2) c->lanes = 8;
+        if (!c->star_nb && c->lanes < 2) c->lanes = 2;
+        return layout_pieces<R>(c, s, st);
     }
     unsigned long long solved = 0;
     for (unsigned v : c->color_solve) solved += v;
     c->lanes = 8;
-    if (solved < 50000) return AVBD_OK;
+    const bool whole = c->persistent && s.no == 0 && !c->dyn && solved > 0;  // iterations are one launch
+    if (!whole && solved < 50000) return AVBD_OK;
+    // with the iterations in one launch, more threads a vertex shorten the
+    // chain between two barriers of a small color (8: 17^3 638 against 655 us a
+    // pass with 4, 662 with 16) and fewer take less instructions of a large one
+    // (59,000 vertices a color: 3.16 ms with 4, 3.59 with 1, 5.42 with 8)
+    std::vector<int> choices = {2, 4, 8, 16};
+    if (!c->star_nb) choices = {2, 8};
+    else if (whole) choices = c->max_color_solve < 20000 ? std::vector<int>{4, 8} : std::vector<int>{1, 4};
     using V4 = typename Vec4Of<R>::T;
     V4* snap = nullptr;
     CUDA_OR_FAIL(cudaMalloc(&snap, sizeof(V4) * s.n));
-    cudaStream_t st = c->stream;
     CUDA_OR_FAIL(cudaMemcpyAsync(snap, s.x, sizeof(V4) * s.n, cudaMemcpyDeviceToDevice, st));
     StepConsts k = consts(c);
     cudaEvent_t a, b;
@@ -1318,11 +1323,16 @@ int autotune_impl(avbd_ctx* c, DevState<R>& s) {
     const unsigned long long launches0 = c->stats.kernel_launches;
     int best = 8;
     float best_ms = 1e30f;
-    for (int l : {2, 4, 8, 16}) {
-        if (!c->star_nb && l != 2 && l != 8) continue;
+    for (int l : choices) {
         c->lanes = l;
+        if (whole)
+            if (int r = layout_pieces<R>(c, s, st)) return r;
         for (int rep = 0; rep < 2; rep++) {  // rep 0 warms up, rep 1 is timed
             if (rep == 1) CUDA_OR_FAIL(cudaEventRecord(a, st));
+            IterLaunch L;
+            L.n = solved < 50000 ? 16 : 2;
+            L.sweep_only = true;
+            if (launch_iterate<R>(c, s, k, st, L)) continue;
             for (unsigned col = 0; col < c->num_colors; col++) {
                 if (!c->color_solve[col]) continue;
                 if (c->solver.residual_tolerance > 0 && c->d_solve_ranges) {  // the launches a step will use
@@ -1332,8 +1342,8 @@ int autotune_impl(avbd_ctx* c, DevState<R>& s) {
                     launch_solve_color<R>(c, s, k, c->color_begin[col], c->color_solve[col], st);
                 }
             }
-            if (rep == 1) CUDA_OR_FAIL(cudaEventRecord(b, st));
         }
+        CUDA_OR_FAIL(cudaEventRecord(b, st));
         CUDA_OR_FAIL(cudaEventSynchronize(b));
         float ms = 0;
         CUDA_OR_FAIL(cudaEventElapsedTime(&ms, a, b));
@@ -1349,7 +1359,11 @@ int autotune_impl(avbd_ctx* c, DevState<R>& s) {
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     cudaFree(snap);
-    c->lanes = best;
+    if (c->lanes != best) {
+        c->lanes = best;
+        if (whole)
+            if (int r = layout_pieces<R>(c, s, st)) return r;
+    }
     c->stats.kernel_launches = launches0;
     if (getenv("AVBD_TRACE")) fprintf(stderr, "[avbd] autotune: %d threads per vertex (%.3f ms per sweep)\n", best, best_ms);
     return AVBD_OK;
@@ -1414,6 +1428,7 @@ int build_tol_graph(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaStream
     if (e != cudaSuccess) return abandon("graph capture: ", e);
     enqueue_begin<R>(c, s, k, st);  // no host step without dynamic contacts: cannot fail
     launch_tol_init(c, st);
+    launch_iter_set(c, st);
     cudaStreamCaptureStatus cs;
     const cudaGraphNode_t* deps = nullptr;
     size_t ndeps = 0;
@@ -1438,13 +1453,23 @@ int build_tol_graph(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaStream
     e = cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, mode);
     if (e != cudaSuccess) return abandon("graph capture: ", e);
     const unsigned long long body0 = c->stats.kernel_launches;
-    enqueue_sweep<R>(c, s, k, st, loopT);
-    enqueue_chebyshev<R>(c, s, k, 1.0, 0, st, loopT);
-    launch_tol_decide_a(c, tol, st);
-    enqueue_residual<R>(c, s, k, nullptr, st, resT);
-    launch_tol_decide_b(c, tol, max_it, st);
-    const unsigned body_launches = (unsigned)(c->stats.kernel_launches - body0);
-    launch_tol_loop_next(c, h, max_it, body_launches, st);
+    IterLaunch L;
+    L.n = TOL_ITERS_PER_LAUNCH;
+    L.tol = tol;
+    L.max_it = max_it;
+    L.loop = &h;
+    unsigned body_launches;
+    if (launch_iterate<R>(c, s, k, st, L)) {
+        body_launches = (unsigned)(c->stats.kernel_launches - body0);
+    } else {
+        enqueue_sweep<R>(c, s, k, st, loopT);
+        enqueue_chebyshev<R>(c, s, k, 1.0, 0, st, loopT);
+        launch_tol_decide_a(c, tol, st);
+        enqueue_residual<R>(c, s, k, nullptr, st, resT);
+        launch_tol_decide_b(c, tol, max_it, st);
+        body_launches = (unsigned)(c->stats.kernel_launches - body0);
+        launch_tol_loop_next(c, h, max_it, body_launches, st);
+    }
     e = cudaStreamEndCapture(st, &body);
     if (e != cudaSuccess) return abandon("graph capture: ", e);
     // step end
@@ -1517,17 +1542,28 @@ int step_impl(avbd_ctx* c, DevState<R>& s, unsigned n_steps) {
             CUDA_OR_FAIL(cudaGetLastError());
             return AVBD_OK;
         }
+        if (int r = ensure_omega_table(c, max_it, st)) return r;
         for (unsigned t = 0; t < n_steps; t++) {
             if (int r = enqueue_begin<R>(c, s, k, st)) return r;
             launch_tol_init(c, st);
             double omega = 1;
-            for (unsigned it = 0; it < max_it; it++) {
-                omega = omega_at(it, c->solver.iter_acceleration, omega);
-                enqueue_sweep<R>(c, s, k, st, solveT);
-                enqueue_chebyshev<R>(c, s, k, omega, it, st, solveT);
-                launch_tol_decide_a(c, tol, st);
-                enqueue_residual<R>(c, s, k, nullptr, st, resT);
-                launch_tol_decide_b(c, tol, max_it, st);
+            IterLaunch L;
+            L.n = TOL_ITERS_PER_LAUNCH;
+            L.tol = tol;
+            L.max_it = max_it;
+            for (unsigned it = 0; it < max_it;) {
+                L.it0 = it;
+                if (launch_iterate<R>(c, s, k, st, L)) {
+                    it += L.n;
+                } else {
+                    omega = omega_at(it, c->solver.iter_acceleration, omega);
+                    enqueue_sweep<R>(c, s, k, st, solveT);
+                    enqueue_chebyshev<R>(c, s, k, omega, it, st, solveT);
+                    launch_tol_decide_a(c, tol, st);
+                    enqueue_residual<R>(c, s, k, nullptr, st, resT);
+                    launch_tol_decide_b(c, tol, max_it, st);
+                    it++;
+                }
                 int n_active = 0;
                 CUDA_OR_FAIL(cudaMemcpyAsync(&n_active, c->d_tol_count, sizeof(int), cudaMemcpyDeviceToHost, st));
                 CUDA_OR_FAIL(cudaStreamSynchronize(st));
@@ -1538,6 +1574,7 @@ int step_impl(avbd_ctx* c, DevState<R>& s, unsigned n_steps) {
         CUDA_OR_FAIL(cudaGetLastError());
         return AVBD_OK;
     }
+    if (int r = ensure_omega_table(c, c->solver.solver_iters, st)) return r;
     if (capturable && !c->graph) {
         unsigned long long before = c->stats.kernel_launches;
         cudaGraph_t g;
@@ -1832,11 +1869,11 @@ int avbd_debug_block(avbd_ctx* c, unsigned p, double* G, double* H, int* dof) {
 
 namespace {
 
-// One run-to-tolerance step with the launches the timed step uses (the
-// per-scene pieces of every color slab, converged scenes gated out), driven
-// from the host like the graph-less path, with CUDA events around every
-// color's sweep launch.  Bytes: the algorithmic bytes of the scenes still
-// iterating when each sweep starts.
+// One run-to-tolerance step driven from the host, with CUDA events around its
+// solve launches: of tetrahedral contexts each iteration as one launch of the
+// timed step's kernel (its decisions included; the timed step runs up to 32
+// per launch), else the per-scene pieces of every color slab.  Bytes: the
+// algorithmic bytes of the scenes still iterating when each launch starts.
 template <typename R>
 int profile_step_impl(avbd_ctx* c, DevState<R>& s, double* solve_ms, double* solve_bytes, unsigned* launches,
                       unsigned* iterations) {
@@ -1848,6 +1885,16 @@ int profile_step_impl(avbd_ctx* c, DevState<R>& s, double* solve_ms, double* sol
     SceneTol solveT{c->d_scene, c->d_scene_active, nullptr, c->d_scene_r2, nullptr};
     SceneTol resT{c->d_scene, nullptr, c->d_scene_cand, nullptr, c->d_scene_ex};
     std::vector<uint8_t> act(S);
+    std::vector<unsigned> sb = c->scene_begin;
+    if (sb.back() != s.n) sb.push_back(s.n);
+    // Chebyshev and ground duals of one vertex, inside the whole-iteration launch
+    const double V4B = sizeof(typename Vec4Of<R>::T);
+    const double cheb_b = 4 * V4B + 6 + (c->ground.empty() ? 0.0 : 5 * V4B + 2);
+    IterLaunch L;
+    L.n = 1;
+    L.tol = tol;
+    L.max_it = max_it;
+    if (int r = ensure_omega_table(c, max_it, st)) return r;
     std::vector<cudaEvent_t> ev(2ull * nc);
     for (auto& e : ev) CUDA_OR_FAIL(cudaEventCreate(&e));
     double ms = 0, bytes = 0;
@@ -1862,42 +1909,43 @@ int profile_step_impl(avbd_ctx* c, DevState<R>& s, double* solve_ms, double* sol
             rc = fail(AVBD_ERR_CUDA, "profile: scene flags");
             break;
         }
-        // the persistent sweep: one launch (and its 12-byte sync reset) timed
-        // for all colors
-        bool persist = false;
-        if (c->persistent && s.no == 0) {
-            cudaEventRecord(ev[0], st);
-            persist = launch_sweep_persistent<R>(c, s, k, st, solveT);
-            cudaEventRecord(ev[1], st);
-        }
-        for (unsigned col = 0; col < nc; col++) {
-            if (!persist) cudaEventRecord(ev[2 * col], st);
-            if (c->color_solve[col]) {
-                if (!persist) {
+        for (unsigned sc = 0; sc < S; sc++)
+            if (act[sc])
+                for (unsigned col = 0; col < nc; col++) bytes += c->color_scene_bytes[(size_t)col * S + sc];
+        // tetrahedral contexts: the whole iteration is one launch
+        cudaEventRecord(ev[0], st);
+        L.it0 = it;
+        const bool whole = launch_iterate<R>(c, s, k, st, L);
+        cudaEventRecord(ev[1], st);
+        if (whole) {
+            nl++;
+            for (unsigned sc = 0; sc < S; sc++)
+                if (act[sc]) bytes += cheb_b * (sb[sc + 1] - sb[sc]);
+        } else {
+            for (unsigned col = 0; col < nc; col++) {
+                cudaEventRecord(ev[2 * col], st);
+                if (c->color_solve[col]) {
                     const unsigned r0 = c->solve_range_off[col], r1 = c->solve_range_off[col + 1];
                     launch_solve_color<R>(c, s, k, 0, 0, st, solveT, nullptr, c->d_solve_ranges + r0, r1 - r0);
                     nl++;
                 }
-                for (unsigned sc = 0; sc < S; sc++)
-                    if (act[sc]) bytes += c->color_scene_bytes[(size_t)col * S + sc];
+                cudaEventRecord(ev[2 * col + 1], st);
+                if (c->color_orient[col])
+                    launch_solve_rod<R>(c, s, k, c->color_begin[col] + c->color_solve[col], c->color_orient[col], st,
+                                        solveT, 0, nullptr);
             }
-            if (!persist) cudaEventRecord(ev[2 * col + 1], st);
-            if (c->color_orient[col])
-                launch_solve_rod<R>(c, s, k, c->color_begin[col] + c->color_solve[col], c->color_orient[col], st,
-                                    solveT, 0, nullptr);
+            enqueue_chebyshev<R>(c, s, k, omega, it, st, solveT);
+            launch_tol_decide_a(c, tol, st);
+            enqueue_residual<R>(c, s, k, nullptr, st, resT);
+            launch_tol_decide_b(c, tol, max_it, st);
         }
-        if (persist) nl++;
-        enqueue_chebyshev<R>(c, s, k, omega, it, st, solveT);
-        launch_tol_decide_a(c, tol, st);
-        enqueue_residual<R>(c, s, k, nullptr, st, resT);
-        launch_tol_decide_b(c, tol, max_it, st);
         int n_active = 0;
         if (cudaMemcpyAsync(&n_active, c->d_tol_count, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess) {
             rc = fail(AVBD_ERR_CUDA, "profile: iteration count");
             break;
         }
-        for (unsigned col = 0; col < (persist ? 1u : nc); col++) {
+        for (unsigned col = 0; col < (whole ? 1u : nc); col++) {
             float t = 0;
             if (cudaEventElapsedTime(&t, ev[2 * col], ev[2 * col + 1]) == cudaSuccess) ms += t;
         }

@@ -75,10 +75,13 @@ struct Sym3 {
     R a00, a11, a22, a01, a02, a12;
 };
 
-// Solves (A) x = b for a symmetric 3x3 through the adjugate.  Returns the
-// condition estimate kappa = |A|_F |adj A|_F / |det A| (infinite when singular).
+// Solves (A) x = b for a symmetric 3x3 through the adjugate.  False when the
+// condition estimate |A|_F |adj A|_F / |det A| exceeds kappa_max (or is not a
+// number); compared squared, each norm scaled by the determinant first, which
+// needs no square root and stays in range where the product of the norms
+// would not.
 template <typename R>
-AVBD_D R solve_sym3(const Sym3<R>& A, V3<R> b, V3<R>& x) {
+AVBD_D bool solve_sym3(const Sym3<R>& A, V3<R> b, R kappa_max, V3<R>& x) {
     R c00 = A.a11 * A.a22 - A.a12 * A.a12;
     R c01 = A.a02 * A.a12 - A.a01 * A.a22;
     R c02 = A.a01 * A.a12 - A.a02 * A.a11;
@@ -92,7 +95,7 @@ AVBD_D R solve_sym3(const Sym3<R>& A, V3<R> b, V3<R>& x) {
     x.z = (c02 * b.x + c12 * b.y + c22 * b.z) * inv;
     R na = A.a00 * A.a00 + A.a11 * A.a11 + A.a22 * A.a22 + R(2) * (A.a01 * A.a01 + A.a02 * A.a02 + A.a12 * A.a12);
     R nc = c00 * c00 + c11 * c11 + c22 * c22 + R(2) * (c01 * c01 + c02 * c02 + c12 * c12);
-    return sqrt(na * nc) * fabs(inv);
+    return (na * fabs(inv)) * (nc * fabs(inv)) <= kappa_max * kappa_max;
 }
 
 // Dense LU with row pivoting for small N in FP64 (the fallback for

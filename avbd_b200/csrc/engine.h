@@ -50,6 +50,9 @@ static_assert(sizeof(IncRec<double>) == 112, "FP64 incidence record must be 112 
 // and 8 a neighbour instead of 64 a tet (FP32 records), and a quarter of the
 // arithmetic of forming F.  W and a, r are the same numbers in the lists of
 // all four vertices of a tet, so the element forces balance exactly.
+// A neighbour's id is tagged (n added) when it is solved in an earlier color:
+// k_iterate keeps this iteration's solved positions in the second half of x
+// and the accelerated ones in the first.
 template <typename R> struct StarNb;
 template <> struct alignas(8) StarNb<float> { uint32_t idx; float w; };
 template <> struct alignas(16) StarNb<double> { uint32_t idx, pad; double w; };
@@ -72,6 +75,15 @@ struct TetElems {
     const RS* hd = nullptr;               // per vertex
     const float* mol = nullptr;           // per vertex: sum of mu/lambda over its tets (warm-start feature)
     unsigned max_nb = 0;                  // largest neighbour count of the context
+    // the same lists as k_iterate streams them with `lanes` threads a vertex
+    // (null: not laid out): per piece of 32 / lanes consecutive vertices of a
+    // color, rounds of 32 entries, entry i of a round being thread i's, so a
+    // warp's load is contiguous.  Filled up with the vertex itself at weight
+    // 0 and with tets of constants 0.
+    const uint4* piece = nullptr;         // first neighbour entry, rounds, first tet entry, rounds
+    const StarNb<RS>* pnb = nullptr;
+    const StarTet<RS>* ptet = nullptr;
+    const uint32_t* ploc = nullptr;
 };
 
 enum VertexFlags : uint8_t { VF_FIXED = 1, VF_ORIENTED = 2, VF_GROUND = 4 };
@@ -105,6 +117,8 @@ struct DevState {
     // Iteration k reads o_(k-2) from buffer k&1 (xl even, xll odd) and writes
     // its accelerated iterate o_k there; both hold the step's start position
     // before iteration 0.
+    // x has 2 n entries: the positions, then the solved positions of the
+    // iteration in flight (k_iterate)
     V4 *x = nullptr, *y = nullptr, *xp = nullptr, *xl = nullptr, *xll = nullptr, *v = nullptr, *vp = nullptr;
     uint8_t* flags = nullptr;
     TetElems<R> el;
@@ -321,15 +335,16 @@ struct avbd_ctx {
     // run-to-tolerance steps launch one block per piece
     uint4* d_solve_ranges = nullptr;
     std::vector<unsigned> solve_range_off;
-    uint32_t* d_solve_range_off = nullptr;  // device copy of solve_range_off
     unsigned solve_chunk = 512;
-    // persistent sweep (default; AVBD_PERSISTENT=0 turns it off): all colors
-    // of an iteration in one cooperative launch with grid barriers;
-    // [ticket, arrivals, generation]
+    // iterations of tetrahedral contexts in one cooperative launch with grid
+    // barriers (default; AVBD_PERSISTENT=0 turns it off)
     bool persistent = true;
-    uint32_t* d_sweep_sync = nullptr;
+    uint4* d_slabs = nullptr;           // per color: first internal vertex, solved positional vertices, first piece
+    std::vector<uint2> star_off;        // host copy of TetElems::star, during finalize
+    std::vector<void*> piece_alloc;     // the laid-out lists (TetElems::piece ...), replaced by each lane choice
+    uint32_t* d_sweep_sync = nullptr;   // IterArgs::sync
     unsigned num_sms = 0;
-    int sweep_blocks_per_sm = 0;        // 0: not queried yet, -1: the kernel cannot run
+    int8_t iterate_fits[2][5] = {};     // [run to tolerance][lanes 2, 4, 8, 16, 1]: 0 not queried, 1 yes, -1 no
     unsigned long long host_iterations = 0;  // scene-iterations of fixed-iteration steps
 
     // CUDA graph of one full step: fixed iterations, or (graph_tol) the
@@ -415,10 +430,27 @@ template <typename R>
 void launch_solve_color(avbd_ctx* c, DevState<R>& s, const StepConsts& k, unsigned begin, unsigned count,
                         cudaStream_t st, const SceneTol& T = SceneTol(), const uint32_t* list = nullptr,
                         const uint4* ranges = nullptr, unsigned nranges = 0);
-// the whole sweep of a run-to-tolerance iteration as one cooperative launch
-// (persistent contexts); false when the context does not qualify
+// up to n iterations from it0 of a tetrahedral context as one cooperative
+// launch (solve.cu, k_iterate); tol > 0: run to tolerance with the step's
+// iteration cap max_it, in a graph's while loop when `loop` is given (the
+// first iteration is then d_tol_it's).  False, having launched nothing, when
+// the context does not qualify: oriented particles, dynamic contacts,
+// AVBD_PERSISTENT=0, no cooperative launches.
+struct IterLaunch {
+    unsigned it0 = 0, n = 0;
+    double tol = 0;
+    unsigned max_it = 0;
+    const cudaGraphConditionalHandle* loop = nullptr;
+    bool sweep_only = false;            // the colors' solves alone (timing of the lane choice)
+};
+// iterations of one launch of a run-to-tolerance loop
+constexpr unsigned TOL_ITERS_PER_LAUNCH = 32;
 template <typename R>
-bool launch_sweep_persistent(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaStream_t st, const SceneTol& T);
+bool launch_iterate(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaStream_t st, const IterLaunch& L);
+// lays the star form out for k_iterate at c->lanes threads a vertex (nothing
+// to do without the star form or at 2 lanes)
+template <typename R>
+int layout_pieces(avbd_ctx* c, DevState<R>& s, cudaStream_t st);
 // poll limit of the persistent sweep's grid barriers (avbd_debug_set_wait_limit)
 int solve_set_wait_limit(unsigned polls);
 // poll limit of the recoloring's grid barriers (avbd_debug_set_wait_limit)

@@ -16,6 +16,9 @@
 //   GroundCollisionEnergySolver                  energy/collision/GroundCollisionEnergySolver.hpp:14-91
 #include <cuda_bf16.h>
 
+#include <algorithm>
+#include <type_traits>
+
 #include "engine.h"
 #include "contact_dyn.cuh"
 
@@ -32,6 +35,7 @@ static Consts<R> mkc(const StepConsts& k) {
 }
 
 static inline unsigned nblocks(unsigned n, unsigned per) { return (n + per - 1) / per; }
+static constexpr unsigned ITER_WARPS_MIN = 4;  // warps of work per block of an iteration launch, at least
 
 // ----------------------------------------------------------- step start
 // Energy hooks of the step start for per-vertex ground contact
@@ -289,23 +293,75 @@ AVBD_D StarTet<double> ld_once(const StarTet<double>* p) {
 // vertex read different j and neighbouring vertices mostly the same j, so the
 // stride is skewed by a half-warp's (FP64) or a warp's (FP32) width over
 // LANES to spread both over the banks.
-template <typename P, int LANES>
+template <typename P, int LANES, int THREADS = 256>
 struct StarStage {
-    static constexpr unsigned GROUPS = 256 / LANES;
+    static constexpr unsigned GROUPS = THREADS / LANES;
     static constexpr unsigned STRIDE = GROUPS + (sizeof(P) == 8 ? 16 : 32) / LANES;
     static unsigned bytes(unsigned max_nb) { return 3 * max_nb * STRIDE * (unsigned)sizeof(P); }
 };
+
+// double of a float whose magnitude is normal or zero (element constants, see
+// build_star), by integer arithmetic: the mantissa moves up 29 bits and the
+// exponent's bias grows by 896.  The conversion instruction runs on a unit of
+// a few lanes (at one conversion per constant it was the busiest pipe of the
+// mixed solve); zero becomes 2^-127, which vanishes next to any element.
+AVBD_D double widen(float f) {
+    const uint32_t u = __float_as_uint(f);
+    const unsigned long long m = (unsigned long long)(u & 0x7FFFFFFFu) * 0x20000000ull + 0x3800000000000000ull;
+    return __hiloint2double((int)((uint32_t)(m >> 32) | (u & 0x80000000u)), (int)(uint32_t)m);
+}
+template <typename P> AVBD_D P const_as(float f) { return (P)f; }
+template <> AVBD_D double const_as<double>(float f) { return widen(f); }
+template <typename P> AVBD_D P const_as(double f) { return (P)f; }
+
+// One tet of the star form: its edges from the staging slot.
+template <typename P, typename RS, typename HT, unsigned ST>
+AVBD_D void star_tet(const StarTet<RS>& q, uint32_t l, const P* es, unsigned K, Block3<P, HT>& B) {
+    const P* p1 = es + (l & 255u) * ST;
+    const P* p2 = es + (l >> 8 & 255u) * ST;
+    const P* p3 = es + (l >> 16) * ST;
+    const V3<P> e1 = mk3(p1[0], p1[K * ST], p1[2 * K * ST]);
+    const V3<P> f2 = mk3(p2[0], p2[K * ST], p2[2 * K * ST]) - e1;
+    const V3<P> f3 = mk3(p3[0], p3[K * ST], p3[2 * K * ST]) - e1;
+    const V3<P> N = cross3(f2, f3);
+    const P qa = const_as<P>(q.a);
+    const P h = qa * (const_as<P>(q.r) - dot3(e1, N));
+    B.g0 += h * N.x;
+    B.g1 += h * N.y;
+    B.g2 += h * N.z;
+    const HT nx = (HT)N.x, ny = (HT)N.y, nz = (HT)N.z, a = (HT)qa;
+    const HT ax = a * nx, ay = a * ny, az = a * nz;
+    B.h00 += ax * nx;
+    B.h11 += ay * ny;
+    B.h22 += az * nz;
+    B.h01 += ax * ny;
+    B.h02 += ax * nz;
+    B.h12 += ay * nz;
+}
+
+// One neighbour of the star form: its edge staged, its weight applied.
+template <typename P, typename RS, typename HT, unsigned ST>
+AVBD_D void star_edge(RS wr, V3<P> e, P* d, unsigned K, Block3<P, HT>& B) {
+    d[0] = e.x;
+    d[K * ST] = e.y;
+    d[2 * K * ST] = e.z;
+    const P w = const_as<P>(wr);
+    B.g0 += w * e.x;
+    B.g1 += w * e.y;
+    B.g2 += w * e.z;
+}
 
 // The block of a vertex from its star form (StarNb): the edges to the distinct
 // neighbours are gathered once (14 instead of 61 positions on the split hex
 // grids) and staged in shared memory, the deviatoric part summed over them;
 // then each tet takes its three edges from there.  es: this vertex's slot.
-template <typename P, typename RS, typename HT, int LANES, bool COH>
+template <typename P, typename RS, typename HT, int LANES, bool COH, int THREADS>
 AVBD_D void accumulate_star(const DevState<P>& s, const TetElems<RS>& el, uint2 o0, uint2 o1, unsigned lane, V3<P> xi,
                             P* es, Block3<P, HT>& B) {
-    constexpr unsigned ST = StarStage<P, LANES>::STRIDE;
+    constexpr unsigned ST = StarStage<P, LANES, THREADS>::STRIDE;
     constexpr unsigned U = LANES <= 2 ? 4 : 2;  // neighbour gathers in flight per lane
-    const unsigned K = el.max_nb;
+    const unsigned K = el.max_nb, n = s.n;
+    auto plain = [n](unsigned idx) { return idx < n ? idx : idx - n; };  // of a tagged id (StarNb)
     for (unsigned j = o0.x + lane; j < o1.x; j += U * LANES) {
         StarNb<RS> q[U];
         V3<P> e[U];
@@ -314,45 +370,17 @@ AVBD_D void accumulate_star(const DevState<P>& s, const TetElems<RS>& el, uint2 
             if (j + u * LANES < o1.x) q[u] = ld_once(el.nb + j + u * LANES);
 #pragma unroll
         for (unsigned u = 0; u < U; u++)
-            if (j + u * LANES < o1.x) e[u] = xyz(COH ? s.x[q[u].idx] : ld_ro(s.x + q[u].idx));
+            if (j + u * LANES < o1.x) e[u] = xyz(COH ? s.x[plain(q[u].idx)] : ld_ro(s.x + plain(q[u].idx)));
 #pragma unroll
         for (unsigned u = 0; u < U; u++)
-            if (j + u * LANES < o1.x) {
-                e[u] = e[u] - xi;
-                P* d = es + (j + u * LANES - o0.x) * ST;
-                d[0] = e[u].x;
-                d[K * ST] = e[u].y;
-                d[2 * K * ST] = e[u].z;
-                const P w = (P)q[u].w;
-                B.g0 += w * e[u].x;
-                B.g1 += w * e[u].y;
-                B.g2 += w * e[u].z;
-            }
+            if (j + u * LANES < o1.x)
+                star_edge<P, RS, HT, ST>(q[u].w, e[u] - xi, es + (j + u * LANES - o0.x) * ST, K, B);
     }
     __syncwarp();
 #pragma unroll 2
     for (unsigned t = o0.y + lane; t < o1.y; t += LANES) {
         const StarTet<RS> q = ld_once(el.tet + t);
-        const uint32_t l = ld_once(el.loc + t);
-        const P* p1 = es + (l & 255u) * ST;
-        const P* p2 = es + (l >> 8 & 255u) * ST;
-        const P* p3 = es + (l >> 16) * ST;
-        const V3<P> e1 = mk3(p1[0], p1[K * ST], p1[2 * K * ST]);
-        const V3<P> f2 = mk3(p2[0], p2[K * ST], p2[2 * K * ST]) - e1;
-        const V3<P> f3 = mk3(p3[0], p3[K * ST], p3[2 * K * ST]) - e1;
-        const V3<P> N = cross3(f2, f3);
-        const P h = (P)q.a * ((P)q.r - dot3(e1, N));
-        B.g0 += h * N.x;
-        B.g1 += h * N.y;
-        B.g2 += h * N.z;
-        const HT nx = (HT)N.x, ny = (HT)N.y, nz = (HT)N.z, a = (HT)q.a;
-        const HT ax = a * nx, ay = a * ny, az = a * nz;
-        B.h00 += ax * nx;
-        B.h11 += ay * ny;
-        B.h22 += az * nz;
-        B.h01 += ax * ny;
-        B.h02 += ax * nz;
-        B.h12 += ay * nz;
+        star_tet<P, RS, HT, ST>(q, ld_once(el.loc + t), es, K, B);
     }
     __syncwarp();  // the slot is refilled for the lane group's next vertex
 }
@@ -361,25 +389,25 @@ AVBD_D void accumulate_star(const DevState<P>& s, const TetElems<RS>& el, uint2 
 // with GroundCollisionConstraintSolver): the Hessian k grad C grad C^T is always
 // added, the gradient is gated by the clamped multipliers.
 template <typename P, typename HT>
-AVBD_D void accumulate_ground(const DevState<P>& s, unsigned p, V3<P> xi, Block3<P, HT>& B) {
-    typename Vec4Of<P>::T k = s.gk[p], lam = s.glam[p], cp = s.gcp[p];
-    uint8_t gf = s.gflag[p];
+AVBD_D void accumulate_ground(typename Vec4Of<P>::T k, typename Vec4Of<P>::T lam, typename Vec4Of<P>::T cp, uint8_t gf,
+                              V3<P> xi, Block3<P, HT>& B) {
     P Cn = -xi.y, Ct = xi.x - cp.x, Cb = xi.z - cp.y;
     P cc = Cn - P(AVBD_ALPHA) * lam.w;
     P ln = k.x * cc + lam.x;
-    P lnp = ln > P(0) ? ln : P(0);
-    P lt = k.y * Ct + lam.y, lb = k.z * Cb + lam.z;
-    P mag = sqrt(lt * lt + lb * lb);
-    P mu = (gf & GF_USE_STATIC) ? cp.z : cp.w;
-    P mx = mu * lnp;
-    if (mag > mx) {
-        P sc = mx / (mag + P(1e-8));
-        lt = lt * sc;
-        lb = lb * sc;
+    if (ln > P(0)) {  // out of contact the Coulomb cone is a point: no force
+        P lt = k.y * Ct + lam.y, lb = k.z * Cb + lam.z;
+        P mag = sqrt(lt * lt + lb * lb);
+        P mu = (gf & GF_USE_STATIC) ? cp.z : cp.w;
+        P mx = mu * ln;
+        if (mag > mx) {
+            P sc = mx / (mag + P(1e-8));
+            lt = lt * sc;
+            lb = lb * sc;
+        }
+        B.g0 += lt;
+        B.g1 += -ln;
+        B.g2 += lb;
     }
-    B.g0 += lt;
-    B.g1 += -lnp;
-    B.g2 += lb;
     B.h00 += (HT)k.y;
     B.h11 += (HT)k.x;
     B.h22 += (HT)k.z;
@@ -402,6 +430,18 @@ AVBD_D void reduce_block(Block3<P, HT>& B) {
 }
 
 enum { MODE_SOLVE = 0, MODE_RESIDUAL = 1, MODE_DEBUG = 2, MODE_FEATURES = 3 };
+
+// FP64 solve of a block above the condition threshold; counted.
+template <typename P>
+__device__ __noinline__ V3<P> solve_block_d(Sym3<P> A, V3<P> rhs, unsigned long long* counters) {
+    double M[3][3] = {{(double)A.a00, (double)A.a01, (double)A.a02},
+                      {(double)A.a01, (double)A.a11, (double)A.a12},
+                      {(double)A.a02, (double)A.a12, (double)A.a22}};
+    double bb[3] = {(double)rhs.x, (double)rhs.y, (double)rhs.z}, xx[3];
+    lu_solve_d<3>(M, bb, xx);
+    atomicAdd(counters, 1ull);
+    return mk3<P>((P)xx[0], (P)xx[1], (P)xx[2]);
+}
 
 
 // Vertex block solve of one color slab: LANES threads per vertex stream the
@@ -427,7 +467,8 @@ struct SolveMinBlocks {
 // without or with damping.
 enum ElemForm { FORM_STAR = 0, FORM_REC = 1, FORM_DAMP = 2 };
 
-template <typename P, typename RS, typename HT, int LANES, int FORM, bool GROUND, int MODE, bool DYN, bool COH = false>
+template <typename P, typename RS, typename HT, int LANES, int FORM, bool GROUND, int MODE, bool DYN, bool COH = false,
+          int THREADS = 256>
 __device__ __forceinline__ void tet_vertex(const DevState<P>& s, const TetElems<RS>& el, unsigned begin,
                                            unsigned count, unsigned gi, unsigned lane, const Consts<P>& c,
                                            unsigned long long* counters, double* out, const SceneTol& T,
@@ -456,7 +497,7 @@ __device__ __forceinline__ void tet_vertex(const DevState<P>& s, const TetElems<
             o0 = el.star[p];
             o1 = el.star[p + 1];
         }
-        accumulate_star<P, RS, HT, LANES, COH>(s, el, o0, o1, lane, xi, es, B);
+        accumulate_star<P, RS, HT, LANES, COH, THREADS>(s, el, o0, o1, lane, xi, es, B);
         if (active && lane == 0) {
             const HT hd = (HT)el.hd[p];
             B.h00 += hd;
@@ -468,7 +509,8 @@ __device__ __forceinline__ void tet_vertex(const DevState<P>& s, const TetElems<
                 const uint32_t l = el.loc[t];
 #pragma unroll
                 for (int j = 0; j < 3; j++) {
-                    typename Vec4Of<P>::T vo = s.v[el.nb[o0.x + (l >> 8 * j & 255u)].idx];
+                    const unsigned o = el.nb[o0.x + (l >> 8 * j & 255u)].idx;
+                    typename Vec4Of<P>::T vo = s.v[o < s.n ? o : o - s.n];
                     fv0 += (float)vo.x;
                     fv1 += (float)vo.y;
                     fv2 += (float)vo.z;
@@ -538,7 +580,8 @@ __device__ __forceinline__ void tet_vertex(const DevState<P>& s, const TetElems<
     }
     double r2 = 0.0, mg2 = 0.0;
     if (active && lane == 0) {
-        if (GROUND && (fl & VF_GROUND)) accumulate_ground<P, HT>(s, p, xi, B);
+        if (GROUND && (fl & VF_GROUND))
+            accumulate_ground<P, HT>(s.gk[p], s.glam[p], s.gcp[p], s.gflag[p], xi, B);
         typename Vec4Of<P>::T y4 = s.y[p];
         P m = y4.w;
         P cm = m * c.inv_dt2;
@@ -553,16 +596,7 @@ __device__ __forceinline__ void tet_vertex(const DevState<P>& s, const TetElems<
                 else atomicAdd(T.r2 + T.scene[p], q);
             }
             V3<P> dx;
-            P kappa = solve_sym3<P>(A, rhs, dx);
-            if (!(kappa <= c.kappa_max)) {
-                double M[3][3] = {{(double)A.a00, (double)A.a01, (double)A.a02},
-                                  {(double)A.a01, (double)A.a11, (double)A.a12},
-                                  {(double)A.a02, (double)A.a12, (double)A.a22}};
-                double bb[3] = {(double)rhs.x, (double)rhs.y, (double)rhs.z}, xx[3];
-                lu_solve_d<3>(M, bb, xx);
-                dx = mk3<P>((P)xx[0], (P)xx[1], (P)xx[2]);
-                atomicAdd(counters, 1ull);
-            }
+            if (!solve_sym3<P>(A, rhs, c.kappa_max, dx)) dx = solve_block_d(A, rhs, counters);
             typename Vec4Of<P>::T o = make4<P>(xi + dx, P(0));
             // an intra-color conflict buffers the update (VBDSolver.hpp:505-509)
             if (DYN && s.conflicted[p]) s.buffered[p] = o;
@@ -572,7 +606,7 @@ __device__ __forceinline__ void tet_vertex(const DevState<P>& s, const TetElems<
             Sym3<P> A{cm + (P)B.h00, cm + (P)B.h11, cm + (P)B.h22, (P)B.h01, (P)B.h02, (P)B.h12};
             V3<P> rhs = mk3<P>(-cm * d.x - B.g0, -cm * d.y - B.g1, -cm * d.z - B.g2);
             V3<P> dx;
-            solve_sym3<P>(A, rhs, dx);
+            solve_sym3<P>(A, rhs, c.kappa_max, dx);
             const float sc = 1.0f / (float)(c.g * c.dt * c.dt);
             const float h = (float)c.dt, icm = 1.0f / (float)cm;
             typename Vec4Of<P>::T v4 = s.v[p];
@@ -731,53 +765,54 @@ __global__ void __launch_bounds__(256, (SolveMinBlocks<P, RS, FORM>::value)) k_s
 // up (avbd_debug_set_wait_limit lowers it so that tests can make it run out).
 __device__ uint32_t g_sweep_wait_polls = AVBD_DEFAULT_WAIT_POLLS;
 
-AVBD_D bool grid_barrier(unsigned* sync, int* err) {
-    return grid_barrier_bounded(sync, err, *(volatile uint32_t*)&g_sweep_wait_polls);
-}
-
-// The whole sweep of a run-to-tolerance iteration in one cooperative launch:
-// for each color in turn the blocks draw its pieces from a shared ticket
-// counter (dynamic, so uneven pieces balance), then meet at a grid barrier
-// before the next color reads the positions this one wrote.  In color k each
-// block draws exactly one ticket past the color's pieces, so color k's tickets
-// start at sum over earlier colors of (pieces + blocks).  sync: [ticket,
-// arrivals, generation], zeroed before each launch.
-template <typename P, typename RS, typename HT, int LANES, int FORM, bool GROUND>
-__global__ void __launch_bounds__(256, (SolveMinBlocks<P, RS, FORM>::value))
-    k_sweep_persistent(DevState<P> s, TetElems<RS> el, Consts<P> c, unsigned long long* counters,
-                       SceneTol T, const uint4* __restrict__ ranges, const unsigned* __restrict__ color_off,
-                       unsigned ncolors, unsigned* sync) {
-    __shared__ unsigned ticket;
-    unsigned base = 0;
-    for (unsigned col = 0; col < ncolors; col++) {
-        const unsigned r0 = color_off[col], np = color_off[col + 1] - r0;
-        for (;;) {
-            __syncthreads();  // every thread has read the previous ticket
-            if (threadIdx.x == 0) ticket = atomicAdd(sync, 1u) - base;
-            __syncthreads();
-            const unsigned t = ticket;
-            if (t >= np) break;
-            solve_piece<P, RS, HT, LANES, FORM, GROUND, MODE_SOLVE, false, true>(s, el, ranges[r0 + t], c,
-                                                                                 counters, nullptr, T, nullptr,
-                                                                                  nullptr);
-        }
-        base += np + gridDim.x;
-        if (col + 1 < ncolors && !grid_barrier(sync + 1, s.err)) return;
-    }
-}
-
-// Chebyshev acceleration of every particle fused with the ground-contact dual
-// update that follows it (CollisionConstraintEnergySolver::updateAfterIteration);
-// a ground energy reads only its own particle, so the fusion is exact.
+// Dual update of a ground contact at the accelerated position xn
+// (CollisionConstraintEnergySolver::updateAfterIteration); true when the
+// penalties grew, which they do only in contact: elsewhere k is not stored back.
 template <typename R>
-__global__ void __launch_bounds__(256) k_chebyshev_dual(DevState<R> s, R omega, unsigned it, SceneTol T) {
-    unsigned p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= s.n) return;
-    uint8_t fl = s.flags[p];
-    if (fl & VF_ORIENTED) return;
-    if (T.active && !T.active[T.scene[p]]) return;
-    if (T.omega) omega = (R)*T.omega;
-    if (T.it) it = *T.it;
+AVBD_D bool ground_dual(typename Vec4Of<R>::T& k, typename Vec4Of<R>::T& lam, typename Vec4Of<R>::T cp, uint8_t& gf,
+                        V3<R> xn) {
+    R Cn = -xn.y, Ct = xn.x - cp.x, Cb = xn.z - cp.y;
+    R cc = Cn - R(AVBD_ALPHA) * lam.w;
+    R ln = k.x * cc + lam.x;
+    R lt = k.y * Ct + lam.y;
+    R lb = k.z * Cb + lam.z;
+    bool k_grows = ln > R(0);
+    bool st = gf & GF_USE_STATIC;
+    if (!k_grows && !st) {  // out of contact, sliding coefficient: the cone is a point
+        lam.x = R(0);
+        lam.y = R(0) * lt;
+        lam.z = R(0) * lb;
+        gf &= ~GF_UNCLAMPED;
+        return false;
+    }
+    if (ln > R(0)) k.x += R(AVBD_BETA) * fabs(cc);
+    lam.x = ln > R(0) ? ln : R(0);
+    R mag = sqrt(lt * lt + lb * lb);
+    R mx = (st ? cp.z : cp.w) * lam.x;
+    if (mag < mx) {
+        k_grows = true;
+        k.y += R(AVBD_BETA) * fabs(Ct);
+        k.z += R(AVBD_BETA) * fabs(Cb);
+        lam.y = lt;
+        lam.z = lb;
+        gf |= GF_UNCLAMPED;
+    } else {
+        if (st) {
+            gf &= ~GF_USE_STATIC;
+            mx = cp.w * ln;
+        }
+        lam.y = lt / (mag + R(1e-8)) * mx;
+        lam.z = lb / (mag + R(1e-8)) * mx;
+        gf &= ~GF_UNCLAMPED;
+    }
+    return k_grows;
+}
+
+// Chebyshev acceleration of a vertex fused with the ground-contact dual
+// update that follows it; a ground energy reads only its own particle, so the
+// fusion is exact.
+template <typename R>
+AVBD_D void chebyshev_dual_vertex(const DevState<R>& s, unsigned p, uint8_t fl, R omega, unsigned it) {
     // o_k = omega (x - o_(k-2)) + o_(k-2); o_k replaces o_(k-2) in its buffer
     typename Vec4Of<R>::T* h = (it & 1u) ? s.xll : s.xl;
     typename Vec4Of<R>::T x4 = s.x[p], ll4 = h[p];
@@ -789,37 +824,687 @@ __global__ void __launch_bounds__(256) k_chebyshev_dual(DevState<R> s, R omega, 
     if (fl & VF_GROUND) {
         typename Vec4Of<R>::T k = s.gk[p], lam = s.glam[p], cp = s.gcp[p];
         uint8_t gf = s.gflag[p];
-        R Cn = -xn.y, Ct = xn.x - cp.x, Cb = xn.z - cp.y;
-        R cc = Cn - R(AVBD_ALPHA) * lam.w;
-        R ln = k.x * cc + lam.x;
-        R lt = k.y * Ct + lam.y;
-        R lb = k.z * Cb + lam.z;
-        // the penalties grow only in contact: elsewhere k is not stored back
-        bool k_grows = ln > R(0);
-        if (ln > R(0)) k.x += R(AVBD_BETA) * fabs(cc);
-        lam.x = ln > R(0) ? ln : R(0);
-        R mag = sqrt(lt * lt + lb * lb);
-        bool st = gf & GF_USE_STATIC;
-        R mx = (st ? cp.z : cp.w) * lam.x;
-        if (mag < mx) {
-            k_grows = true;
-            k.y += R(AVBD_BETA) * fabs(Ct);
-            k.z += R(AVBD_BETA) * fabs(Cb);
-            lam.y = lt;
-            lam.z = lb;
-            gf |= GF_UNCLAMPED;
-        } else {
-            if (st) {
-                gf &= ~GF_USE_STATIC;
-                mx = cp.w * ln;
-            }
-            lam.y = lt / (mag + R(1e-8)) * mx;
-            lam.z = lb / (mag + R(1e-8)) * mx;
-            gf &= ~GF_UNCLAMPED;
-        }
-        if (k_grows) s.gk[p] = k;
+        if (ground_dual<R>(k, lam, cp, gf, xn)) s.gk[p] = k;
         s.glam[p] = lam;
         s.gflag[p] = gf;
+    }
+}
+
+template <typename R>
+__global__ void __launch_bounds__(256) k_chebyshev_dual(DevState<R> s, R omega, unsigned it, SceneTol T) {
+    unsigned p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= s.n) return;
+    uint8_t fl = s.flags[p];
+    if (fl & VF_ORIENTED) return;
+    if (T.active && !T.active[T.scene[p]]) return;
+    if (T.omega) omega = (R)*T.omega;
+    if (T.it) it = *T.it;
+    chebyshev_dual_vertex<R>(s, p, fl, omega, it);
+}
+
+// Barrier over the blocks of an iteration launch.  sync[0] counts arrivals and
+// only grows: the barrier numbered b (from 1) opens when it reaches b gridDim.x,
+// so one word serves arrival and release.  sync[1] is set by a block whose
+// polls ran out; the others see it while they poll, and every block leaves.
+AVBD_D bool iterate_barrier(unsigned* sync, unsigned number, int* err) {
+    __shared__ int ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const unsigned target = number * gridDim.x;
+        int good = 1;
+        // the block's writes (ordered before by the block barrier) are released
+        // with the arrival, the others' acquired with the poll that sees it
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(sync) : "memory");
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(sync) : "memory");
+        const unsigned limit = g_sweep_wait_polls;
+        for (unsigned polls = 0; (int)(v - target) < 0; polls++) {
+            if (polls >= limit || ((polls & 63u) == 63u && *(volatile unsigned*)(sync + 1) != 0)) {
+                good = 0;
+                break;
+            }
+            if (polls > 256) __nanosleep(100);
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(sync) : "memory");
+        }
+        if (!good) {
+            atomicExch(sync + 1, 1u);
+            atomicCAS(err, 0, (int)AVBD_ERR_BARRIER_TIMEOUT);
+        }
+        ok = good;
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+// Threads of an iteration block (one per SM): the prefetching sweeps of the
+// star form with a double state take 168 registers (with 128 they spilled and
+// a batch of 24 scenes ran 10.3 instead of 7.3 ms a pass), the others 128.
+template <typename P, int FORM, int LANES = 8>
+struct IterThreads {
+    static constexpr int value = FORM == FORM_STAR && sizeof(P) == 8 && LANES > 2 ? 384 : 512;
+};
+
+// A piece of 32 / LANES vertices of the star form whose constant data are on
+// their way into registers: this thread's entries of the first rounds (16
+// neighbours and 24 or 32 tets a vertex; the rest is read when its turn comes).
+template <typename RS, int LANES>
+struct StarPiece {
+    static constexpr int UN = 16 / LANES, UT = LANES == 16 ? 2 : 24 / LANES;
+    uint4 h;  // TetElems::piece
+    StarNb<RS> nb[UN];
+    StarTet<RS> tet[UT];
+    uint32_t loc[UT];
+
+    AVBD_D void lists(const TetElems<RS>& el, unsigned wl) {
+#pragma unroll
+        for (int u = 0; u < UN; u++)
+            if (u < (int)h.y) nb[u] = ld_once(el.pnb + h.x + u * 32 + wl);
+#pragma unroll
+        for (int u = 0; u < UT; u++)
+            if (u < (int)h.w) {
+                tet[u] = ld_once(el.ptet + h.z + u * 32 + wl);
+                loc[u] = ld_once(el.ploc + h.z + u * 32 + wl);
+            }
+    }
+};
+
+// Staging rows of k_iterate: whole rounds of LANES neighbours.
+AVBD_HD unsigned star_rows(unsigned max_nb, unsigned lanes) { return (max_nb + lanes - 1) / lanes * lanes; }
+
+// Arguments of an iteration launch.
+struct IterArgs {
+    const uint4* slabs;       // per color: first internal vertex, solved positional vertices, first piece
+    unsigned ncolors;
+    const double* omega;      // Chebyshev weights by iteration
+    unsigned it0, n;          // first iteration, iterations at most
+    bool sweep_only;          // the solves alone (lane choice): histories and multipliers untouched
+    unsigned* sync;           // barrier, zeroed before
+    // run to tolerance
+    unsigned max_it;          // iteration cap of the step
+    uint32_t* it_dev;         // loop of a graph: first iteration from device memory, advanced at the end
+    double tol, g2;
+    const double* m2;
+    uint8_t *active, *cand;
+    uint32_t* iters;
+    double *r2, *ex, *rin;    // r2: 3 buffers of S by iteration, ex: 2 by residual pass (k_iterate)
+    unsigned S;
+    unsigned long long* scene_iterations;
+    unsigned long long* maxr;
+    int* n_active;
+    cudaGraphConditionalHandle loop;  // continue condition of the graph's loop (has_loop)
+    bool has_loop;
+    unsigned long long* launches;
+};
+
+AVBD_D double scene_R(double r2, double mg2) { return mg2 > 0 ? sqrt(r2) / sqrt(mg2) : sqrt(r2); }
+
+AVBD_D unsigned long long ord_enc64(double d) {
+    unsigned long long u = (unsigned long long)__double_as_longlong(d);
+    return (u >> 63) ? ~u : (u | 0x8000000000000000ull);
+}
+
+// Residual terms of a warp's consecutive pieces, one atomic per scene run.
+struct SceneSum {
+    double* sums;
+    unsigned run = 0xFFFFFFFFu;
+    double racc = 0.0;
+    AVBD_D SceneSum(double* s) : sums(s) {}
+    AVBD_D void flush() {
+        double t = racc;
+#pragma unroll
+        for (int m = 16; m >= 1; m >>= 1) t += __shfl_xor_sync(0xffffffffu, t, m);
+        if ((threadIdx.x & 31u) == 0 && run != 0xFFFFFFFFu) atomicAdd(sums + run, t);
+        run = 0xFFFFFFFFu;
+        racc = 0.0;
+    }
+    AVBD_D void add(unsigned scene, double term) {
+        const unsigned sc0 = __shfl_sync(0xffffffffu, scene, 0);
+        if (__all_sync(0xffffffffu, scene == sc0)) {
+            if (sc0 != run) {
+                flush();
+                run = sc0;
+            }
+            racc += term;
+        } else if (term != 0.0) {
+            atomicAdd(sums + scene, term);
+        }
+    }
+};
+
+// Scenes as bits in shared memory: every block keeps its own copy of which
+// scenes iterate and which are candidates, computed from the same sums.
+struct SceneBits {
+    uint32_t* w;
+    AVBD_D bool get(unsigned s) const { return w[s >> 5] >> (s & 31u) & 1u; }
+};
+
+// The solved vertices [begin, begin + count) of a color in MODE, a warp taking
+// 32 / LANES consecutive ones at a time (see k_iterate).  TOL: vertices of
+// scenes outside the gate are skipped; the residual terms go to the scenes' sums.
+template <typename P, typename RS, typename HT, int LANES, int FORM, bool GROUND, bool TOL, int MODE>
+AVBD_D void color_phase(const DevState<P>& s, const TetElems<RS>& el, const Consts<P>& c,
+                        unsigned long long* counters, const uint32_t* scene, unsigned begin, unsigned count,
+                        SceneBits gate, double* sums, bool spread) {
+    constexpr int THREADS = IterThreads<P, FORM, LANES>::value;
+    constexpr unsigned WARPS = THREADS / 32, V = 32 / LANES;
+    const unsigned warp = threadIdx.x >> 5, wl = threadIdx.x & 31u, lane = wl % LANES;
+    const unsigned B = gridDim.x, b = blockIdx.x;
+    const unsigned nch = (count + V - 1) / V;
+    const unsigned per = (nch + B - 1) / B;
+    unsigned k = spread ? b * WARPS + warp : b * per + warp;
+    const unsigned end = spread ? nch : min(nch, (b + 1) * per);
+    const unsigned step = spread ? B * WARPS : WARPS;
+    SceneSum sum(sums);
+    SceneTol TB;
+    if constexpr (TOL) {
+        TB.r2 = MODE == MODE_SOLVE ? sums : nullptr;
+        TB.ex = MODE == MODE_RESIDUAL ? sums : nullptr;
+        TB.scene = scene;
+    }
+    for (; k < end; k += step) {
+        unsigned gi = k * V + wl / LANES;
+        unsigned sc = 0;
+        if constexpr (TOL) {
+            sc = scene[begin + min(gi, count - 1)];
+            if (!gate.get(sc)) gi = count;
+            if (!__any_sync(0xffffffffu, gi < count)) continue;
+        }
+        double acc = 0.0;
+        tet_vertex<P, RS, HT, LANES, FORM, GROUND, MODE, false, true, THREADS>(
+            s, el, begin, count, gi, lane, c, counters, nullptr, TB, nullptr, nullptr, TOL ? &acc : nullptr);
+        if constexpr (TOL) {
+            __syncwarp();
+            sum.add(sc, acc);
+        }
+    }
+    if constexpr (TOL) sum.flush();
+}
+
+// The exact residual of the candidate scenes: rare, and kept out of line so
+// that it takes no registers from the sweeps.
+template <typename P, typename RS, typename HT, int LANES, int FORM, bool GROUND>
+__device__ __noinline__ void residual_phase(const DevState<P>& s, const TetElems<RS>& el, const Consts<P>& c,
+                                            const uint32_t* scene, const IterArgs& A, SceneBits cand, double* ex) {
+    for (unsigned col = 0; col < A.ncolors; col++) {
+        const uint4 sl = A.slabs[col];
+        if (sl.y)
+            color_phase<P, RS, HT, LANES, FORM, GROUND, true, MODE_RESIDUAL>(s, el, c, nullptr, scene, sl.x, sl.y,
+                                                                             cand, ex, true);
+    }
+}
+
+// After a sweep: an iterating scene whose in-sweep residual is at the
+// tolerance becomes a candidate.  Returns the number of candidates (uniform
+// over the block).
+__device__ __noinline__ unsigned iterate_candidates(const IterArgs& A, SceneBits on, SceneBits cand, const double* r2,
+                                                    unsigned* red) {
+    for (unsigned i = threadIdx.x; i < (A.S + 31) / 32; i += blockDim.x) cand.w[i] = 0;
+    if (threadIdx.x == 0) *red = 0;
+    __syncthreads();
+    const double t2 = A.tol * A.tol * A.g2 * (1 + 1e-9);  // a cheap bound first, then the exact comparison
+    unsigned n = 0;
+    for (unsigned q = threadIdx.x; q < A.S; q += blockDim.x)
+        if (on.get(q)) {
+            const double r = __ldcg(r2 + q), m = A.m2[q];
+            if ((r <= t2 * m || !(m > 0)) && scene_R(r, m * A.g2) <= A.tol) {
+                atomicOr(cand.w + (q >> 5), 1u << (q & 31u));
+                n++;
+            }
+        }
+    if (n) atomicAdd(red, n);
+    __syncthreads();
+    const unsigned total = *red;
+    __syncthreads();  // red may be reused
+    return total;
+}
+
+// Stop decision: candidates whose exact residual is at the tolerance stop; at
+// the iteration cap every scene does.  The recording block also stores the
+// scenes' iteration counts, the step's largest final residual (maxr[0]: the
+// exact one where it was evaluated in the stopping iteration, else the
+// in-sweep one of a capped scene) and the number of capped scenes (maxr[1]).
+// Returns the number of scenes that stopped.
+__device__ __noinline__ unsigned iterate_stop(const IterArgs& A, SceneBits on, SceneBits cand, const double* r2,
+                                              const double* ex, unsigned iters, bool record, unsigned* red) {
+    if (threadIdx.x == 0) *red = 0;
+    __syncthreads();
+    const bool cap = iters >= A.max_it;
+    unsigned n = 0;
+    for (unsigned q = threadIdx.x; q < A.S; q += blockDim.x) {
+        if (!on.get(q)) continue;
+        const bool cd = cand.get(q);
+        if (!cd && !cap) continue;
+        const double R = scene_R(__ldcg((cd ? ex : r2) + q), A.m2[q] * A.g2);
+        const bool met = cd && R <= A.tol;
+        if (!met && !cap) continue;
+        n++;
+        atomicAnd(on.w + (q >> 5), ~(1u << (q & 31u)));
+        if (record) {
+            A.iters[q] = iters;
+            atomicMax(A.maxr, ord_enc64(R));
+            if (!met) atomicAdd(A.maxr + 1, 1ull);
+        }
+    }
+    if (n) atomicAdd(red, n);
+    __syncthreads();
+    const unsigned total = *red;
+    __syncthreads();
+    return total;
+}
+
+// 32-byte accesses of a vertex record of four doubles (float4 is one already).
+// Loads are coherent: other blocks of the launch write the positions.
+AVBD_D float4 ld_vec(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+AVBD_D double4a ld_vec(const double4a* p) {
+    double4a v;
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
+AVBD_D void st_vec(float4* p, float4 v) { *p = v; }
+AVBD_D void st_vec(double4a* p, double4a v) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v.x), "d"(v.y), "d"(v.z), "d"(v.w) : "memory");
+}
+
+// What follows the accumulated block of a vertex in k_iterate: the 3x3 solve,
+// the solved position for the later colors, the accelerated one and the
+// history for the next iteration.  Returns the accelerated position.
+template <typename P, typename HT>
+AVBD_D V3<P> block_rhs(const Block3<P, HT>& B, V3<P> xi, typename Vec4Of<P>::T y4, P inv_dt2) {
+    const P cm = y4.w * inv_dt2;
+    const V3<P> d = xi - xyz(y4);
+    return mk3<P>(-cm * d.x - B.g0, -cm * d.y - B.g1, -cm * d.z - B.g2);
+}
+template <typename P>
+AVBD_D double sum_sq(V3<P> v) {
+    return (double)v.x * (double)v.x + (double)v.y * (double)v.y + (double)v.z * (double)v.z;
+}
+template <typename P, typename HT>
+AVBD_D V3<P> finish_vertex(const DevState<P>& s, const Consts<P>& c, const IterArgs& A, unsigned long long* counters,
+                           const Block3<P, HT>& B, V3<P> rhs, V3<P> xi, unsigned p, P mass, V3<P> h, P om,
+                           typename Vec4Of<P>::T* hist) {
+    const P cm = mass * c.inv_dt2;
+    Sym3<P> M{cm + (P)B.h00, cm + (P)B.h11, cm + (P)B.h22, (P)B.h01, (P)B.h02, (P)B.h12};
+    V3<P> dx;
+    if (!solve_sym3<P>(M, rhs, c.kappa_max, dx)) dx = solve_block_d(M, rhs, counters);
+    const V3<P> xs = xi + dx;
+    st_vec(s.x + s.n + p, make4<P>(xs, P(0)));
+    const V3<P> xa = A.sweep_only ? xs : om * (xs - h) + h;
+    const typename Vec4Of<P>::T o = make4<P>(xa, P(0));
+    st_vec(s.x + p, o);
+    if (!A.sweep_only) st_vec(hist + p, o);
+    return xa;
+}
+// The ground contact's duals at the accelerated position; what does not change
+// (most vertices are out of contact) is not stored back.
+template <typename P>
+AVBD_D void finish_ground(const DevState<P>& s, unsigned p, typename Vec4Of<P>::T k, typename Vec4Of<P>::T lam,
+                          typename Vec4Of<P>::T cp, uint8_t gf, V3<P> xa) {
+    const uint8_t g0 = gf;
+    const V3<P> l0 = xyz(lam);
+    if (ground_dual<P>(k, lam, cp, gf, xa)) st_vec(s.gk + p, k);
+    if (l0.x != lam.x || l0.y != lam.y || l0.z != lam.z) st_vec(s.glam + p, lam);
+    if (gf != g0) s.gflag[p] = gf;
+}
+
+// The pieces of one color at one thread a vertex: no lane idles in the solve
+// and nothing is reduced, so a vertex takes a third of the instructions of 4
+// threads; for colors that fill the SMs' warps this way.
+template <typename P, typename RS, bool GROUND, bool TOL>
+AVBD_D void color_wide(const DevState<P>& s, const TetElems<RS>& el, const Consts<P>& c, const IterArgs& A,
+                       unsigned long long* counters, const uint32_t* scene, uint4 sl, SceneBits on, bool spread, P om,
+                       typename Vec4Of<P>::T* hist, double* r2, P* es) {
+    using V4 = typename Vec4Of<P>::T;
+    constexpr int THREADS = IterThreads<P, FORM_STAR, 1>::value;
+    constexpr unsigned WARPS = THREADS / 32, ST = StarStage<P, 1, THREADS>::STRIDE, U = 4;
+    const unsigned warp = threadIdx.x >> 5, wl = threadIdx.x & 31u, K = el.max_nb;
+    const unsigned B = gridDim.x, b = blockIdx.x;
+    const unsigned nch = (sl.y + 31) / 32, per = (nch + B - 1) / B;
+    const unsigned end = spread ? nch : min(nch, (b + 1) * per), step = spread ? B * WARPS : WARPS;
+    SceneSum sum(r2);
+    for (unsigned k = spread ? b * WARPS + warp : b * per + warp; k < end; k += step) {
+        const unsigned gi = k * 32 + wl, p = sl.x + min(gi, sl.y - 1);
+        bool live = gi < sl.y;
+        unsigned sc = 0;
+        if constexpr (TOL) {
+            sc = scene[p];
+            live = live && on.get(sc);
+            if (!__any_sync(0xffffffffu, live)) continue;
+        }
+        const uint4 h = el.piece[sl.z + k];
+        const V3<P> xi = xyz(ld_vec(s.x + p));
+        Block3<P, P> Bk;
+        for (unsigned u0 = 0; u0 < h.y; u0 += U) {
+            StarNb<RS> q[U];
+            V3<P> xo[U];
+#pragma unroll
+            for (unsigned u = 0; u < U; u++)
+                if (u0 + u < h.y) q[u] = ld_once(el.pnb + h.x + (u0 + u) * 32 + wl);
+#pragma unroll
+            for (unsigned u = 0; u < U; u++)
+                if (u0 + u < h.y) xo[u] = xyz(ld_vec(s.x + q[u].idx));
+#pragma unroll
+            for (unsigned u = 0; u < U; u++)
+                if (u0 + u < h.y) star_edge<P, RS, P, ST>(q[u].w, xo[u] - xi, es + (u0 + u) * ST, K, Bk);
+        }
+        StarTet<RS> q[U];
+        uint32_t l[U];
+#pragma unroll
+        for (unsigned u = 0; u < U; u++)
+            if (u < h.w) {
+                q[u] = ld_once(el.ptet + h.z + u * 32 + wl);
+                l[u] = ld_once(el.ploc + h.z + u * 32 + wl);
+            }
+        for (unsigned u0 = 0; u0 < h.w; u0 += U) {
+#pragma unroll
+            for (unsigned u = 0; u < U; u++)
+                if (u0 + u < h.w) {
+                    star_tet<P, RS, P, ST>(q[u], l[u], es, K, Bk);
+                    if (u0 + u + U < h.w) {  // a group ahead
+                        q[u] = ld_once(el.ptet + h.z + (u0 + u + U) * 32 + wl);
+                        l[u] = ld_once(el.ploc + h.z + (u0 + u + U) * 32 + wl);
+                    }
+                }
+        }
+        const P hd = (P)el.hd[p];
+        Bk.h00 += hd;
+        Bk.h11 += hd;
+        Bk.h22 += hd;
+        V4 gk, gl, cp;
+        uint8_t fl = 0, gf = 0;
+        if constexpr (GROUND) {
+            fl = live ? s.flags[p] : (uint8_t)0;
+            cp = ld_vec(s.gcp + p);
+            gk = ld_vec(s.gk + p);
+            gl = ld_vec(s.glam + p);
+            gf = s.gflag[p];
+            if (fl & VF_GROUND) accumulate_ground<P, P>(gk, gl, cp, gf, xi, Bk);
+        }
+        double acc = 0.0;
+        if (live) {
+            const V4 y4 = ld_vec(s.y + p);
+            const V3<P> rhs = block_rhs(Bk, xi, y4, c.inv_dt2);
+            if (TOL) acc = sum_sq(rhs);
+            const V3<P> xa = finish_vertex<P, P>(s, c, A, counters, Bk, rhs, xi, p, y4.w, xyz(ld_vec(hist + p)), om, hist);
+            if constexpr (GROUND)
+                if ((fl & VF_GROUND) && !A.sweep_only) finish_ground<P>(s, p, gk, gl, cp, gf, xa);
+        }
+        if constexpr (TOL) {
+            __syncwarp();
+            sum.add(sc, acc);
+        }
+    }
+    if constexpr (TOL) sum.flush();
+}
+
+// The iterations of a step in one cooperative launch of a block per SM, with a
+// grid barrier between colors (about 1 us, against about 3 us for a launch of
+// a graph).  Small scenes are bounded by these phases, not by their bytes: what
+// follows a barrier is a chain of round trips to L2 and of FP64 latencies.
+//
+// Star form: the Chebyshev acceleration and the ground duals need only the
+// vertex's own solved position, so they follow its solve instead of taking a
+// pass and a barrier of their own: the solved position goes to the second half
+// of x, where the later colors of this iteration read it (tagged ids, StarNb),
+// the accelerated one to x itself, for the next iteration.  At 4 or more lanes
+// (PIPE) a warp's pieces (32 / LANES consecutive vertices) run as one sequence
+// over the colors: the next piece's header is loaded while the current one
+// gathers, its lists while the current one reduces and solves -- also across
+// the barrier, since they are constant -- so a phase is one round trip for the
+// positions and the arithmetic.  Measured: a barrier with the release and the
+// first read behind it 1.9 us, a color of an 8^3 cube 2.9 us (4.6 with the
+// loads of the lists behind the barrier, 3.7 as a launch of a graph).
+// Records, and the star form at 2 lanes (AVBD_LANES): every color is a pass of
+// tet_vertex and the acceleration another.
+//
+// While every scene iterates, the blocks own contiguous parts of a color
+// (neighbouring vertices share their neighbours in L1); once scenes have
+// stopped the pieces are dealt round robin, which spreads the remaining scenes
+// over the SMs.  TOL: scenes run to their residual tolerance.  Every block
+// evaluates the decisions itself from the scenes' sums (3 buffers by
+// iteration, so that none is cleared while another block reads it); only an
+// iteration with candidates pays for the exact residual and a barrier.
+template <typename P, typename RS, typename HT, int LANES, int FORM, bool GROUND, bool TOL>
+__global__ void __launch_bounds__((IterThreads<P, FORM, LANES>::value), 1)
+    k_iterate(const __grid_constant__ DevState<P> s, const __grid_constant__ TetElems<RS> el,
+              const __grid_constant__ Consts<P> c, unsigned long long* counters, const uint32_t* scene,
+              const __grid_constant__ IterArgs A) {
+    using V4 = typename Vec4Of<P>::T;
+    constexpr int THREADS = IterThreads<P, FORM, LANES>::value;
+    constexpr unsigned WARPS = THREADS / 32, V = 32 / LANES;
+    constexpr bool STAR = FORM == FORM_STAR && LANES != 2;  // accelerates as it solves
+    constexpr bool PIPE = STAR && LANES > 1;
+    constexpr unsigned ST = StarStage<P, LANES, THREADS>::STRIDE;
+    using Piece = StarPiece<RS, PIPE ? LANES : 4>;
+    __shared__ unsigned red;
+    extern __shared__ __align__(16) unsigned char stage[];
+    const unsigned warp = threadIdx.x >> 5, wl = threadIdx.x & 31u, lane = wl % LANES;
+    const unsigned B = gridDim.x, b = blockIdx.x;
+    const unsigned K = PIPE ? star_rows(el.max_nb, LANES) : el.max_nb;
+    P* const es = reinterpret_cast<P*>(stage) + threadIdx.x / LANES;
+    unsigned bar = 0;
+    const unsigned first = TOL && A.it_dev ? *A.it_dev : A.it0;
+    unsigned last = first + A.n;
+    if (TOL && last > A.max_it) last = A.max_it;
+    unsigned it = first, na = 0, exn = 0;
+    unsigned done_it = 0;  // scene-iterations of this launch
+    SceneBits on{nullptr}, cand{nullptr};
+    if constexpr (TOL) {
+        // a block that leaves at a barrier ends the graph's loop: the condition
+        // is only set again once the launch has run to its end
+        if (A.has_loop && b == B - 1 && threadIdx.x == 0) cudaGraphSetConditional(A.loop, 0u);
+        on.w = reinterpret_cast<uint32_t*>(stage + (FORM == FORM_STAR ? 3 * K * ST * sizeof(P) : 0));
+        cand.w = on.w + (A.S + 31) / 32;
+        for (unsigned q0 = warp * 32; q0 < A.S; q0 += THREADS) {
+            const unsigned m = __ballot_sync(0xffffffffu, q0 + wl < A.S && A.active[min(q0 + wl, A.S - 1)]);
+            if (wl == 0) on.w[q0 >> 5] = m;
+        }
+        na = (unsigned)*A.n_active;
+        // the first residual pass adds to buffer 0 (a barrier away)
+        if (b == B - 1)
+            for (unsigned q = threadIdx.x; q < A.S; q += THREADS) A.ex[q] = 0;
+        __syncthreads();
+    }
+
+    Piece cur;
+    // `cur` is piece ck of phase cphase; this thread's vertex of it, solved when clive
+    unsigned ck = 0, cend = 0, cstep = 0, cbegin = 0, ccount = 1, cpiece = 0, cphase = 0, cp = 0;
+    bool clive = false;
+    auto next_color = [&](unsigned col) {  // the next color with vertices, cyclic
+        do col = col + 1 < A.ncolors ? col + 1 : 0;
+        while (A.slabs[col].y == 0);
+        return col;
+    };
+    auto load_header = [&](bool spread) {  // of piece ck; stopped scenes' pieces are passed over
+        for (; ck < cend; ck += cstep) {
+            const unsigned gi = ck * V + wl / LANES;
+            clive = gi < ccount;
+            cp = cbegin + min(gi, ccount - 1);
+            if constexpr (TOL)
+                if (spread) {
+                    clive = clive && on.get(scene[cp]);
+                    if (!__any_sync(0xffffffffu, clive)) continue;
+                }
+            cur.h = el.piece[cpiece + ck];
+            return;
+        }
+    };
+    auto start_color = [&](unsigned col, bool spread, unsigned phase) {
+        const uint4 sl = A.slabs[col];
+        const unsigned nch = (sl.y + V - 1) / V, per = (nch + B - 1) / B;
+        cbegin = sl.x;
+        ccount = sl.y;
+        cpiece = sl.z;
+        cphase = phase;
+        ck = spread ? b * WARPS + warp : b * per + warp;
+        cend = spread ? nch : min(nch, (b + 1) * per);
+        cstep = spread ? B * WARPS : WARPS;
+        load_header(spread);
+    };
+
+    bool spread = TOL && na < A.S;
+    unsigned phase = 0;
+    const unsigned color0 = next_color(A.ncolors - 1);
+    if constexpr (PIPE) {
+        start_color(color0, spread, phase);
+        if (ck < cend) cur.lists(el, wl);
+    }
+    for (; it < last && (!TOL || na > 0); it++) {
+        double* const r2 = TOL ? A.r2 + (size_t)(it % 3u) * A.S : nullptr;
+        if constexpr (TOL) done_it += na;
+        const P om = A.sweep_only ? P(1) : (P)A.omega[it];
+        if constexpr (STAR && !PIPE) {
+            for (unsigned col = 0; col < A.ncolors; col++) {
+                const uint4 sl = A.slabs[col];
+                if (sl.y == 0) continue;
+                color_wide<P, RS, GROUND, TOL>(s, el, c, A, counters, scene, sl, on, spread, om, (it & 1u) ? s.xll : s.xl,
+                                               r2, es);
+                if (!iterate_barrier(A.sync, ++bar, s.err)) return;
+            }
+        } else if constexpr (PIPE) {
+            V4* const hist = (it & 1u) ? s.xll : s.xl;
+            SceneSum sum(r2);
+            for (unsigned col = 0; col < A.ncolors; col++) {
+                if (A.slabs[col].y == 0) continue;
+                while (cphase == phase && ck < cend) {
+                    const unsigned p = cp;
+                    const bool live = clive;
+                    const uint4 h = cur.h;
+                    Block3<P, HT> Bk;
+                    // positions, then what lanes 0 (inertia, history) and 1 (ground contact) add
+                    const V3<P> xi = xyz(ld_vec(s.x + p));
+                    V3<P> xo[Piece::UN];
+#pragma unroll
+                    for (int u = 0; u < Piece::UN; u++)
+                        if (u < (int)h.y) xo[u] = xyz(ld_vec(s.x + cur.nb[u].idx));
+                    V4 r0 = make4<P>(mk3<P>(0, 0, 0), P(0)), r1 = r0, r2v = r0;  // y, history | gcp, k, lambda
+                    HT hd = 0;
+                    uint8_t fl = 0, gf = 0;
+                    if (live && lane == 0) {
+                        r0 = ld_vec(s.y + p);
+                        r1 = ld_vec(hist + p);
+                        hd = (HT)el.hd[p];
+                    }
+                    if (GROUND && live && lane == 1) {
+                        fl = s.flags[p];
+                        r0 = ld_vec(s.gcp + p);
+                        r1 = ld_vec(s.gk + p);
+                        r2v = ld_vec(s.glam + p);
+                        gf = s.gflag[p];
+                    }
+                    RS w[Piece::UN];
+#pragma unroll
+                    for (int u = 0; u < Piece::UN; u++) w[u] = cur.nb[u].w;
+                    // the next piece: of this color, else the first of the next
+                    ck += cstep;
+                    load_header(spread);
+                    if (ck >= cend) start_color(next_color(col), spread, phase + 1);
+#pragma unroll
+                    for (int u = 0; u < Piece::UN; u++)
+                        if (u < (int)h.y)
+                            star_edge<P, RS, HT, ST>(w[u], xo[u] - xi, es + (lane + u * LANES) * ST, K, Bk);
+                    for (unsigned u = Piece::UN; u < h.y; u++) {
+                        const StarNb<RS> q = ld_once(el.pnb + h.x + u * 32 + wl);
+                        star_edge<P, RS, HT, ST>(q.w, xyz(ld_vec(s.x + q.idx)) - xi, es + (lane + u * LANES) * ST, K, Bk);
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int u = 0; u < Piece::UT; u++)
+                        if (u < (int)h.w) star_tet<P, RS, HT, ST>(cur.tet[u], cur.loc[u], es, K, Bk);
+                    for (unsigned u = Piece::UT; u < h.w; u++)
+                        star_tet<P, RS, HT, ST>(ld_once(el.ptet + h.z + u * 32 + wl),
+                                                ld_once(el.ploc + h.z + u * 32 + wl), es, K, Bk);
+                    __syncwarp();  // the slot is refilled for the next piece
+                    if (ck < cend) cur.lists(el, wl);
+                    if (GROUND && (fl & VF_GROUND)) accumulate_ground<P, HT>(r1, r2v, r0, gf, xi, Bk);
+                    Bk.h00 += hd;
+                    Bk.h11 += hd;
+                    Bk.h22 += hd;
+                    reduce_block<LANES>(Bk);
+                    double acc = 0.0;
+                    V3<P> xa = xi;
+                    if (live && lane == 0) {
+                        const V3<P> rhs = block_rhs(Bk, xi, r0, c.inv_dt2);
+                        if (TOL) acc = sum_sq(rhs);
+                        xa = finish_vertex<P, HT>(s, c, A, counters, Bk, rhs, xi, p, r0.w, xyz(r1), om, hist);
+                    }
+                    if constexpr (GROUND) {
+                        xa.x = __shfl_sync(0xffffffffu, xa.x, wl & ~(LANES - 1));
+                        xa.y = __shfl_sync(0xffffffffu, xa.y, wl & ~(LANES - 1));
+                        xa.z = __shfl_sync(0xffffffffu, xa.z, wl & ~(LANES - 1));
+                        if ((fl & VF_GROUND) && !A.sweep_only) finish_ground<P>(s, p, r1, r2v, r0, gf, xa);
+                    }
+                    const unsigned sc = TOL ? scene[p] : 0u;
+                    if constexpr (TOL) {
+                        __syncwarp();
+                        sum.add(sc, acc);
+                    }
+                }
+                if constexpr (TOL) sum.flush();
+                if (cphase == phase) {  // a warp without a piece in this color
+                    start_color(next_color(col), spread, phase + 1);
+                    if (ck < cend) cur.lists(el, wl);
+                }
+                phase++;
+                if (!iterate_barrier(A.sync, ++bar, s.err)) return;
+            }
+        } else {
+            for (unsigned col = 0; col < A.ncolors; col++) {
+                const uint4 sl = A.slabs[col];
+                if (sl.y == 0) continue;
+                color_phase<P, RS, HT, LANES, FORM, GROUND, TOL, MODE_SOLVE>(s, el, c, counters, scene, sl.x, sl.y, on,
+                                                                             r2, spread);
+                if (!iterate_barrier(A.sync, ++bar, s.err)) return;
+            }
+            if (A.sweep_only) continue;
+            for (unsigned p = b * THREADS + threadIdx.x; p < s.n; p += B * THREADS) {
+                if (TOL && !on.get(scene[p])) continue;
+                chebyshev_dual_vertex<P>(s, p, GROUND ? s.flags[p] : (uint8_t)0, om, it);
+            }
+            if (!iterate_barrier(A.sync, ++bar, s.err)) return;
+        }
+        if constexpr (TOL) {
+            // the buffer of the iteration after the next: last read a barrier ago
+            if (b == B - 1)
+                for (unsigned q = threadIdx.x; q < A.S; q += THREADS) A.r2[(size_t)((it + 2) % 3u) * A.S + q] = 0;
+            const unsigned nc = iterate_candidates(A, on, cand, r2, &red);
+            if (nc == 0 && it + 1 < A.max_it) continue;
+            double* const ex = A.ex + (size_t)(exn & 1u) * A.S;
+            if (nc) {
+                if (b == B - 1)  // the other buffer, last read before the sweep
+                    for (unsigned q = threadIdx.x; q < A.S; q += THREADS) A.ex[(size_t)(~exn & 1u) * A.S + q] = 0;
+                residual_phase<P, RS, HT, LANES, FORM, GROUND>(s, el, c, scene, A, cand, ex);
+                if (!iterate_barrier(A.sync, ++bar, s.err)) return;
+                exn++;
+            }
+            na -= iterate_stop(A, on, cand, r2, ex, it + 1, b == B - 1, &red);
+            if (na > 0 && na < A.S) {  // scenes have stopped: other pieces than those on their way
+                spread = true;
+                if constexpr (PIPE) {
+                    start_color(color0, spread, phase);
+                    if (ck < cend) cur.lists(el, wl);
+                }
+            }
+        }
+    }
+    if (TOL && b == B - 1) {
+        for (unsigned q = threadIdx.x; q < A.S; q += THREADS) {
+            const bool live = on.get(q);
+            A.active[q] = live;
+            if (live) A.iters[q] = it;
+        }
+        if (threadIdx.x == 0) {
+            *A.n_active = (int)na;
+            *A.scene_iterations += done_it;
+            if (A.it_dev) *A.it_dev = it;
+            if (A.has_loop) {
+                *A.launches += 1;
+                cudaGraphSetConditional(A.loop, na > 0 && it < A.max_it ? 1u : 0u);
+            }
+        }
     }
 }
 
@@ -962,6 +1647,7 @@ static void solve_lanes_t(avbd_ctx* c, DevState<P>& s, const TetElems<RS>& el, c
             solve_dispatch<P, RS, HT, 8, MODE, true>(c, s, el, k, begin, count, st, out, T, list);
     } else {
         switch (c->lanes) {
+            case 1:  // one thread a vertex only in k_iterate
             case 2: solve_dispatch<P, RS, HT, 2, MODE>(c, s, el, k, begin, count, st, out, T, list, ranges, nranges); break;
             case 4: solve_dispatch<P, RS, HT, 4, MODE>(c, s, el, k, begin, count, st, out, T, list, ranges, nranges); break;
             case 16: solve_dispatch<P, RS, HT, 16, MODE>(c, s, el, k, begin, count, st, out, T, list, ranges, nranges); break;
@@ -986,72 +1672,6 @@ static void solve_lanes(avbd_ctx* c, DevState<double>& s, const StepConsts& k, u
         solve_lanes_t<double, float, float, MODE>(c, s, s.el32, k, begin, count, st, out, T, list, ranges, nranges);
     else
         solve_lanes_t<double, double, double, MODE>(c, s, s.el, k, begin, count, st, out, T, list, ranges, nranges);
-}
-
-// The persistent sweep (default; AVBD_PERSISTENT=0 at context creation turns
-// it off): one cooperative launch per iteration instead of one per color.  Taken for the run-to-tolerance
-// sweeps of contexts whose solve runs 2 threads per vertex with no damping,
-// no oriented particles and no dynamic contacts (the caller checks the last
-// two); returns false, having launched nothing, otherwise.
-template <typename P, typename RS, typename HT>
-static bool sweep_persistent_t(avbd_ctx* c, DevState<P>& s, const TetElems<RS>& el, const StepConsts& k,
-                               cudaStream_t st, const SceneTol& T) {
-    if (!c->persistent || c->lanes != 2 || c->damping || !c->d_solve_ranges || !c->d_solve_range_off ||
-        !c->d_sweep_sync || c->num_sms == 0)
-        return false;
-    const bool ground = !c->ground.empty();
-    auto kern = el.star ? (ground ? k_sweep_persistent<P, RS, HT, 2, FORM_STAR, true>
-                                  : k_sweep_persistent<P, RS, HT, 2, FORM_STAR, false>)
-                        : (ground ? k_sweep_persistent<P, RS, HT, 2, FORM_REC, true>
-                                  : k_sweep_persistent<P, RS, HT, 2, FORM_REC, false>);
-    const unsigned smem = el.star ? StarStage<P, 2>::bytes(el.max_nb) : 0;
-    if (!stage_smem(kern, smem)) return false;
-    // resident blocks per SM of this context's instantiation, queried once
-    // (-1 where the device cannot launch cooperative kernels: per-color
-    // launches then)
-    if (c->sweep_blocks_per_sm == 0) {
-        int per_sm = 0, coop = 0;
-        if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device) != cudaSuccess || !coop ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem) != cudaSuccess || per_sm < 1) {
-            cudaGetLastError();
-            c->sweep_blocks_per_sm = -1;
-        } else {
-            c->sweep_blocks_per_sm = per_sm;
-        }
-    }
-    if (c->sweep_blocks_per_sm < 1) return false;
-    const int per_sm = c->sweep_blocks_per_sm;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)per_sm * c->num_sms);
-    cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaMemsetAsync(c->d_sweep_sync, 0, 3 * sizeof(unsigned), st);
-    // a failed launch is left in the runtime's last error, which the step checks
-    cudaLaunchKernelEx(&cfg, kern, s, el, mkc<P>(k), c->d_counters, T, (const uint4*)c->d_solve_ranges,
-                       (const unsigned*)c->d_solve_range_off, c->num_colors, c->d_sweep_sync);
-    count_launch(c);
-    return true;
-}
-static bool sweep_persistent(avbd_ctx* c, DevState<float>& s, const StepConsts& k, cudaStream_t st,
-                             const SceneTol& T) {
-    return sweep_persistent_t<float, float, float>(c, s, s.el, k, st, T);
-}
-static bool sweep_persistent(avbd_ctx* c, DevState<double>& s, const StepConsts& k, cudaStream_t st,
-                             const SceneTol& T) {
-    if (c->solver.precision == AVBD_PRECISION_MIXED)
-        return sweep_persistent_t<double, float, float>(c, s, s.el32, k, st, T);
-    return sweep_persistent_t<double, double, double>(c, s, s.el, k, st, T);
-}
-
-template <typename R>
-bool launch_sweep_persistent(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaStream_t st, const SceneTol& T) {
-    return sweep_persistent(c, s, k, st, T);
 }
 
 int solve_set_wait_limit(unsigned polls) {
@@ -1096,46 +1716,39 @@ void launch_residual(avbd_ctx* c, DevState<R>& s, const StepConsts& k, double* o
 
 // ------------------------------------------- per-scene run-to-tolerance
 __global__ void k_tol_init(uint8_t* active, uint8_t* cand, double* r2, double* ex, uint32_t* iters, unsigned S,
-                           unsigned long long* maxr, uint32_t* it, double* omega, const double* omega_tab) {
+                           unsigned long long* maxr, uint32_t* it, double* omega, const double* omega_tab,
+                           int* n_active) {
     unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s == 0) {
         *maxr = 0ull;
+        *n_active = (int)S;
         *it = 0;
         if (omega_tab) *omega = omega_tab[0];
     }
     if (s >= S) return;
     active[s] = 1;
     cand[s] = 0;
-    r2[s] = 0;
-    ex[s] = 0;
+    r2[s] = r2[S + s] = r2[2 * S + s] = 0;
+    ex[s] = ex[S + s] = 0;
     iters[s] = 0;
 }
 
-AVBD_D double scene_R(double r2, double mg2) { return mg2 > 0 ? sqrt(r2) / sqrt(mg2) : sqrt(r2); }
-
-// After a sweep: every active scene counts the iteration and becomes a
-// candidate when its in-sweep residual is at the tolerance.
-// The in-sweep residual is kept (rin) as the final residual of a scene that
-// then stops at the cap without becoming a candidate.
-__global__ void k_tol_decide_a(uint8_t* active, uint8_t* cand, double* r2, const double* m2, uint32_t* iters,
-                               unsigned S, double tol, double g2, unsigned long long* scene_iterations,
-                               double* rin) {
+// In-sweep decision of a scene after a sweep: an active scene counts the
+// iteration and becomes a candidate when its in-sweep residual is at the
+// tolerance.  The in-sweep residual is kept (rin) as the final residual of a
+// scene that then stops at the cap without becoming a candidate.
+__global__ void k_tol_decide_a(IterArgs A) {
     unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    cand[s] = 0;
-    if (active[s]) {
-        iters[s]++;
-        atomicAdd(scene_iterations, 1ull);
-        const double R = scene_R(r2[s], m2[s] * g2);
-        rin[s] = R;
-        cand[s] = R <= tol;
+    if (s >= A.S) return;
+    A.cand[s] = 0;
+    if (A.active[s]) {
+        A.iters[s]++;
+        atomicAdd(A.scene_iterations, 1ull);
+        const double R = scene_R(A.r2[s], A.m2[s] * A.g2);
+        A.rin[s] = R;
+        A.cand[s] = R <= A.tol;
     }
-    r2[s] = 0;
-}
-
-AVBD_D unsigned long long ord_enc64(double d) {
-    unsigned long long u = (unsigned long long)__double_as_longlong(d);
-    return (u >> 63) ? ~u : (u | 0x8000000000000000ull);
+    A.r2[s] = 0;
 }
 
 // Candidates whose exact residual is at the tolerance stop; so does every
@@ -1143,58 +1756,257 @@ AVBD_D unsigned long long ord_enc64(double d) {
 // receives the largest final residual of the step's scenes: the exact one
 // where it was evaluated in the stopping iteration, else the in-sweep one of
 // a capped scene; maxr[1] counts the capped scenes.
-__global__ void k_tol_decide_b(uint8_t* active, uint8_t* cand, double* ex, const double* m2, const uint32_t* iters,
-                               unsigned S, double tol, double g2, unsigned max_it, int* n_active,
-                               unsigned long long* maxr, const double* rin) {
+__global__ void k_tol_decide_b(IterArgs A) {
     unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    if (active[s]) {
+    if (s >= A.S) return;
+    if (A.active[s]) {
         bool done = false;
-        double R = rin[s];
-        if (cand[s]) {
-            R = scene_R(ex[s], m2[s] * g2);
-            done = R <= tol;
+        double R = A.rin[s];
+        if (A.cand[s]) {
+            R = scene_R(A.ex[s], A.m2[s] * A.g2);
+            done = R <= A.tol;
         }
-        if (!done && iters[s] >= max_it) {  // stopped at the cap, unconverged
+        if (!done && A.iters[s] >= A.max_it) {  // stopped at the cap, unconverged
             done = true;
-            atomicAdd(maxr + 1, 1ull);
+            atomicAdd(A.maxr + 1, 1ull);
         }
         if (done) {
-            active[s] = 0;
-            atomicMax(maxr, ord_enc64(R));
+            A.active[s] = 0;
+            atomicMax(A.maxr, ord_enc64(R));
         } else {
-            atomicAdd(n_active, 1);
+            atomicAdd(A.n_active, 1);
         }
     }
-    cand[s] = 0;
-    ex[s] = 0;
+    A.cand[s] = 0;
+    A.ex[s] = 0;
+}
+
+// the run-to-tolerance part of an iteration launch's arguments
+static IterArgs tol_args(avbd_ctx* c, double tol, unsigned max_it) {
+    IterArgs A = {};
+    A.max_it = max_it;
+    A.tol = tol;
+    A.g2 = c->params.g_accel * c->params.g_accel;
+    A.m2 = c->d_scene_mg2;
+    A.active = c->d_scene_active;
+    A.cand = c->d_scene_cand;
+    A.iters = c->d_scene_iters;
+    A.r2 = c->d_scene_r2;
+    A.ex = c->d_scene_ex;
+    A.rin = c->d_scene_rin;
+    A.S = c->num_scenes;
+    A.scene_iterations = c->d_counters + 1;
+    A.maxr = c->d_counters + 2;
+    A.n_active = c->d_tol_count;
+    return A;
 }
 
 void launch_tol_init(avbd_ctx* c, cudaStream_t st) {
     unsigned S = c->num_scenes;
     k_tol_init<<<nblocks(S, 256), 256, 0, st>>>(c->d_scene_active, c->d_scene_cand, c->d_scene_r2, c->d_scene_ex,
                                                 c->d_scene_iters, S, c->d_counters + 2, c->d_tol_it, c->d_tol_omega,
-                                                c->d_omega_tab);
+                                                c->d_omega_tab, c->d_tol_count);
     count_launch(c);
 }
 
 void launch_tol_decide_a(avbd_ctx* c, double tol, cudaStream_t st) {
-    unsigned S = c->num_scenes;
-    k_tol_decide_a<<<nblocks(S, 256), 256, 0, st>>>(c->d_scene_active, c->d_scene_cand, c->d_scene_r2,
-                                                    c->d_scene_mg2, c->d_scene_iters, S, tol,
-                                                    c->params.g_accel * c->params.g_accel, c->d_counters + 1,
-                                                    c->d_scene_rin);
+    k_tol_decide_a<<<nblocks(c->num_scenes, 256), 256, 0, st>>>(tol_args(c, tol, 0));
     count_launch(c);
 }
 
 void launch_tol_decide_b(avbd_ctx* c, double tol, unsigned max_it, cudaStream_t st) {
-    unsigned S = c->num_scenes;
     cudaMemsetAsync(c->d_tol_count, 0, sizeof(int), st);
-    k_tol_decide_b<<<nblocks(S, 256), 256, 0, st>>>(c->d_scene_active, c->d_scene_cand, c->d_scene_ex,
-                                                    c->d_scene_mg2, c->d_scene_iters, S, tol,
-                                                    c->params.g_accel * c->params.g_accel, max_it, c->d_tol_count,
-                                                    c->d_counters + 2, c->d_scene_rin);
+    k_tol_decide_b<<<nblocks(c->num_scenes, 256), 256, 0, st>>>(tol_args(c, tol, max_it));
     count_launch(c);
+}
+
+// One warp per piece: its vertices' lists, filled up to whole rounds.
+template <typename RS>
+__global__ void k_layout_pieces(TetElems<RS> el, const uint4* slabs, unsigned ncolors, unsigned lanes, uint4* piece,
+                                unsigned npieces, StarNb<RS>* pnb, StarTet<RS>* ptet, uint32_t* ploc) {
+    const unsigned k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, wl = threadIdx.x & 31u;
+    if (k >= npieces) return;
+    unsigned col = 0;
+    while (col + 1 < ncolors && slabs[col + 1].z <= k) col++;
+    const uint4 sl = slabs[col];
+    const uint4 h = piece[k];
+    const unsigned V = 32 / lanes, gi = (k - sl.z) * V + wl / lanes, lane = wl % lanes;
+    const bool live = gi < sl.y;
+    const unsigned p = sl.x + min(gi, sl.y - 1);
+    const uint2 o0 = el.star[p], o1 = live ? el.star[p + 1] : o0;
+    for (unsigned u = 0; u < h.y; u++) {
+        const unsigned j = o0.x + lane + u * lanes;
+        StarNb<RS> q{};
+        q.idx = p;
+        if (j < o1.x) q = el.nb[j];
+        pnb[h.x + u * 32 + wl] = q;
+    }
+    for (unsigned u = 0; u < h.w; u++) {
+        const unsigned t = o0.y + lane + u * lanes;
+        const bool in = t < o1.y;
+        ptet[h.z + u * 32 + wl] = in ? el.tet[t] : StarTet<RS>{RS(0), RS(0)};
+        ploc[h.z + u * 32 + wl] = in ? el.loc[t] : 0u;
+    }
+}
+
+template <typename R, typename RS>
+static int layout_pieces_t(avbd_ctx* c, TetElems<RS>& el, cudaStream_t st) {
+    for (void* p : c->piece_alloc) cudaFree(p);
+    c->piece_alloc.clear();
+    el.piece = nullptr;
+    const unsigned lanes = (unsigned)c->lanes;
+    if (!el.star || lanes == 2 || c->star_off.empty()) return AVBD_OK;
+    const unsigned V = 32 / lanes;
+    std::vector<uint4> slabs(c->num_colors), piece;
+    size_t nn = 0, nt = 0;
+    for (unsigned k = 0; k < c->num_colors; k++) {
+        const unsigned b = c->color_begin[k], e = b + c->color_solve[k];
+        slabs[k] = make_uint4(b, e - b, (unsigned)piece.size(), 0);
+        for (unsigned i = b; i < e; i += V) {
+            unsigned mn = 0, mt = 0;
+            for (unsigned j = i; j < std::min(i + V, e); j++) {
+                mn = std::max(mn, c->star_off[j + 1].x - c->star_off[j].x);
+                mt = std::max(mt, c->star_off[j + 1].y - c->star_off[j].y);
+            }
+            const uint4 h = make_uint4((unsigned)nn, nblocks(mn, lanes), (unsigned)nt, nblocks(mt, lanes));
+            piece.push_back(h);
+            nn += 32ull * h.y;
+            nt += 32ull * h.w;
+        }
+    }
+    if (piece.empty() || nn > UINT32_MAX || nt > UINT32_MAX) return AVBD_OK;  // not laid out: launches per color
+    uint4* dp = nullptr;
+    StarNb<RS>* dn = nullptr;
+    StarTet<RS>* dt = nullptr;
+    uint32_t* dl = nullptr;
+    auto al = [&](auto** p, size_t bytes) {
+        if (cudaMalloc((void**)p, std::max(bytes, (size_t)16)) != cudaSuccess) return false;
+        c->piece_alloc.push_back((void*)*p);
+        return true;
+    };
+    if (!al(&dp, sizeof(uint4) * piece.size()) || !al(&dn, sizeof(StarNb<RS>) * nn) ||
+        !al(&dt, sizeof(StarTet<RS>) * nt) || !al(&dl, sizeof(uint32_t) * nt)) {
+        return set_error(AVBD_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(cudaGetLastError()));
+    }
+    cudaMemcpyAsync(dp, piece.data(), sizeof(uint4) * piece.size(), cudaMemcpyHostToDevice, st);
+    cudaMemcpyAsync(c->d_slabs, slabs.data(), sizeof(uint4) * slabs.size(), cudaMemcpyHostToDevice, st);
+    const unsigned np = (unsigned)piece.size();
+    k_layout_pieces<RS><<<nblocks(np, 8), 256, 0, st>>>(el, c->d_slabs, c->num_colors, lanes, dp, np, dn, dt, dl);
+    const cudaError_t e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return set_error(AVBD_ERR_CUDA, cudaGetErrorString(e));
+    el.piece = dp;
+    el.pnb = dn;
+    el.ptet = dt;
+    el.ploc = dl;
+    return AVBD_OK;
+}
+template <typename R>
+int layout_pieces(avbd_ctx* c, DevState<R>& s, cudaStream_t st) {
+    if (c->solver.precision == AVBD_PRECISION_MIXED) return layout_pieces_t<R>(c, s.el32, st);
+    return layout_pieces_t<R>(c, s.el, st);
+}
+
+// Blocks of an iteration launch: one per SM, fewer where a color has less
+// than a few warps of work for each (a barrier over fewer blocks is cheaper).
+static unsigned iterate_blocks(const avbd_ctx* c, unsigned lanes) {
+    const unsigned chunks = nblocks(c->max_color_solve, 32 / lanes);
+    return std::max(1u, std::min(c->num_sms, nblocks(chunks, ITER_WARPS_MIN)));
+}
+
+template <typename P, typename RS, typename HT, int LANES, int FORM>
+static bool iterate_launch(avbd_ctx* c, DevState<P>& s, const TetElems<RS>& el, const StepConsts& k, cudaStream_t st,
+                           const IterArgs& A) {
+    constexpr int THREADS = IterThreads<P, FORM, LANES>::value;
+    const bool ground = !c->ground.empty(), tol = A.max_it != 0;
+    auto kern = tol ? (ground ? k_iterate<P, RS, HT, LANES, FORM, true, true> : k_iterate<P, RS, HT, LANES, FORM, false, true>)
+                    : (ground ? k_iterate<P, RS, HT, LANES, FORM, true, false> : k_iterate<P, RS, HT, LANES, FORM, false, false>);
+    constexpr bool STAR = FORM == FORM_STAR && LANES != 2;
+    if (STAR && !el.piece) return false;
+    unsigned smem = FORM == FORM_STAR
+                        ? StarStage<P, LANES, THREADS>::bytes(STAR ? star_rows(el.max_nb, LANES) : el.max_nb)
+                        : 0;
+    if (tol) smem += 2 * nblocks(A.S, 32) * (unsigned)sizeof(uint32_t);
+    if (!stage_smem(kern, smem)) {
+        cudaGetLastError();
+        return false;
+    }
+    // whether one block per SM is resident (the grid barrier needs all of
+    // them), queried once per lane count and kind of step
+    int8_t& fits = c->iterate_fits[tol][LANES == 1 ? 4 : LANES == 2 ? 0 : LANES == 4 ? 1 : LANES == 8 ? 2 : 3];
+    if (fits == 0) {
+        int per_sm = 0, coop = 0;
+        fits = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device) == cudaSuccess && coop &&
+                       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, THREADS, smem) == cudaSuccess &&
+                       per_sm >= 1
+                   ? 1
+                   : -1;
+        cudaGetLastError();
+    }
+    if (fits < 0) return false;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(iterate_blocks(c, LANES));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaMemsetAsync(c->d_sweep_sync, 0, 4 * sizeof(unsigned), st);
+    // a failed launch is left in the runtime's last error, which the step checks
+    cudaLaunchKernelEx(&cfg, kern, s, el, mkc<P>(k), c->d_counters, (const uint32_t*)c->d_scene, A);
+    count_launch(c);
+    return true;
+}
+
+template <typename P, typename RS, typename HT>
+static bool iterate_t(avbd_ctx* c, DevState<P>& s, const TetElems<RS>& el, const StepConsts& k, cudaStream_t st,
+                      const IterArgs& A) {
+    if (el.star) {
+        switch (c->lanes) {
+            case 1: return iterate_launch<P, RS, P, 1, FORM_STAR>(c, s, el, k, st, A);
+            case 2: return iterate_launch<P, RS, HT, 2, FORM_STAR>(c, s, el, k, st, A);
+            case 4: return iterate_launch<P, RS, P, 4, FORM_STAR>(c, s, el, k, st, A);
+            case 16: return iterate_launch<P, RS, P, 16, FORM_STAR>(c, s, el, k, st, A);
+            default: return iterate_launch<P, RS, P, 8, FORM_STAR>(c, s, el, k, st, A);
+        }
+    }
+    if (c->damping)
+        return c->lanes == 2 ? iterate_launch<P, RS, HT, 2, FORM_DAMP>(c, s, el, k, st, A)
+                             : iterate_launch<P, RS, HT, 8, FORM_DAMP>(c, s, el, k, st, A);
+    return c->lanes == 2 ? iterate_launch<P, RS, HT, 2, FORM_REC>(c, s, el, k, st, A)
+                         : iterate_launch<P, RS, HT, 8, FORM_REC>(c, s, el, k, st, A);
+}
+static bool iterate(avbd_ctx* c, DevState<float>& s, const StepConsts& k, cudaStream_t st, const IterArgs& A) {
+    return iterate_t<float, float, float>(c, s, s.el, k, st, A);
+}
+static bool iterate(avbd_ctx* c, DevState<double>& s, const StepConsts& k, cudaStream_t st, const IterArgs& A) {
+    if (c->solver.precision == AVBD_PRECISION_MIXED) return iterate_t<double, float, float>(c, s, s.el32, k, st, A);
+    return iterate_t<double, double, double>(c, s, s.el, k, st, A);
+}
+
+template <typename R>
+bool launch_iterate(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaStream_t st, const IterLaunch& L) {
+    if (!c->persistent || s.no != 0 || c->dyn || c->num_sms == 0 || c->max_color_solve == 0) return false;
+    IterArgs A = {};
+    if (L.tol > 0) {
+        A = tol_args(c, L.tol, L.max_it);
+        if (L.loop) {
+            A.it_dev = c->d_tol_it;
+            A.loop = *L.loop;
+            A.has_loop = true;
+            A.launches = c->d_counters + 5;
+        }
+    }
+    A.slabs = c->d_slabs;
+    A.ncolors = c->num_colors;
+    A.omega = c->d_omega_tab;
+    A.it0 = L.it0;
+    A.n = L.n;
+    A.sync = c->d_sweep_sync;
+    A.sweep_only = L.sweep_only;
+    return iterate(c, s, k, st, A);
 }
 
 // End of one iteration of the device-driven loop: counts it and continues the
@@ -1303,8 +2115,8 @@ void launch_store_vec(const DevState<R>& s, int which, double* dst, const uint32
     template void launch_tet_eprev<R>(avbd_ctx*, DevState<R>&, const StepConsts&, cudaStream_t);                \
     template void launch_solve_color<R>(avbd_ctx*, DevState<R>&, const StepConsts&, unsigned, unsigned,         \
                                         cudaStream_t, const SceneTol&, const uint32_t*, const uint4*, unsigned); \
-    template bool launch_sweep_persistent<R>(avbd_ctx*, DevState<R>&, const StepConsts&, cudaStream_t,           \
-                                             const SceneTol&);                                                  \
+    template bool launch_iterate<R>(avbd_ctx*, DevState<R>&, const StepConsts&, cudaStream_t, const IterLaunch&); \
+    template int layout_pieces<R>(avbd_ctx*, DevState<R>&, cudaStream_t);                                        \
     template void launch_chebyshev_dual<R>(avbd_ctx*, DevState<R>&, const StepConsts&, double, unsigned, cudaStream_t,    \
                                            const SceneTol&);                                                    \
     template void launch_velocity<R>(avbd_ctx*, DevState<R>&, const StepConsts&, cudaStream_t);                 \
