@@ -93,8 +93,9 @@ AVBD_D bool solve_sym3(const Sym3<R>& A, V3<R> b, R kappa_max, V3<R>& x) {
     x.x = (c00 * b.x + c01 * b.y + c02 * b.z) * inv;
     x.y = (c01 * b.x + c11 * b.y + c12 * b.z) * inv;
     x.z = (c02 * b.x + c12 * b.y + c22 * b.z) * inv;
-    R na = A.a00 * A.a00 + A.a11 * A.a11 + A.a22 * A.a22 + R(2) * (A.a01 * A.a01 + A.a02 * A.a02 + A.a12 * A.a12);
-    R nc = c00 * c00 + c11 * c11 + c22 * c22 + R(2) * (c01 * c01 + c02 * c02 + c12 * c12);
+    // (sums in pairs: the solve is a chain of dependent operations)
+    R na = (A.a00 * A.a00 + A.a11 * A.a11) + (A.a22 * A.a22 + R(2) * ((A.a01 * A.a01 + A.a02 * A.a02) + A.a12 * A.a12));
+    R nc = (c00 * c00 + c11 * c11) + (c22 * c22 + R(2) * ((c01 * c01 + c02 * c02) + c12 * c12));
     return (na * fabs(inv)) * (nc * fabs(inv)) <= kappa_max * kappa_max;
 }
 

@@ -1280,7 +1280,10 @@ __global__ void __launch_bounds__((IterThreads<P, FORM, LANES>::value), 1)
     constexpr unsigned ST = StarStage<P, LANES, THREADS>::STRIDE;
     using Piece = StarPiece<RS, PIPE ? LANES : 4>;
     __shared__ unsigned red;
+    __shared__ uint4 slabs[256];  // A.slabs: a load from global memory at each phase would sit on its chain
     extern __shared__ __align__(16) unsigned char stage[];
+    for (unsigned q = threadIdx.x; q < A.ncolors; q += blockDim.x) slabs[q] = A.slabs[q];
+    __syncthreads();
     const unsigned warp = threadIdx.x >> 5, wl = threadIdx.x & 31u, lane = wl % LANES;
     const unsigned B = gridDim.x, b = blockIdx.x;
     const unsigned K = PIPE ? star_rows(el.max_nb, LANES) : el.max_nb;
@@ -1315,7 +1318,7 @@ __global__ void __launch_bounds__((IterThreads<P, FORM, LANES>::value), 1)
     bool clive = false;
     auto next_color = [&](unsigned col) {  // the next color with vertices, cyclic
         do col = col + 1 < A.ncolors ? col + 1 : 0;
-        while (A.slabs[col].y == 0);
+        while (slabs[col].y == 0);
         return col;
     };
     auto load_header = [&](bool spread) {  // of piece ck; stopped scenes' pieces are passed over
@@ -1333,7 +1336,7 @@ __global__ void __launch_bounds__((IterThreads<P, FORM, LANES>::value), 1)
         }
     };
     auto start_color = [&](unsigned col, bool spread, unsigned phase) {
-        const uint4 sl = A.slabs[col];
+        const uint4 sl = slabs[col];
         const unsigned nch = (sl.y + V - 1) / V, per = (nch + B - 1) / B;
         cbegin = sl.x;
         ccount = sl.y;
@@ -1358,7 +1361,7 @@ __global__ void __launch_bounds__((IterThreads<P, FORM, LANES>::value), 1)
         const P om = A.sweep_only ? P(1) : (P)A.omega[it];
         if constexpr (STAR && !PIPE) {
             for (unsigned col = 0; col < A.ncolors; col++) {
-                const uint4 sl = A.slabs[col];
+                const uint4 sl = slabs[col];
                 if (sl.y == 0) continue;
                 color_wide<P, RS, GROUND, TOL>(s, el, c, A, counters, scene, sl, on, spread, om, (it & 1u) ? s.xll : s.xl,
                                                r2, es);
@@ -1368,7 +1371,7 @@ __global__ void __launch_bounds__((IterThreads<P, FORM, LANES>::value), 1)
             V4* const hist = (it & 1u) ? s.xll : s.xl;
             SceneSum sum(r2);
             for (unsigned col = 0; col < A.ncolors; col++) {
-                if (A.slabs[col].y == 0) continue;
+                if (slabs[col].y == 0) continue;
                 while (cphase == phase && ck < cend) {
                     const unsigned p = cp;
                     const bool live = clive;
@@ -1453,7 +1456,7 @@ __global__ void __launch_bounds__((IterThreads<P, FORM, LANES>::value), 1)
             }
         } else {
             for (unsigned col = 0; col < A.ncolors; col++) {
-                const uint4 sl = A.slabs[col];
+                const uint4 sl = slabs[col];
                 if (sl.y == 0) continue;
                 color_phase<P, RS, HT, LANES, FORM, GROUND, TOL, MODE_SOLVE>(s, el, c, counters, scene, sl.x, sl.y, on,
                                                                              r2, spread);
@@ -1586,11 +1589,11 @@ void launch_tet_eprev(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaStre
     count_launch(c);
 }
 
-// Dynamic shared memory of a kernel's neighbour staging; above 48 KB the
-// kernel has to opt in.
+// Dynamic shared memory of a kernel's neighbour staging; above 48 KB, with
+// the static part (under 8 KB), the kernel has to opt in.
 template <typename K>
 static bool stage_smem(K kern, unsigned bytes) {
-    return bytes <= 48 * 1024 ||
+    return bytes <= 40 * 1024 ||
            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
 }
 
