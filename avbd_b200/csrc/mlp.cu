@@ -1,7 +1,7 @@
 // mlp.cu -- the learned warm start's multilayer perceptron on the tensor
-// cores: a generic BF16 GEMM (training), the fused persistent inference
-// kernel (the hot path: features -> 4 layers -> x0 update), and the training
-// kernels (bias + SiLU, loss, activation gradient, transposes, Adam).
+// cores: a generic BF16 GEMM, the fused persistent inference kernel (the hot
+// path: features -> 4 layers -> x0 update), the fused forward and backward
+// pass of training, and Adam.
 //
 // The reference has no learned component; this is new functionality.  All
 // matrix products run as tcgen05.mma (kind::f16, BF16 operands in shared
@@ -36,8 +36,8 @@ AVBD_D float silu(float z) { return z / (1.0f + __expf(-z)); }
 // The same function as z/2 (1 + tanh(z/2)) with the hardware tanh
 // approximation (one special-function operation instead of two; its error,
 // about 2^-11 relative, is below the BF16 rounding of the result).
-AVBD_D float silu_fast(float z) {
-    const float h = 0.5f * z;
+// h = z / 2.
+AVBD_D float silu_half(float h) {
     float t;
     asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(h));
     return fmaf(h, t, h);
@@ -219,14 +219,19 @@ struct MlpSink {
     unsigned long long* applied;  // count of accepted corrections (may be null)
 };
 
-constexpr unsigned SM_W1 = 0, SM_W2 = 8192, SM_W3 = 40960, SM_W4 = 73728, SM_X = 77824, SM_H = 94208,
-                   SM_BIAS = 126976, SM_BAR = 128576, SM_TSLOT = 128584, SM_TOTAL = 128640;  // X: 2 x 8 KB
+// Thread groups of the fused inference: each takes its own tile through the
+// layers with its own buffers (X: 2 x 8 KB, H: 32 KB), accumulator and
+// barriers; the weights are shared.
+constexpr unsigned GROUPS = 3, GTHREADS = 256;
+constexpr unsigned SM_W1 = 0, SM_W2 = 8192, SM_W3 = 40960, SM_W4 = 73728, SM_X = 77824,
+                   SM_H = SM_X + GROUPS * 16384, SM_BIAS = SM_H + GROUPS * 32768, SM_BAR = SM_BIAS + 1600,
+                   SM_TSLOT = SM_BAR + 8 * GROUPS, SM_TOTAL = SM_TSLOT + 8;
 
 // Feature tile (128 rows x 32 BF16) -> canonical K-major shared layout with
 // cp.async (rows >= rows_valid are zero-filled), so the next tile streams in
 // while this one runs through the layers.
-AVBD_D void load_x_async(uint8_t* dst, const bf16* src, unsigned rows_valid, unsigned tid) {
-    for (unsigned i = tid; i < 128 * (IN / 8); i += blockDim.x) {
+AVBD_D void load_x_async(uint8_t* dst, const bf16* src, unsigned rows_valid, unsigned tid, unsigned nthreads) {
+    for (unsigned i = tid; i < 128 * (IN / 8); i += nthreads) {
         const unsigned r = i % 128, c = i / 128;
         const bool in = r < rows_valid;
         const bf16* g = in ? src + (size_t)r * IN + c * 8 : src;
@@ -237,25 +242,44 @@ AVBD_D void load_x_async(uint8_t* dst, const bf16* src, unsigned rows_valid, uns
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-// TMEM accumulator -> bias + SiLU -> BF16 into the H operand.  16 warps:
-// warp w reads lanes 32 (w % 4).. (rows) and the column quarter w / 4 (16
-// warps rather than 8: 4 % less time per launch, the epilogue being
-// latency-bound).
-AVBD_D void epilogue_hidden(uint32_t tacc, const float* bias, uint8_t* H, unsigned warp, unsigned lane) {
-    const unsigned q = warp & 3u, hf = warp >> 2;  // 16 warps: column quarters
+// TMEM accumulator -> bias + SiLU -> BF16 into the H operand.  8 warps: warp w
+// reads lanes 32 (w % 4).. (rows) and the column half w / 4.  hbias: half the
+// biases, so that the tanh's argument (v + b) / 2 is one multiply-add.
+AVBD_D void epilogue_hidden(uint32_t tacc, const float* hbias, uint8_t* H, unsigned warp, unsigned lane) {
+    const unsigned q = warp & 3u, hf = warp >> 2;
     const unsigned r = q * 32 + lane;
     const uint32_t base = tacc + ((q * 32u) << 16);
 #pragma unroll
-    for (unsigned c = hf * 32; c < hf * 32 + 32; c += 16) {
+    for (unsigned c = hf * 64; c < hf * 64 + 64; c += 16) {
         float v[16];
         tc::tmem_ld16(base + c, v);
         uint32_t pk[8];
 #pragma unroll
-        for (int j = 0; j < 8; j++)
-            pk[j] = pack2(silu_fast(v[2 * j] + bias[c + 2 * j]), silu_fast(v[2 * j + 1] + bias[c + 2 * j + 1]));
+        for (int j = 0; j < 16; j += 4) {
+            const float4 b = *reinterpret_cast<const float4*>(hbias + c + j);
+            pk[j / 2] = pack2(silu_half(fmaf(0.5f, v[j], b.x)), silu_half(fmaf(0.5f, v[j + 1], b.y)));
+            pk[j / 2 + 1] = pack2(silu_half(fmaf(0.5f, v[j + 2], b.z)), silu_half(fmaf(0.5f, v[j + 3], b.w)));
+        }
         *reinterpret_cast<uint4*>(H + (c / 8) * (128 * 16) + r * 16) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
         *reinterpret_cast<uint4*>(H + (c / 8 + 1) * (128 * 16) + r * 16) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
     }
+}
+
+AVBD_D void group_sync(unsigned g) { asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "r"(GTHREADS) : "memory"); }
+// the group's threads wait for its barrier's phase; false (for all of them) if it timed out
+AVBD_D bool group_wait(uint64_t* bar, uint32_t& phase, unsigned g) {
+    const uint32_t got = tc::mbar_wait(bar, phase, *(volatile uint32_t*)&g_wait_polls) ? 1u : 0u;
+    phase ^= 1u;
+    uint32_t all;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "bar.red.and.pred q, %2, %3, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}\n"
+        : "=r"(all)
+        : "r"(got), "r"(g + 1), "r"(GTHREADS)
+        : "memory");
+    return all != 0;
 }
 
 // Acceptance of the correction y (in units of s = g h^2) of one vertex.  The
@@ -277,112 +301,92 @@ AVBD_D bool accept(const uint8_t* Xs, unsigned r, const float* y, float kappa) {
 }
 
 // Persistent: one CTA per SM, weights resident in shared memory, 128 feature
-// rows per tile; layers alternate between TMEM columns [0,128) and [128,256).
+// rows per tile and thread group.  Bound by the hidden epilogues (a tanh per
+// activation: 3,072 cycles of the special-function units a tile).  The layers
+// of one tile are a chain (product, accumulator read, SiLU, operand store,
+// fences); with one tile in flight per SM a million rows took 336 us, three
+// times the tanh bound.  Three groups of 8 warps, each with a tile of its own
+// and no barrier in common, fill one another's waits.
 template <typename P>
-__global__ void __launch_bounds__(512, 1) k_mlp_apply(MlpW w, const bf16* __restrict__ feat, unsigned n,
-                                                       MlpSink<P> sink, int* err) {
+__global__ void __launch_bounds__(GROUPS * GTHREADS, 1) k_mlp_apply(MlpW w, const bf16* __restrict__ feat, unsigned n,
+                                                                    MlpSink<P> sink, int* err) {
     extern __shared__ __align__(1024) uint8_t sm[];
+    constexpr unsigned NT = GROUPS * GTHREADS;
     uint8_t* W1s = sm + SM_W1;
     uint8_t* W2s = sm + SM_W2;
     uint8_t* W3s = sm + SM_W3;
     uint8_t* W4s = sm + SM_W4;
-    uint8_t* Xbuf = sm + SM_X;  // two 8 KB tiles
-    uint8_t* Hs = sm + SM_H;
-    float* bias = reinterpret_cast<float*>(sm + SM_BIAS);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + SM_BAR);
+    const unsigned g = threadIdx.x / GTHREADS, tid = threadIdx.x % GTHREADS, warp = tid >> 5, lane = tid & 31;
+    uint8_t* Xbuf = sm + SM_X + g * 16384;  // two 8 KB tiles
+    uint8_t* Hs = sm + SM_H + g * 32768;
+    float* bias = reinterpret_cast<float*>(sm + SM_BIAS);  // halved for the hidden layers
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + SM_BAR) + g;
     uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + SM_TSLOT);
-    const unsigned tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-    load_kmaj(W1s, w.w1, IN, HID, IN, HID, tid, 512);
-    load_kmaj(W2s, w.w2, HID, HID, HID, HID, tid, 512);
-    load_kmaj(W3s, w.w3, HID, HID, HID, HID, tid, 512);
-    load_kmaj(W4s, w.w4, HID, OUT, HID, OUT, tid, 512);
-    for (unsigned i = tid; i < 3 * HID + OUT; i += 512) bias[i] = w.b[i];
-    if (warp == 0) tc::tmem_alloc(tslot, 256);
+    load_kmaj(W1s, w.w1, IN, HID, IN, HID, threadIdx.x, NT);
+    load_kmaj(W2s, w.w2, HID, HID, HID, HID, threadIdx.x, NT);
+    load_kmaj(W3s, w.w3, HID, HID, HID, HID, threadIdx.x, NT);
+    load_kmaj(W4s, w.w4, HID, OUT, HID, OUT, threadIdx.x, NT);
+    for (unsigned i = threadIdx.x; i < 3 * HID + OUT; i += NT) bias[i] = i < 3 * HID ? 0.5f * w.b[i] : w.b[i];
+    if (threadIdx.x < 32) tc::tmem_alloc(tslot, 512);
     if (tid == 0) tc::mbar_init(bar, 1);
     tc::fence_async_smem();
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
-    const uint32_t tmem = *tslot;
-    const uint32_t accA = tmem, accB = tmem + 128;
+    const uint32_t acc = *tslot + g * 128;
     const uint32_t id_h = tc::idesc_bf16(128, HID), id_o = tc::idesc_bf16(128, OUT);
     const uint32_t aH = tc::smem_u32(Hs);
     uint32_t phase = 0;
     bool ok = true;
-    const unsigned ntiles = (n + 127) / 128;
-    if (blockIdx.x < ntiles) {
-        const unsigned r0 = blockIdx.x * 128;
-        load_x_async(Xbuf, feat + (size_t)r0 * IN, min(128u, n - r0), tid);
-    }
+    const unsigned ntiles = (n + 127) / 128, step = gridDim.x * GROUPS, first = blockIdx.x + gridDim.x * g;
+    if (first < ntiles) load_x_async(Xbuf, feat + (size_t)first * 128 * IN, min(128u, n - first * 128), tid, GTHREADS);
     unsigned buf = 0;
-    for (unsigned tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, buf ^= 1u) {
+    for (unsigned tile = first; tile < ntiles; tile += step, buf ^= 1u) {
         const unsigned row0 = tile * 128;
         uint8_t* Xs = Xbuf + buf * 8192;
         const uint32_t aX = tc::smem_u32(Xs);
-        const unsigned next = tile + gridDim.x;
+        const unsigned next = tile + step;
         if (next < ntiles) {  // the other buffer was last read by the previous tile, finished
-            const unsigned r1 = next * 128;
-            load_x_async(Xbuf + (buf ^ 1u) * 8192, feat + (size_t)r1 * IN, min(128u, n - r1), tid);
+            load_x_async(Xbuf + (buf ^ 1u) * 8192, feat + (size_t)next * 128 * IN, min(128u, n - next * 128), tid,
+                         GTHREADS);
             asm volatile("cp.async.wait_group 1;" ::: "memory");
         } else {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
-        tc::fence_async_smem();
-        __syncthreads();
-        // layer 1: X W1^T -> accA
-        if (tid == 0) {
+        // one layer: D = A W^T into the group's accumulator
+        auto layer = [&](uint32_t a, const uint8_t* W, unsigned rows, unsigned ksteps, uint32_t id) {
+            tc::fence_before();  // the accumulator's readers are done
+            tc::fence_async_smem();
+            group_sync(g);
+            if (tid == 0) {
+                tc::fence_after();
+                issue(acc, a, 128, tc::smem_u32(W), rows, ksteps, id, false);
+                tc::commit(bar);
+            }
+            const bool got = group_wait(bar, phase, g);
             tc::fence_after();
-            issue(accA, aX, 128, tc::smem_u32(W1s), HID, IN / 16, id_h, false);
-            tc::commit(bar);
-        }
-        if (!(ok = block_wait(bar, phase))) break;
-        tc::fence_after();
-        epilogue_hidden(accA, bias, Hs, warp, lane);
-        tc::fence_before();
-        tc::fence_async_smem();
-        __syncthreads();
-        // layer 2: H W2^T -> accB
-        if (tid == 0) {
-            tc::fence_after();
-            issue(accB, aH, 128, tc::smem_u32(W2s), HID, HID / 16, id_h, false);
-            tc::commit(bar);
-        }
-        if (!(ok = block_wait(bar, phase))) break;
-        tc::fence_after();
-        epilogue_hidden(accB, bias + HID, Hs, warp, lane);
-        tc::fence_before();
-        tc::fence_async_smem();
-        __syncthreads();
-        // layer 3: H W3^T -> accA
-        if (tid == 0) {
-            tc::fence_after();
-            issue(accA, aH, 128, tc::smem_u32(W3s), HID, HID / 16, id_h, false);
-            tc::commit(bar);
-        }
-        if (!(ok = block_wait(bar, phase))) break;
-        tc::fence_after();
-        epilogue_hidden(accA, bias + 2 * HID, Hs, warp, lane);
-        tc::fence_before();
-        tc::fence_async_smem();
-        __syncthreads();
-        // layer 4: H W4^T -> accB columns [0, 16)
-        if (tid == 0) {
-            tc::fence_after();
-            issue(accB, aH, 128, tc::smem_u32(W4s), OUT, HID / 16, id_o, false);
-            tc::commit(bar);
-        }
-        if (!(ok = block_wait(bar, phase))) break;
-        tc::fence_after();
+            return got;
+        };
+        if (!(ok = layer(aX, W1s, HID, IN / 16, id_h))) break;
+        epilogue_hidden(acc, bias, Hs, warp, lane);
+        if (!(ok = layer(aH, W2s, HID, HID / 16, id_h))) break;
+        epilogue_hidden(acc, bias + HID, Hs, warp, lane);
+        if (!(ok = layer(aH, W3s, HID, HID / 16, id_h))) break;
+        epilogue_hidden(acc, bias + 2 * HID, Hs, warp, lane);
+        if (!(ok = layer(aH, W4s, OUT, HID / 16, id_o))) break;
         if (warp < 4) {
             float v[16];
-            tc::tmem_ld16(accB + ((warp * 32u) << 16), v);
+            tc::tmem_ld16(acc + ((warp * 32u) << 16), v);
             const unsigned row = row0 + warp * 32 + lane;
             if (row < n) {
                 const float* b4 = bias + 3 * HID;
                 if (sink.out) {
+                    float4* o = reinterpret_cast<float4*>(sink.out + (size_t)row * OUT);
 #pragma unroll
-                    for (int j = 0; j < 16; j++) sink.out[(size_t)row * OUT + j] = v[j] + b4[j];
+                    for (int j = 0; j < 4; j++)
+                        o[j] = make_float4(v[4 * j] + b4[4 * j], v[4 * j + 1] + b4[4 * j + 1],
+                                           v[4 * j + 2] + b4[4 * j + 2], v[4 * j + 3] + b4[4 * j + 3]);
                 } else if (!(sink.flags[row] & (VF_FIXED | VF_ORIENTED))) {
                     const float y[3] = {v[0] + b4[0], v[1] + b4[1], v[2] + b4[2]};
                     if (accept(Xs, warp * 32 + lane, y, sink.kappa)) {
@@ -398,126 +402,289 @@ __global__ void __launch_bounds__(512, 1) k_mlp_apply(MlpW w, const bf16* __rest
                 }
             }
         }
-        tc::fence_before();
-        __syncthreads();
+        group_sync(g);  // Xs is refilled by the next tile's prefetch
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");  // no copy may land after the exit
-    if (!ok) drain_after_timeout(bar, phase);
+    if (!ok && tid == 0) tc::mbar_wait(bar, phase ^ 1u, kDrainPolls);  // as drain_after_timeout
     tc::fence_before();
     __syncthreads();
-    if (warp == 0) {
-        tc::tmem_dealloc(tmem, 256);
+    if (threadIdx.x < 32) {
+        tc::tmem_dealloc(*tslot, 512);
         tc::tmem_relinquish();
     }
     if (!ok && tid == 0) atomicExch(err, (int)AVBD_ERR_BARRIER_TIMEOUT);
 }
 
 // ------------------------------------------------------ training kernels
-// Z [B x N] += bias (kept as the pre-activation); H = act(Z) in BF16, both
-// row-major [B][N] and transposed [N][B]
-__global__ void k_bias_act(float* Z, const float* bias, unsigned B, unsigned N, bool act, bf16* H, bf16* HT) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)B * N) return;
-    unsigned r = (unsigned)(i / N), c = (unsigned)(i % N);
-    float z = Z[i] + bias[c];
-    Z[i] = z;
-    float h = act ? silu(z) : z;
-    bf16 hb = __float2bfloat16_rn(h);
-    if (H) H[i] = hb;
-    if (HT) HT[(size_t)c * B + r] = hb;
+// Shared memory of the fused training pass: weights, the feature tile, the
+// three activations (each overwritten by its layer's gradient in the backward
+// pass), dY, biases, bias gradients.
+constexpr unsigned TR_X = SM_X, TR_H = TR_X + 8192, TR_DY = TR_H + 3 * 32768, TR_BIAS = TR_DY + 4096,
+                   TR_DB = TR_BIAS + 1600, TR_LOSS = TR_DB + 1600, TR_BAR = TR_LOSS + 8, TR_TSLOT = TR_BAR + 8,
+                   TR_TOTAL = TR_TSLOT + 8;
+
+// descriptors of the same stored matrix (rows r, columns c; R rows) as a
+// K-major operand (K along c) and as an MN-major one (K along r)
+AVBD_D uint64_t desc_k(uint32_t a, uint32_t R, unsigned step) { return tc::sdesc(a + step * 2 * R * 16, R * 16, 128); }
+AVBD_D uint64_t desc_mn(uint32_t a, uint32_t R, unsigned step) { return tc::sdesc(a + step * 256, 128, R * 16); }
+
+// Sums over a warp's 32 rows of 16 columns: halves are exchanged and kept, so
+// that lane l ends with column (l / 2) of the 16 (16 shuffles instead of 80).
+AVBD_D float column_sum16(const float (&d)[16], unsigned lane) {
+    float a[8], b[4], e[2];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const float keep = lane & 16u ? d[j + 8] : d[j], give = lane & 16u ? d[j] : d[j + 8];
+        a[j] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const float keep = lane & 8u ? a[j + 4] : a[j], give = lane & 8u ? a[j] : a[j + 4];
+        b[j] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+    }
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        const float keep = lane & 4u ? b[j + 2] : b[j], give = lane & 4u ? b[j] : b[j + 2];
+        e[j] = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+    }
+    const float keep = lane & 2u ? e[1] : e[0], give = lane & 2u ? e[0] : e[1];
+    const float f = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+    return f + __shfl_xor_sync(0xffffffffu, f, 1);
 }
 
-// loss = mean over rows and the 3 outputs of w (y - t)^2, w the row's
-// weight (target column 3); dY = dloss/dy in BF16 ([B][16] and [16][B]);
-// db4 += column sums
-__global__ void k_loss(const float* Y, const float* T, unsigned B, bf16* dY, bf16* dYT, float* loss, float* db4) {
-    unsigned r = blockIdx.x * blockDim.x + threadIdx.x;
-    float l = 0, g[AVBD_MLP_OUT] = {0, 0, 0};
-    if (r < B) {
-        const float w = T[(size_t)r * 4 + 3];
+AVBD_D void red_add4(float* p, float a, float b, float c, float d) {
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d)
+                 : "memory");
+}
+
+// Forward and backward of a mini-batch, 128 rows a tile, one CTA per SM: the
+// pre-activations stay in tensor memory (3 x 128 FP32 columns, the fourth
+// 128 take the output and the activation gradients), the activations in
+// shared memory, and each weight gradient of the tile accumulates where its
+// layer's pre-activations were, to be added to G with 16-byte reductions.
+// The transposed operands (dZ^T, H^T, W) are the stored ones read MN-major.
+// Replaces 26 launches that passed every layer through memory twice (once
+// transposed), one of them with an atomic per element on 128 addresses: a
+// mini-batch of 8,192 took 0.42 ms of them.
+// loss = mean over rows and the 3 outputs of w (y - t)^2, w the row's weight
+// (target column 3); precisions as in the separate kernels: Z, dH and the
+// accumulators FP32, H, dY and dZ rounded to BF16, bias gradients summed from
+// the unrounded FP32 values.
+__global__ void __launch_bounds__(512, 1) k_train(MlpW w, const bf16* __restrict__ feat, const float* __restrict__ T,
+                                                   unsigned B, float* __restrict__ G, float* loss, int* err) {
+    extern __shared__ __align__(1024) uint8_t sm[];
+    uint8_t *W1s = sm + SM_W1, *W2s = sm + SM_W2, *W3s = sm + SM_W3, *W4s = sm + SM_W4;
+    uint8_t *Xs = sm + TR_X, *dYs = sm + TR_DY;
+    uint8_t* Hs[3] = {sm + TR_H, sm + TR_H + 32768, sm + TR_H + 65536};
+    float* bias = reinterpret_cast<float*>(sm + TR_BIAS);
+    float* db = reinterpret_cast<float*>(sm + TR_DB);
+    float* lsum = reinterpret_cast<float*>(sm + TR_LOSS);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + TR_BAR);
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + TR_TSLOT);
+    const unsigned tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    load_kmaj(W1s, w.w1, IN, HID, IN, HID, tid, 512);
+    load_kmaj(W2s, w.w2, HID, HID, HID, HID, tid, 512);
+    load_kmaj(W3s, w.w3, HID, HID, HID, HID, tid, 512);
+    load_kmaj(W4s, w.w4, HID, OUT, HID, OUT, tid, 512);
+    for (unsigned i = tid; i < 3 * HID + OUT; i += 512) {
+        bias[i] = w.b[i];
+        db[i] = 0.f;
+    }
+    if (tid == 0) *lsum = 0.f;
+    if (warp == 0) tc::tmem_alloc(tslot, 512);
+    if (tid == 0) tc::mbar_init(bar, 1);
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    const uint32_t tmem = *tslot, work = tmem + 384;
+    const uint32_t id_h = tc::idesc_bf16(128, HID), id_o = tc::idesc_bf16(128, OUT);
+    const uint32_t id_hb = tc::idesc_bf16(128, HID, false, true);  // dH = dZ W: B MN-major
+    const uint32_t id_w = tc::idesc_bf16(128, HID, true, true), id_w1 = tc::idesc_bf16(128, IN, true, true),
+                   id_w4 = tc::idesc_bf16(128, OUT, true, true);   // dW: both MN-major
+    // this thread's part of a 128 x 128 accumulator: row r, columns c0 .. c0 + 31
+    const unsigned q = warp & 3u, c0 = (warp >> 2) * 32, r = q * 32 + lane;
+    const uint32_t trow = (q * 32u) << 16;
+    uint32_t phase = 0;
+    bool ok = true;
+    // operands written by all threads are ready and the accumulators read: issue, then wait
+    auto run = [&](auto&& products, auto&& meanwhile) {
+        tc::fence_before();
+        tc::fence_async_smem();
+        __syncthreads();
+        if (tid == 0) {
+            tc::fence_after();
+            products();
+            tc::commit(bar);
+        }
+        __syncwarp();
+        meanwhile();
+        ok = block_wait(bar, phase);
+        tc::fence_after();
+        return ok;
+    };
+    auto nothing = [] {};
+    auto product = [&](uint32_t d, const uint8_t* A, bool a_mn, const uint8_t* Bm, unsigned b_rows, bool b_mn,
+                       unsigned ksteps, uint32_t id) {
+        const uint32_t a = tc::smem_u32(A), bb = tc::smem_u32(Bm);
+        for (unsigned s = 0; s < ksteps; s++)
+            tc::mma_bf16(d, a_mn ? desc_mn(a, 128, s) : desc_k(a, 128, s),
+                         b_mn ? desc_mn(bb, b_rows, s) : desc_k(bb, b_rows, s), id, s > 0 ? 1u : 0u);
+    };
+    // hidden layer's activation: Z + b -> SiLU -> BF16 into H
+    auto activate = [&](uint32_t z, const float* b, uint8_t* H) {
 #pragma unroll
-        for (int j = 0; j < (int)OUT; j++) {
-            float d = 0;
-            if (j < AVBD_MLP_OUT) {
-                float e = Y[(size_t)r * OUT + j] - T[(size_t)r * 4 + j];
-                l += w * e * e;
-                d = 2.0f * w * e / (float)(B * AVBD_MLP_OUT);
-                g[j] = d;
+        for (unsigned c = 0; c < 32; c += 16) {
+            float v[16];
+            tc::tmem_ld16(z + trow + c0 + c, v);
+            uint32_t pk[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+                pk[j] = pack2(silu(v[2 * j] + b[c0 + c + 2 * j]), silu(v[2 * j + 1] + b[c0 + c + 2 * j + 1]));
+            uint8_t* d = H + ((c0 + c) / 8) * 2048 + r * 16;
+            *reinterpret_cast<uint4*>(d) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            *reinterpret_cast<uint4*>(d + 2048) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+        }
+    };
+    // dZ = dH silu'(Z + b) -> BF16 into H's buffer; bias gradient
+    auto activate_grad = [&](uint32_t z, const float* b, uint8_t* H, float* dbl) {
+#pragma unroll
+        for (unsigned c = 0; c < 32; c += 16) {
+            float v[16], d[16];
+            tc::tmem_ld16(z + trow + c0 + c, v);
+            tc::tmem_ld16(work + trow + c0 + c, d);
+#pragma unroll
+            for (int j = 0; j < 16; j++) d[j] *= silu_grad(v[j] + b[c0 + c + j]);
+            uint8_t* o = H + ((c0 + c) / 8) * 2048 + r * 16;
+            *reinterpret_cast<uint4*>(o) = make_uint4(pack2(d[0], d[1]), pack2(d[2], d[3]), pack2(d[4], d[5]), pack2(d[6], d[7]));
+            *reinterpret_cast<uint4*>(o + 2048) =
+                make_uint4(pack2(d[8], d[9]), pack2(d[10], d[11]), pack2(d[12], d[13]), pack2(d[14], d[15]));
+            const float t = column_sum16(d, lane);
+            if (!(lane & 1u)) atomicAdd(dbl + c0 + c + (lane >> 1), t);
+        }
+    };
+    // a tile's weight gradient [128][128] added to G
+    auto flush = [&](uint32_t acc, float* g) {
+#pragma unroll
+        for (unsigned c = 0; c < 32; c += 16) {
+            float v[16];
+            tc::tmem_ld16(acc + trow + c0 + c, v);
+#pragma unroll
+            for (int j = 0; j < 16; j += 4) red_add4(g + r * HID + c0 + c + j, v[j], v[j + 1], v[j + 2], v[j + 3]);
+        }
+    };
+
+    for (unsigned tile = blockIdx.x; tile < B / 128; tile += gridDim.x) {
+        const unsigned row0 = tile * 128;
+        load_x_async(Xs, feat + (size_t)row0 * IN, 128, tid, 512);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        // forward
+        if (!run([&] { product(tmem, Xs, false, W1s, HID, false, IN / 16, id_h); }, nothing)) break;
+        activate(tmem, bias, Hs[0]);
+        if (!run([&] { product(tmem + 128, Hs[0], false, W2s, HID, false, HID / 16, id_h); }, nothing)) break;
+        activate(tmem + 128, bias + HID, Hs[1]);
+        if (!run([&] { product(tmem + 256, Hs[1], false, W3s, HID, false, HID / 16, id_h); }, nothing)) break;
+        activate(tmem + 256, bias + 2 * HID, Hs[2]);
+        if (!run([&] { product(work, Hs[2], false, W4s, OUT, false, HID / 16, id_o); }, nothing)) break;
+        // loss, dY
+        if (warp < 4) {
+            float v[16], d[16];
+            tc::tmem_ld16(work + trow, v);
+            const float* t = T + (size_t)(row0 + r) * 4;
+            const float wt = t[3];
+            float l = 0.f;
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                d[j] = 0.f;
+                if (j < AVBD_MLP_OUT) {
+                    const float e = (v[j] + bias[3 * HID + j]) - t[j];
+                    l += wt * e * e;
+                    d[j] = 2.0f * wt * e / (float)(B * AVBD_MLP_OUT);
+                }
             }
-            bf16 db = __float2bfloat16_rn(d);
-            dY[(size_t)r * OUT + j] = db;
-            dYT[(size_t)j * B + r] = db;
+            *reinterpret_cast<uint4*>(dYs + r * 16) =
+                make_uint4(pack2(d[0], d[1]), pack2(d[2], d[3]), pack2(d[4], d[5]), pack2(d[6], d[7]));
+            *reinterpret_cast<uint4*>(dYs + 2048 + r * 16) = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+            for (int m = 16; m >= 1; m >>= 1) {
+                l += __shfl_xor_sync(0xffffffffu, l, m);
+#pragma unroll
+                for (int j = 0; j < AVBD_MLP_OUT; j++) d[j] += __shfl_xor_sync(0xffffffffu, d[j], m);
+            }
+            if (lane == 0) {
+                atomicAdd(lsum, l / (float)(B * AVBD_MLP_OUT));
+#pragma unroll
+                for (int j = 0; j < AVBD_MLP_OUT; j++) atomicAdd(db + 3 * HID + j, d[j]);
+            }
+        }
+        // dW4^T = H3^T dY, then dH3 = dY W4
+        if (!run([&] { product(work, Hs[2], true, dYs, 128, true, 8, id_w4); }, nothing)) break;
+        if (warp < 4) {
+            float v[16];
+            tc::tmem_ld16(work + trow, v);
+#pragma unroll
+            for (int j = 0; j < AVBD_MLP_OUT; j++) atomicAdd(G + OFF_W4 + j * HID + r, v[j]);
+        }
+        if (!run([&] { product(work, dYs, false, W4s, OUT, true, 1, id_hb); }, nothing)) break;
+        // layer 3
+        activate_grad(tmem + 256, bias + 2 * HID, Hs[2], db + 2 * HID);
+        if (!run([&] {
+                product(tmem + 256, Hs[2], true, Hs[1], 128, true, 8, id_w);
+                product(work, Hs[2], false, W3s, HID, true, HID / 16, id_hb);
+            }, nothing))
+            break;
+        // layer 2, layer 3's gradient flushed beside its products
+        activate_grad(tmem + 128, bias + HID, Hs[1], db + HID);
+        if (!run([&] {
+                product(tmem + 128, Hs[1], true, Hs[0], 128, true, 8, id_w);
+                product(work, Hs[1], false, W2s, HID, true, HID / 16, id_hb);
+            }, [&] { flush(tmem + 256, G + OFF_W3); }))
+            break;
+        // layer 1
+        activate_grad(tmem, bias, Hs[0], db);
+        if (!run([&] { product(tmem, Hs[0], true, Xs, 128, true, 8, id_w1); }, [&] { flush(tmem + 128, G + OFF_W2); })) break;
+        if (warp < 8) {  // [128][32]: warp w rows 32 (w % 4).., columns 16 (w / 4)..
+            const unsigned cc = (warp >> 2) * 16;
+            float v[16];
+            tc::tmem_ld16(tmem + trow + cc, v);
+#pragma unroll
+            for (int j = 0; j < 16; j += 4)
+                red_add4(G + OFF_W1 + r * IN + cc + j, v[j], v[j + 1], v[j + 2], v[j + 3]);
         }
     }
-#pragma unroll
-    for (int m = 16; m >= 1; m >>= 1) {
-        l += __shfl_xor_sync(0xffffffffu, l, m);
-#pragma unroll
-        for (int j = 0; j < AVBD_MLP_OUT; j++) g[j] += __shfl_xor_sync(0xffffffffu, g[j], m);
+    if (!ok) drain_after_timeout(bar, phase);
+    tc::fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc::tmem_dealloc(tmem, 512);
+        tc::tmem_relinquish();
     }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(loss, l / (float)(B * AVBD_MLP_OUT));
-        for (int j = 0; j < AVBD_MLP_OUT; j++) atomicAdd(db4 + j, g[j]);
+    if (tid < HID) {
+        atomicAdd(G + OFF_B1 + tid, db[tid]);
+        atomicAdd(G + OFF_B2 + tid, db[HID + tid]);
+        atomicAdd(G + OFF_B3 + tid, db[2 * HID + tid]);
+    }
+    if (tid < AVBD_MLP_OUT) atomicAdd(G + OFF_B4 + tid, db[3 * HID + tid]);
+    if (tid == 0) {
+        atomicAdd(loss, *lsum);
+        if (!ok) atomicExch(err, (int)AVBD_ERR_BARRIER_TIMEOUT);
     }
 }
 
-// dZ = dH * silu'(Z) in BF16 ([B][N] and [N][B]); db += column sums
-__global__ void k_act_grad(const float* dH, const float* Z, unsigned B, unsigned N, bf16* dZ, bf16* dZT, float* db) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)B * N) return;
-    unsigned r = (unsigned)(i / N), c = (unsigned)(i % N);
-    float d = dH[i] * silu_grad(Z[i]);
-    bf16 b = __float2bfloat16_rn(d);
-    dZ[i] = b;
-    dZT[(size_t)c * B + r] = b;
-    atomicAdd(db + c, d);
+// one master FP32 parameter into its BF16 weight or FP32 bias
+AVBD_D void pack_param(unsigned i, float p, bf16* w1, bf16* w2, bf16* w3, bf16* w4, float* b) {
+    if (i < OFF_B1) w1[i] = __float2bfloat16_rn(p);
+    else if (i < OFF_W2) b[i - OFF_B1] = p;
+    else if (i < OFF_B2) w2[i - OFF_W2] = __float2bfloat16_rn(p);
+    else if (i < OFF_W3) b[HID + i - OFF_B2] = p;
+    else if (i < OFF_B3) w3[i - OFF_W3] = __float2bfloat16_rn(p);
+    else if (i < OFF_W4) b[2 * HID + i - OFF_B3] = p;
+    else if (i < OFF_B4) w4[i - OFF_W4] = __float2bfloat16_rn(p);
+    else b[3 * HID + i - OFF_B4] = p;
 }
 
-__global__ void k_transpose_bf16(const bf16* src, unsigned R, unsigned Cc, unsigned lds, bf16* dst) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)R * Cc) return;
-    unsigned r = (unsigned)(i / Cc), c = (unsigned)(i % Cc);
-    dst[(size_t)c * R + r] = src[(size_t)r * lds + c];
-}
-
-__global__ void k_transpose_f32(const float* src, unsigned R, unsigned Cc, float* dst) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)R * Cc) return;
-    unsigned r = (unsigned)(i / Cc), c = (unsigned)(i % Cc);
-    dst[(size_t)c * R + r] = src[i];
-}
-
-// master FP32 parameters -> BF16 weights ([out][in] and [in][out]) and FP32
-// biases of the four layers
-__global__ void k_pack(const float* P, bf16* w1, bf16* w2, bf16* w3, bf16* w4, bf16* w1t, bf16* w2t, bf16* w3t,
-                       bf16* w4t, float* b) {
+__global__ void k_pack(const float* P, bf16* w1, bf16* w2, bf16* w3, bf16* w4, float* b) {
     unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < HID * IN) {
-        unsigned o = i / IN, k = i % IN;
-        bf16 v = __float2bfloat16_rn(P[OFF_W1 + i]);
-        w1[i] = v;
-        if (w1t) w1t[k * HID + o] = v;
-    }
-    if (i < HID * HID) {
-        unsigned o = i / HID, k = i % HID;
-        bf16 v2 = __float2bfloat16_rn(P[OFF_W2 + i]), v3 = __float2bfloat16_rn(P[OFF_W3 + i]);
-        w2[i] = v2;
-        w3[i] = v3;
-        if (w2t) w2t[k * HID + o] = v2;
-        if (w3t) w3t[k * HID + o] = v3;
-    }
-    if (i < OUT * HID) {
-        unsigned o = i / HID, k = i % HID;
-        bf16 v = __float2bfloat16_rn(P[OFF_W4 + i]);
-        w4[i] = v;
-        if (w4t) w4t[k * OUT + o] = v;
-    }
-    if (i < HID) {
-        b[i] = P[OFF_B1 + i];
-        b[HID + i] = P[OFF_B2 + i];
-        b[2 * HID + i] = P[OFF_B3 + i];
-    }
-    if (i < OUT) b[3 * HID + i] = P[OFF_B4 + i];
+    if (i < NPAR) pack_param(i, P[i], w1, w2, w3, w4, b);
 }
 
 // padding that must stay zero: inputs 27..31 of W1, outputs 3..15 of W4 / b4
@@ -528,7 +695,9 @@ AVBD_D bool frozen(unsigned i) {
     return false;
 }
 
-__global__ void k_adam(float* P, const float* G, float* Mo, float* Vo, float lr, float c1, float c2) {
+// Adam on the master parameters, which are packed again as they change
+__global__ void k_adam(float* P, const float* G, float* Mo, float* Vo, float lr, float c1, float c2, bf16* w1, bf16* w2,
+                       bf16* w3, bf16* w4, float* b) {
     unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= NPAR || frozen(i)) return;
     float g = G[i];
@@ -536,7 +705,9 @@ __global__ void k_adam(float* P, const float* G, float* Mo, float* Vo, float lr,
     float v = 0.999f * Vo[i] + 0.001f * g * g;
     Mo[i] = m;
     Vo[i] = v;
-    P[i] -= lr * (m / c1) / (sqrtf(v / c2) + 1e-8f);
+    const float p = P[i] - lr * (m / c1) / (sqrtf(v / c2) + 1e-8f);
+    P[i] = p;
+    pack_param(i, p, w1, w2, w3, w4, b);
 }
 
 inline unsigned nb(size_t n, unsigned per) { return (unsigned)((n + per - 1) / per); }
@@ -550,6 +721,7 @@ struct MlpDevice {
     float* p32 = nullptr;
     int* err = nullptr;
     int device = 0;
+    bool own_err = true;
     int upload(const float* params, cudaStream_t st);
     void release();
 };
@@ -567,13 +739,13 @@ int MlpDevice::upload(const float* params, cudaStream_t st) {
     }
     if (cudaMemcpyAsync(p32, params, sizeof(float) * NPAR, cudaMemcpyHostToDevice, st) != cudaSuccess)
         return set_error(AVBD_ERR_CUDA, "MLP parameter upload failed");
-    k_pack<<<nb(HID * HID, 256), 256, 0, st>>>(p32, w1, w2, w3, w4, nullptr, nullptr, nullptr, nullptr, b);
+    k_pack<<<nb(NPAR, 256), 256, 0, st>>>(p32, w1, w2, w3, w4, b);
     cudaError_t e = cudaStreamSynchronize(st);
     return e == cudaSuccess ? AVBD_OK : set_error(AVBD_ERR_CUDA, cudaGetErrorString(e));
 }
 
 void MlpDevice::release() {
-    for (void* p : {(void*)w1, (void*)w2, (void*)w3, (void*)w4, (void*)b, (void*)p32, (void*)err})
+    for (void* p : {(void*)w1, (void*)w2, (void*)w3, (void*)w4, (void*)b, (void*)p32, own_err ? (void*)err : nullptr})
         if (p) cudaFree(p);
     w1 = w2 = w3 = w4 = nullptr;
     b = p32 = nullptr;
@@ -598,7 +770,7 @@ static int mlp_launch(const MlpDevice& m, const bf16* feat, unsigned n, const Ml
         done.fetch_or(bit);
     }
     MlpW w{m.w1, m.w2, m.w3, m.w4, m.b};
-    k_mlp_apply<P><<<grid_for(m.device, n), 512, SM_TOTAL, st>>>(w, feat, n, sink, m.err);
+    k_mlp_apply<P><<<grid_for(m.device, n), GROUPS * GTHREADS, SM_TOTAL, st>>>(w, feat, n, sink, m.err);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? AVBD_OK : set_error(AVBD_ERR_CUDA, cudaGetErrorString(e));
 }
@@ -658,13 +830,8 @@ struct avbd_mlp_trainer {
     unsigned B = 0;
     cudaStream_t st = nullptr;
     MlpDevice w;                  // BF16 [out][in] weights + biases
-    bf16 *w1t = nullptr, *w2t = nullptr, *w3t = nullptr, *w4t = nullptr;  // [in][out]
-    float *G = nullptr, *Mo = nullptr, *Vo = nullptr;
-    float *Z1 = nullptr, *Z2 = nullptr, *Z3 = nullptr, *Y = nullptr;      // [B][128] x3, [B][16]
-    bf16 *H1 = nullptr, *H2 = nullptr, *H3 = nullptr;                     // [B][128]
-    bf16 *H1T = nullptr, *H2T = nullptr, *H3T = nullptr, *XT = nullptr;   // [128][B] x3, [32][B]
-    bf16 *dY = nullptr, *dYT = nullptr, *dZ = nullptr, *dZT = nullptr;    // [B][16], [16][B], [B][128], [128][B]
-    float *dH = nullptr, *dW4T = nullptr, *loss = nullptr;                // [B][128], [128][16], 1
+    float *G = nullptr, *Mo = nullptr, *Vo = nullptr;  // G: gradient, then the loss and the kernels' error flag
+    float* status = nullptr;      // pinned host copy of the loss and the flag
     unsigned t = 0;
     std::vector<void*> allocs;
 };
@@ -743,24 +910,14 @@ int avbd_mlp_trainer_create(avbd_mlp_trainer** out, int device, unsigned batch, 
     t->device = device;
     t->B = batch;
     cudaStreamCreateWithFlags(&t->st, cudaStreamNonBlocking);
-    const size_t B = batch;
     bool bad = false;
     auto al = [&](auto** p, size_t bytes) {
         if (bad) return;
         if (cudaMalloc((void**)p, bytes) != cudaSuccess) bad = true;
         else t->allocs.push_back((void*)*p);
     };
-    al(&t->w1t, sizeof(bf16) * HID * IN); al(&t->w2t, sizeof(bf16) * HID * HID);
-    al(&t->w3t, sizeof(bf16) * HID * HID); al(&t->w4t, sizeof(bf16) * OUT * HID);
-    al(&t->G, sizeof(float) * NPAR); al(&t->Mo, sizeof(float) * NPAR); al(&t->Vo, sizeof(float) * NPAR);
-    al(&t->Z1, sizeof(float) * B * HID); al(&t->Z2, sizeof(float) * B * HID); al(&t->Z3, sizeof(float) * B * HID);
-    al(&t->Y, sizeof(float) * B * OUT);
-    al(&t->H1, sizeof(bf16) * B * HID); al(&t->H2, sizeof(bf16) * B * HID); al(&t->H3, sizeof(bf16) * B * HID);
-    al(&t->H1T, sizeof(bf16) * B * HID); al(&t->H2T, sizeof(bf16) * B * HID); al(&t->H3T, sizeof(bf16) * B * HID);
-    al(&t->XT, sizeof(bf16) * B * IN);
-    al(&t->dY, sizeof(bf16) * B * OUT); al(&t->dYT, sizeof(bf16) * B * OUT);
-    al(&t->dZ, sizeof(bf16) * B * HID); al(&t->dZT, sizeof(bf16) * B * HID);
-    al(&t->dH, sizeof(float) * B * HID); al(&t->dW4T, sizeof(float) * HID * OUT); al(&t->loss, sizeof(float));
+    al(&t->G, sizeof(float) * (NPAR + 2)); al(&t->Mo, sizeof(float) * NPAR); al(&t->Vo, sizeof(float) * NPAR);
+    if (!bad && cudaMallocHost((void**)&t->status, 2 * sizeof(float)) != cudaSuccess) bad = true;
     if (bad) {
         avbd_mlp_trainer_destroy(t);
         return set_error(AVBD_ERR_CUDA, "trainer allocation failed");
@@ -772,8 +929,12 @@ int avbd_mlp_trainer_create(avbd_mlp_trainer** out, int device, unsigned batch, 
     }
     cudaMemsetAsync(t->Mo, 0, sizeof(float) * NPAR, t->st);
     cudaMemsetAsync(t->Vo, 0, sizeof(float) * NPAR, t->st);
-    k_pack<<<nb(HID * HID, 256), 256, 0, t->st>>>(t->w.p32, t->w.w1, t->w.w2, t->w.w3, t->w.w4, t->w1t, t->w2t,
-                                                  t->w3t, t->w4t, t->w.b);
+    // the flag lies behind the loss, so that one copy reads both
+    cudaFree(t->w.err);
+    t->w.err = reinterpret_cast<int*>(t->G + NPAR + 1);
+    t->w.own_err = false;
+    cudaMemsetAsync(t->G, 0, sizeof(float) * (NPAR + 2), t->st);
+    cudaFuncSetAttribute(k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, TR_TOTAL);
     if (cudaStreamSynchronize(t->st) != cudaSuccess) {
         avbd_mlp_trainer_destroy(t);
         return set_error(AVBD_ERR_CUDA, "trainer initialisation failed");
@@ -782,67 +943,46 @@ int avbd_mlp_trainer_create(avbd_mlp_trainer** out, int device, unsigned batch, 
     return AVBD_OK;
 }
 
-// forward + backward of one mini-batch into t->G (and t->loss)
+// forward + backward of one mini-batch into t->G (and the loss behind it)
 static int trainer_fwd_bwd(avbd_mlp_trainer* t, const bf16* X, const float* T) {
-    const unsigned B = t->B;
-    cudaStream_t st = t->st;
-    int* err = t->w.err;
-    const float* b = t->w.b;
-    int rc;
-    cudaMemsetAsync(t->G, 0, sizeof(float) * NPAR, st);
-    cudaMemsetAsync(t->loss, 0, sizeof(float), st);
-    // forward
-    if ((rc = gemm_bf16(X, IN, t->w.w1, IN, t->Z1, HID, B, HID, IN, false, st, err))) return rc;
-    k_bias_act<<<nb((size_t)B * HID, 256), 256, 0, st>>>(t->Z1, b, B, HID, true, t->H1, t->H1T);
-    if ((rc = gemm_bf16(t->H1, HID, t->w.w2, HID, t->Z2, HID, B, HID, HID, false, st, err))) return rc;
-    k_bias_act<<<nb((size_t)B * HID, 256), 256, 0, st>>>(t->Z2, b + HID, B, HID, true, t->H2, t->H2T);
-    if ((rc = gemm_bf16(t->H2, HID, t->w.w3, HID, t->Z3, HID, B, HID, HID, false, st, err))) return rc;
-    k_bias_act<<<nb((size_t)B * HID, 256), 256, 0, st>>>(t->Z3, b + 2 * HID, B, HID, true, t->H3, t->H3T);
-    if ((rc = gemm_bf16(t->H3, HID, t->w.w4, HID, t->Y, OUT, B, OUT, HID, false, st, err))) return rc;
-    k_bias_act<<<nb((size_t)B * OUT, 256), 256, 0, st>>>(t->Y, b + 3 * HID, B, OUT, false, nullptr, nullptr);
-    k_transpose_bf16<<<nb((size_t)B * IN, 256), 256, 0, st>>>(X, B, IN, IN, t->XT);
-    // loss and output layer
-    k_loss<<<nb(B, 256), 256, 0, st>>>(t->Y, T, B, t->dY, t->dYT, t->loss, t->G + OFF_B4);
-    if ((rc = gemm_bf16(t->H3T, B, t->dYT, B, t->dW4T, OUT, HID, OUT, B, false, st, err))) return rc;
-    k_transpose_f32<<<nb(HID * OUT, 256), 256, 0, st>>>(t->dW4T, HID, OUT, t->G + OFF_W4);
-    if ((rc = gemm_bf16(t->dY, OUT, t->w4t, OUT, t->dH, HID, B, HID, OUT, false, st, err))) return rc;
-    // layer 3
-    k_act_grad<<<nb((size_t)B * HID, 256), 256, 0, st>>>(t->dH, t->Z3, B, HID, t->dZ, t->dZT, t->G + OFF_B3);
-    if ((rc = gemm_bf16(t->dZT, B, t->H2T, B, t->G + OFF_W3, HID, HID, HID, B, false, st, err))) return rc;
-    if ((rc = gemm_bf16(t->dZ, HID, t->w3t, HID, t->dH, HID, B, HID, HID, false, st, err))) return rc;
-    // layer 2
-    k_act_grad<<<nb((size_t)B * HID, 256), 256, 0, st>>>(t->dH, t->Z2, B, HID, t->dZ, t->dZT, t->G + OFF_B2);
-    if ((rc = gemm_bf16(t->dZT, B, t->H1T, B, t->G + OFF_W2, HID, HID, HID, B, false, st, err))) return rc;
-    if ((rc = gemm_bf16(t->dZ, HID, t->w2t, HID, t->dH, HID, B, HID, HID, false, st, err))) return rc;
-    // layer 1
-    k_act_grad<<<nb((size_t)B * HID, 256), 256, 0, st>>>(t->dH, t->Z1, B, HID, t->dZ, t->dZT, t->G + OFF_B1);
-    if ((rc = gemm_bf16(t->dZT, B, t->XT, B, t->G + OFF_W1, IN, HID, IN, B, false, st, err))) return rc;
+    cudaMemsetAsync(t->G, 0, sizeof(float) * (NPAR + 1), t->st);
+    const MlpW w{t->w.w1, t->w.w2, t->w.w3, t->w.w4, t->w.b};
+    k_train<<<grid_for(t->device, t->B), 512, TR_TOTAL, t->st>>>(w, X, T, t->B, t->G, t->G + NPAR, t->w.err);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? AVBD_OK : set_error(AVBD_ERR_CUDA, cudaGetErrorString(e));
 }
 
-int avbd_mlp_trainer_grad(avbd_mlp_trainer* t, const void* features, const float* targets, float* loss, float* grad) {
-    if (!t || !features || !targets) return set_error(AVBD_ERR_INVALID_ARG, "null argument");
-    if (int rc = trainer_fwd_bwd(t, (const bf16*)features, targets)) return rc;
-    if (loss) cudaMemcpyAsync(loss, t->loss, sizeof(float), cudaMemcpyDeviceToHost, t->st);
-    if (grad) cudaMemcpyAsync(grad, t->G, sizeof(float) * NPAR, cudaMemcpyDeviceToHost, t->st);
+// waits for the stream and reads the loss and the error flag
+static int trainer_status(avbd_mlp_trainer* t, float* loss) {
+    cudaMemcpyAsync(t->status, t->G + NPAR, 2 * sizeof(float), cudaMemcpyDeviceToHost, t->st);
     if (cudaStreamSynchronize(t->st) != cudaSuccess) return set_error(AVBD_ERR_CUDA, "trainer sync failed");
-    return mlp_device_error(&t->w, t->st);
+    if (loss) *loss = t->status[0];
+    int flag;
+    std::memcpy(&flag, t->status + 1, sizeof(flag));
+    return flag ? mlp_device_error(&t->w, t->st) : AVBD_OK;
+}
+
+static int trainer_args(avbd_mlp_trainer* t, const void* features, const float* targets) {
+    if (!t || !features || !targets) return set_error(AVBD_ERR_INVALID_ARG, "null argument");
+    if ((uintptr_t)features & 15) return set_error(AVBD_ERR_INVALID_ARG, "features must be 16-byte aligned");
+    return AVBD_OK;
+}
+
+int avbd_mlp_trainer_grad(avbd_mlp_trainer* t, const void* features, const float* targets, float* loss, float* grad) {
+    if (int rc = trainer_args(t, features, targets)) return rc;
+    if (int rc = trainer_fwd_bwd(t, (const bf16*)features, targets)) return rc;
+    if (grad) cudaMemcpyAsync(grad, t->G, sizeof(float) * NPAR, cudaMemcpyDeviceToHost, t->st);
+    return trainer_status(t, loss);
 }
 
 int avbd_mlp_trainer_step(avbd_mlp_trainer* t, const void* features, const float* targets, float lr, float* loss) {
-    if (!t || !features || !targets) return set_error(AVBD_ERR_INVALID_ARG, "null argument");
+    if (int rc = trainer_args(t, features, targets)) return rc;
     if (int rc = trainer_fwd_bwd(t, (const bf16*)features, targets)) return rc;
     t->t++;
     const float c1 = 1.0f - powf(0.9f, (float)t->t), c2 = 1.0f - powf(0.999f, (float)t->t);
-    k_adam<<<nb(NPAR, 256), 256, 0, t->st>>>(t->w.p32, t->G, t->Mo, t->Vo, lr, c1, c2);
-    k_pack<<<nb(HID * HID, 256), 256, 0, t->st>>>(t->w.p32, t->w.w1, t->w.w2, t->w.w3, t->w.w4, t->w1t, t->w2t,
-                                                  t->w3t, t->w4t, t->w.b);
-    if (loss) {
-        cudaMemcpyAsync(loss, t->loss, sizeof(float), cudaMemcpyDeviceToHost, t->st);
-        if (cudaStreamSynchronize(t->st) != cudaSuccess) return set_error(AVBD_ERR_CUDA, "trainer sync failed");
-        return mlp_device_error(&t->w, t->st);
-    }
+    k_adam<<<nb(NPAR, 256), 256, 0, t->st>>>(t->w.p32, t->G, t->Mo, t->Vo, lr, c1, c2, t->w.w1, t->w.w2, t->w.w3,
+                                             t->w.w4, t->w.b);
+    if (loss) return trainer_status(t, loss);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? AVBD_OK : set_error(AVBD_ERR_CUDA, cudaGetErrorString(e));
 }
@@ -858,6 +998,7 @@ int avbd_mlp_trainer_destroy(avbd_mlp_trainer* t) {
     if (!t) return AVBD_OK;
     if (t->st) cudaStreamSynchronize(t->st);
     for (void* p : t->allocs) cudaFree(p);
+    if (t->status) cudaFreeHost(t->status);
     t->w.release();
     if (t->st) cudaStreamDestroy(t->st);
     delete t;

@@ -10,6 +10,11 @@
 // the descriptor's stride byte offset (between 8-row groups) is 128 and its
 // leading byte offset (between K chunks) is R * 16.  One MMA consumes K = 16
 // (two chunks); the next K step starts 2 * R * 16 bytes further.
+//
+// The same bytes serve as the transposed operand: read MN-major (the operand's
+// M or N index along k, its K index along r), the core matrices are R * 16
+// bytes apart along M / N (stride byte offset) and 128 along K (leading byte
+// offset), and the next K step starts 256 bytes further.
 #pragma once
 
 #include <cstdint>
@@ -36,9 +41,11 @@ AVBD_D uint64_t sdesc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
     return d;
 }
 
-// instruction descriptor, kind::f16: D F32, A and B BF16, both K-major, dense
-AVBD_HD constexpr uint32_t idesc_bf16(uint32_t M, uint32_t N) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
+// instruction descriptor, kind::f16: D F32, A and B BF16, dense; each operand
+// K-major or MN-major
+AVBD_HD constexpr uint32_t idesc_bf16(uint32_t M, uint32_t N, bool a_mn = false, bool b_mn = false) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) |
+           ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
 // D[tmem] (+)= A * B^T for one K = 16 step; issued by a single thread
