@@ -236,6 +236,7 @@ struct LbvhState {
     uint32_t* root = nullptr;
     uint2* pairs = nullptr;
     uint2* range = nullptr;         // leaf range [lo, hi] of each internal node
+    uint4* packed = nullptr;        // 4 per internal node: the traversal's record (lbvh.cu, PackedNode)
     uint32_t* pair_count = nullptr;
     unsigned pair_capacity = 0;
     double* xd = nullptr;           // FP64 copies of positions / velocities

@@ -53,6 +53,23 @@ AVBD_D V3<double> abs_mat_vec(const M3<double>& R, V3<double> v) {
                fabs(R.a[2][0]) * v.x + fabs(R.a[2][1]) * v.y + fabs(R.a[2][2]) * v.z);
 }
 
+// Scene box of the boxes' encoded corners: minima as they are, maxima
+// complemented, so that all six are minima of one fill pattern (0xFF bytes).
+AVBD_D void box_reduce(unsigned long long (&e)[6], unsigned long long* box) {
+#pragma unroll
+    for (int a = 0; a < 6; a++) {
+#pragma unroll
+        for (int m = 16; m >= 1; m >>= 1) {
+            const unsigned long long o = __shfl_xor_sync(0xffffffffu, e[a], m);
+            e[a] = o < e[a] ? o : e[a];
+        }
+    }
+    if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+        for (int a = 0; a < 6; a++) atomicMin(box + a, e[a]);
+    }
+}
+
 // Swept bounds of every primitive and the scene box (exact min/max through
 // order-preserving integer atomics).
 template <typename R>
@@ -135,25 +152,9 @@ __global__ void __launch_bounds__(256) k_prim_bounds(DevState<R> s, LbvhState L,
 #pragma unroll
     for (int a = 0; a < 3; a++) {
         e[a] = valid ? ord_enc(mn[a]) : ~0ull;
-        e[3 + a] = valid ? ord_enc(mx[a]) : 0ull;
+        e[3 + a] = valid ? ~ord_enc(mx[a]) : ~0ull;
     }
-#pragma unroll
-    for (int m = 16; m >= 1; m >>= 1) {
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            unsigned long long o = __shfl_xor_sync(0xffffffffu, e[a], m);
-            e[a] = o < e[a] ? o : e[a];
-            o = __shfl_xor_sync(0xffffffffu, e[3 + a], m);
-            e[3 + a] = o > e[3 + a] ? o : e[3 + a];
-        }
-    }
-    if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            atomicMin(box + a, e[a]);
-            atomicMax(box + 3 + a, e[3 + a]);
-        }
-    }
+    box_reduce(e, box);
 }
 
 AVBD_D uint64_t expand21(uint64_t v) {
@@ -168,14 +169,12 @@ AVBD_D uint64_t expand21(uint64_t v) {
 
 AVBD_D double clamp_ref(double v, double lo, double hi) { return (v < lo) ? lo : (hi < v) ? hi : v; }
 
-__global__ void __launch_bounds__(256) k_morton(LbvhState L, const unsigned long long* box) {
-    unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= L.n) return;
+AVBD_D uint64_t morton_code(const LbvhState& L, unsigned i, const unsigned long long* box) {
     double smin[3], ext[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
         smin[a] = ord_dec(box[a]);
-        double e = __dsub_rn(ord_dec(box[3 + a]), smin[a]);
+        double e = __dsub_rn(ord_dec(~box[3 + a]), smin[a]);
         ext[a] = (e < 1e-6) ? 1e-6 : e;  // extent.cwiseMax(1e-6)
     }
     uint64_t code = 0;
@@ -186,8 +185,89 @@ __global__ void __launch_bounds__(256) k_morton(LbvhState L, const unsigned long
         double q = clamp_ref(__dmul_rn(nx, 2097152.0), 0.0, 2097151.0);
         code |= expand21((uint64_t)q) << a;
     }
-    L.morton[i] = code;
+    return code;
+}
+
+__global__ void __launch_bounds__(256) k_morton(LbvhState L, const unsigned long long* box) {
+    unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= L.n) return;
+    L.morton[i] = morton_code(L, i, box);
     L.sorted[i] = i;
+}
+
+// --------------------------------------------------------- rank sort
+// Up to RANK_SORT_MAX primitives: tiles of 1,024 sorted by (code, index) in
+// shared memory, then every element counts the elements before it in the other
+// tiles by binary search.  The order is the stable radix sort's: equal codes by
+// index, and the tiles are contiguous index ranges, so an earlier tile's equal
+// codes come first.  Two launches instead of 24 (8 passes of count, scan,
+// scatter): 26,000 codes 150 us in the passes' launches.  The searches grow
+// with the square of the tiles, so larger sets keep the passes.
+constexpr unsigned SORT_TILE = 1024, RANK_SORT_MAX = 65536;
+
+__global__ void __launch_bounds__(SORT_TILE) k_sort_tiles(LbvhState L, const unsigned long long* box) {
+    __shared__ uint64_t sk[SORT_TILE];
+    __shared__ uint32_t si[SORT_TILE];
+    const unsigned t = threadIdx.x, i = blockIdx.x * SORT_TILE + t;
+    uint64_t key = i < L.n ? morton_code(L, i, box) : ~0ull;  // codes have 63 bits: the padding sorts last
+    uint32_t idx = i;
+    for (unsigned k = 2; k <= SORT_TILE; k <<= 1)
+        for (unsigned j = k >> 1; j >= 1; j >>= 1) {
+            uint64_t ok;
+            uint32_t oi;
+            if (j < 32) {
+                ok = __shfl_xor_sync(0xffffffffu, key, j);
+                oi = __shfl_xor_sync(0xffffffffu, idx, j);
+            } else {
+                __syncthreads();
+                sk[t] = key;
+                si[t] = idx;
+                __syncthreads();
+                ok = sk[t ^ j];
+                oi = si[t ^ j];
+            }
+            const bool less = ok < key || (ok == key && oi < idx);  // the partner comes first
+            const bool want_min = ((t & j) == 0) == ((t & k) == 0);
+            if (less == want_min) {
+                key = ok;
+                idx = oi;
+            }
+        }
+    if (i < L.n) {
+        L.keys_tmp[i] = key;
+        L.sorted_tmp[i] = idx;
+    }
+}
+
+// 8 lanes per element, the other tiles dealt to them.
+__global__ void __launch_bounds__(256) k_rank_tiles(LbvhState L) {
+    const unsigned g = blockIdx.x * blockDim.x + threadIdx.x, i = g / 8, lane = g & 7u;
+    const unsigned tiles = (L.n + SORT_TILE - 1) / SORT_TILE;
+    const bool in = i < L.n;
+    const uint64_t key = in ? __ldg(L.keys_tmp + i) : 0;
+    const unsigned own = i / SORT_TILE;
+    unsigned rank = 0;
+    if (in)
+        for (unsigned t = lane; t < tiles; t += 8) {
+            if (t == own) continue;
+            const uint64_t* const k = L.keys_tmp + t * SORT_TILE;
+            // elements before: codes <= key in an earlier tile, < key in a later one
+            unsigned lo = 0, hi = min(SORT_TILE, L.n - t * SORT_TILE);
+            while (lo < hi) {
+                const unsigned m = (lo + hi) / 2;
+                const uint64_t v = __ldg(k + m);
+                if (t < own ? v <= key : v < key) lo = m + 1;
+                else hi = m;
+            }
+            rank += lo;
+        }
+#pragma unroll
+    for (int m = 4; m >= 1; m >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, m);
+    if (in && lane == 0) {
+        rank += i % SORT_TILE;
+        L.morton[rank] = key;
+        L.sorted[rank] = L.sorted_tmp[i];
+    }
 }
 
 // ---------------------------------------------------------- radix sort
@@ -301,6 +381,11 @@ __global__ void __launch_bounds__(256) k_karras(LbvhState L, const uint64_t* key
     int n = (int)L.n;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n - 1) return;
+    L.visited[i + n] = 0;
+    if (i == 0) {
+        L.parent[n] = INVALID;  // the root
+        *L.pair_count = 0;
+    }
     const uint32_t* idx = L.sorted;
     int d = (delta_ref(keys, idx, n, i, i + 1) - delta_ref(keys, idx, n, i, i - 1) >= 0) ? 1 : -1;
     int dmin = delta_ref(keys, idx, n, i, i - d);
@@ -333,33 +418,137 @@ AVBD_D unsigned atomic_add_acq_rel(unsigned* p, unsigned v) {
     return old;
 }
 
+// An internal node as the traversal reads it: both children's boxes rounded
+// outwards to FP32 (only to prune; leaf pairs are tested in FP64), their ids
+// and the last leaf of each, 64 bytes.
+struct PackedNode {
+    float lo0[3], hi0[3], lo1[3], hi1[3];
+    uint32_t left, right, last0, last1;
+};
+static_assert(sizeof(PackedNode) == 64, "packed node");
+
+AVBD_D void pack_node(uint4* packed, unsigned i, unsigned n, unsigned left, unsigned right, unsigned last,
+                      const double* A, const double* B) {
+    PackedNode p;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        p.lo0[k] = __double2float_rd(A[k]);
+        p.hi0[k] = __double2float_ru(A[3 + k]);
+        p.lo1[k] = __double2float_rd(B[k]);
+        p.hi1[k] = __double2float_ru(B[3 + k]);
+    }
+    p.left = left;
+    p.right = right;
+    p.last0 = left < n ? left : left - n;  // an internal left child's index is its last leaf
+    p.last1 = last;
+    const uint4* s = reinterpret_cast<const uint4*>(&p);
+#pragma unroll
+    for (int k = 0; k < 4; k++) packed[4ull * i + k] = s[k];
+}
+
 // Bottom-up refit with one visit counter per internal node: the second child
 // to arrive computes the union (LBVHBuilder::assembleBVH).  min/max are exact,
-// so the result does not depend on arrival order.
-__global__ void __launch_bounds__(256) k_refit(LbvhState L) {
-    unsigned l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l >= L.n) return;
-    const double* b = L.aabb + 6ull * L.sorted[l];
+// so the result does not depend on arrival order.  A block climbs from its
+// REFIT_LEAVES leaves; the nodes whose leaves are all its own -- all but a few
+// dozen -- are counted and combined in shared memory, the rest through global
+// memory, where a level costs an acquire-release round trip and two loads
+// (about 1.3 us; with every level there the refit of 12,000 to 26,000 leaves
+// took 54-65 us).
+constexpr unsigned REFIT_LEAVES = 512;
+struct RefitShared {
+    double leaf[6][REFIT_LEAVES], node[6][REFIT_LEAVES];
+    uint32_t left[REFIT_LEAVES], right[REFIT_LEAVES], parent[REFIT_LEAVES], size[REFIT_LEAVES], visited[REFIT_LEAVES];
+    uint2 range[REFIT_LEAVES];
+};
+__global__ void __launch_bounds__(REFIT_LEAVES) k_refit(LbvhState L) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    RefitShared& S = *reinterpret_cast<RefitShared*>(smem);
+    const unsigned n = L.n, t = threadIdx.x, first = blockIdx.x * REFIT_LEAVES, l = first + t;
+    const unsigned end = min(n, first + REFIT_LEAVES);
+    double b[6];
+    unsigned up = INVALID;  // the node to climb to
+    if (l < n) {
+        const double* a = L.aabb + 6ull * L.sorted[l];
+        up = L.parent[l];
 #pragma unroll
-    for (int a = 0; a < 6; a++) L.nbounds[6ull * l + a] = b[a];
-    L.subtree[l] = 1;
-    L.left[l] = INVALID;
-    L.right[l] = INVALID;
-    unsigned node = L.parent[l];
+        for (int k = 0; k < 6; k++) {
+            b[k] = a[k];
+            S.leaf[k][t] = b[k];
+            L.nbounds[6ull * l + k] = b[k];
+        }
+        L.subtree[l] = 1;
+        L.left[l] = INVALID;
+        L.right[l] = INVALID;
+    }
+    S.visited[t] = 0;
+    if (l + 1 < n) {
+        S.left[t] = L.left[n + l];
+        S.right[t] = L.right[n + l];
+        S.parent[t] = L.parent[n + l];
+        S.range[t] = L.range[l];
+    }
+    __syncthreads();
+    // own nodes: index and leaf range within the block's leaves
+    while (up != INVALID) {
+        const unsigned i = up - n;
+        if (i < first || i >= end) break;
+        const unsigned j = i - first;
+        const uint2 rg = S.range[j];
+        if (rg.x < first || rg.y >= end) break;
+        __threadfence_block();
+        if (atomicAdd(&S.visited[j], 1u) == 0) return;
+        __threadfence_block();
+        const unsigned c[2] = {S.left[j], S.right[j]};
+        double B[2][6];
+        unsigned size = 0;
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const bool leaf = c[q] < n;
+            const unsigned m = (leaf ? c[q] : c[q] - n) - first;
+#pragma unroll
+            for (int k = 0; k < 6; k++)
+                B[q][k] = leaf ? *(volatile double*)&S.leaf[k][m] : *(volatile double*)&S.node[k][m];
+            size += leaf ? 1u : *(volatile uint32_t*)&S.size[m];
+        }
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            b[k] = dmin_ref(B[0][k], B[1][k]);
+            b[3 + k] = dmax_ref(B[0][3 + k], B[1][3 + k]);
+        }
+#pragma unroll
+        for (int k = 0; k < 6; k++) {
+            S.node[k][j] = b[k];
+            L.nbounds[6ull * up + k] = b[k];
+        }
+        S.size[j] = size;
+        L.subtree[up] = size;
+        pack_node(L.packed, i, n, c[0], c[1], rg.y, B[0], B[1]);
+        up = S.parent[j];
+    }
+    // the nodes above
+    unsigned node = up;
     while (node != INVALID) {
         // the first child to arrive stops; the second combines both.  The
         // count is an acquire-release RMW at device scope: the first arrival
         // releases its subtree's writes, the second acquires them
         if (atomic_add_acq_rel(&L.visited[node], 1u) == 0) break;
-        unsigned a = L.left[node], c = L.right[node];
+        const unsigned c[2] = {L.left[node], L.right[node]}, last = L.range[node - n].y, next = L.parent[node];
+        double B[2][6];
+        unsigned size = 0;
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+#pragma unroll
+            for (int k = 0; k < 6; k++) B[q][k] = __ldcg(L.nbounds + 6ull * c[q] + k);
+            size += __ldcg(L.subtree + c[q]);
+        }
 #pragma unroll
         for (int k = 0; k < 3; k++) {
-            L.nbounds[6ull * node + k] = dmin_ref(__ldcg(L.nbounds + 6ull * a + k), __ldcg(L.nbounds + 6ull * c + k));
-            L.nbounds[6ull * node + 3 + k] =
-                dmax_ref(__ldcg(L.nbounds + 6ull * a + 3 + k), __ldcg(L.nbounds + 6ull * c + 3 + k));
+            L.nbounds[6ull * node + k] = dmin_ref(B[0][k], B[1][k]);
+            L.nbounds[6ull * node + 3 + k] = dmax_ref(B[0][3 + k], B[1][3 + k]);
         }
-        L.subtree[node] = __ldcg(L.subtree + a) + __ldcg(L.subtree + c);
-        node = L.parent[node];
+        L.subtree[node] = size;
+        pack_node(L.packed, node - n, n, c[0], c[1], last, B[0], B[1]);
+        node = next;
     }
 }
 
@@ -367,50 +556,84 @@ AVBD_D bool overlaps(const double* A, const double* B) {
     return A[0] <= B[3] && A[1] <= B[4] && A[2] <= B[5] && A[3] >= B[0] && A[4] >= B[1] && A[5] >= B[2];
 }
 
-// One thread per leaf a: every leaf b > a whose box overlaps a's box.
-__global__ void __launch_bounds__(128) k_traverse(LbvhState L, const uint2* range, unsigned root, int* err) {
-    unsigned a = blockIdx.x * blockDim.x + threadIdx.x;
+// One thread per leaf a: every leaf b > a whose box overlaps a's box.  The
+// walk is a chain of dependent loads: each step reads one packed node (both
+// children's FP32 boxes), descends into one child and stacks the other, and
+// never visits a child that does not overlap; a box that does not overlap in
+// FP32 (rounded outwards) does not in FP64 either.  Pairs are appended a few
+// at a time, since every append is an atomic on one counter.
+__global__ void __launch_bounds__(64) k_traverse(LbvhState L, int* err) {
+    const unsigned a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= L.n || L.n < 2) return;
+    constexpr unsigned BUF = 8;
     double q[6];
+    float f[6];
 #pragma unroll
     for (int k = 0; k < 6; k++) q[k] = L.nbounds[6ull * a + k];
-    const unsigned n = L.n;
-    unsigned stack[128];
-    int sp = 0;
-    stack[sp++] = root;
-    const unsigned pa = L.sorted[a];
-    const uint8_t ta = L.type[pa];
-    while (sp > 0) {
-        unsigned node = stack[--sp];
-        if (node >= n) {
-            uint2 rg = range[node - n];
-            if (rg.y <= a) continue;
-        } else if (node <= a) {
-            continue;
-        }
-        double nb[6];
 #pragma unroll
-        for (int k = 0; k < 6; k++) nb[k] = L.nbounds[6ull * node + k];
-        if (!overlaps(q, nb)) continue;
-        if (node < n) {
-            unsigned slot = atomicAdd(L.pair_count, 1u);
-            if (slot < L.pair_capacity) L.pairs[slot] = make_uint2(a, node);
-            else atomicExch(err, (int)AVBD_ERR_CAPACITY);  // a dropped pair would be a missed collision
+    for (int k = 0; k < 3; k++) {
+        f[k] = __double2float_rd(q[k]);
+        f[3 + k] = __double2float_ru(q[3 + k]);
+    }
+    const unsigned n = L.n;
+    unsigned stack[128], buf[BUF], nbuf = 0;
+    int sp = 0;
+    const uint8_t ta = L.type[L.sorted[a]];
+    auto flush = [&]() {
+        const unsigned slot = atomicAdd(L.pair_count, nbuf);
+        if (slot + nbuf > L.pair_capacity) atomicExch(err, (int)AVBD_ERR_CAPACITY);  // a dropped pair would be a missed collision
+        for (unsigned k = 0; k < nbuf; k++)
+            if (slot + k < L.pair_capacity) L.pairs[slot + k] = make_uint2(a, buf[k]);
+        nbuf = 0;
+    };
+    unsigned node = 0;  // internal index; the root
+    for (;;) {
+        PackedNode p;
+        uint4* const w = reinterpret_cast<uint4*>(&p);
+#pragma unroll
+        for (int k = 0; k < 4; k++) w[k] = __ldg(L.packed + 4ull * node + k);
+        const bool in[2] = {
+            p.last0 > a && f[0] <= p.hi0[0] && f[1] <= p.hi0[1] && f[2] <= p.hi0[2] && f[3] >= p.lo0[0] &&
+                f[4] >= p.lo0[1] && f[5] >= p.lo0[2],
+            p.last1 > a && f[0] <= p.hi1[0] && f[1] <= p.hi1[1] && f[2] <= p.hi1[2] && f[3] >= p.lo1[0] &&
+                f[4] >= p.lo1[1] && f[5] >= p.lo1[2]};
+        const unsigned c[2] = {p.left, p.right};
+        unsigned next = INVALID;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            if (!in[k]) continue;
+            if (c[k] >= n) {
+                if (next == INVALID) {
+                    next = c[k] - n;
+                } else {
+                    if (sp >= 128) {
+                        atomicExch(err, (int)AVBD_ERR_CAPACITY);
+                        return;
+                    }
+                    stack[sp++] = c[k] - n;
+                }
+                continue;
+            }
+            double nb[6];
+#pragma unroll
+            for (int m = 0; m < 6; m++) nb[m] = L.nbounds[6ull * c[k] + m];
+            if (!overlaps(q, nb)) continue;
+            buf[nbuf++] = c[k];
+            if (nbuf == BUF) flush();
             // narrow-phase dispatch (CollisionDetector.cpp:166-215): triangle-triangle and
             // rod-rod are no-ops; sphere-sphere and sphere-rod throw "Unsupported collision!"
-            uint8_t tb = L.type[L.sorted[node]];
-            bool sph = ta == AVBD_SHAPE_SPHERE || tb == AVBD_SHAPE_SPHERE;
-            bool tri = ta == AVBD_SHAPE_TRIANGLE || tb == AVBD_SHAPE_TRIANGLE;
+            const uint8_t tb = L.type[L.sorted[c[k]]];
+            const bool sph = ta == AVBD_SHAPE_SPHERE || tb == AVBD_SHAPE_SPHERE;
+            const bool tri = ta == AVBD_SHAPE_TRIANGLE || tb == AVBD_SHAPE_TRIANGLE;
             if (sph && !tri) atomicExch(err, (int)AVBD_ERR_UNSUPPORTED_PAIR);
-            continue;
         }
-        if (sp + 2 > 128) {
-            atomicExch(err, (int)AVBD_ERR_CAPACITY);
-            return;
+        if (next == INVALID) {
+            if (sp == 0) break;
+            next = stack[--sp];
         }
-        stack[sp++] = L.left[node];
-        stack[sp++] = L.right[node];
+        node = next;
     }
+    if (nbuf) flush();
 }
 
 // ---------------------------------------------------------------- host
@@ -459,6 +682,7 @@ int lbvh_allocate(avbd_ctx* c, std::string& err) {
         !alloc((void**)&L.scene_box, sizeof(unsigned long long) * 8) || !alloc((void**)&L.root, sizeof(uint32_t) * 2) ||
         !alloc((void**)&L.pairs, sizeof(uint2) * L.pair_capacity) || !alloc((void**)&L.pair_count, sizeof(uint32_t)) ||
         !alloc((void**)&L.range, sizeof(uint2) * std::max(1u, n - 1)) ||
+        !alloc((void**)&L.packed, sizeof(PackedNode) * std::max(1u, n - 1)) ||
         !alloc((void**)&L.obj, sizeof(uint32_t) * n))
         return AVBD_ERR_CUDA;
     if (triangles && (spheres || segments)) {  // room for 64 triangle contacts per sphere, 16 per segment
@@ -491,34 +715,39 @@ void lbvh_stage(avbd_ctx* c, DevState<R>& s, cudaStream_t st) {
     if (n == 0) return;
     const unsigned nn = 2 * n - 1;
     unsigned long long* box = reinterpret_cast<unsigned long long*>(L.scene_box);
-    cudaMemsetAsync(box, 0xFF, 3 * sizeof(unsigned long long), st);
-    cudaMemsetAsync(box + 3, 0x00, 3 * sizeof(unsigned long long), st);
+    cudaMemsetAsync(box, 0xFF, 6 * sizeof(unsigned long long), st);
     k_prim_bounds<R><<<nb(n, 256), 256, 0, st>>>(s, L, c->params.dt, box);
-    k_morton<<<nb(n, 256), 256, 0, st>>>(L, box);
-    count_launch(c, 2);
-    uint64_t *ka = L.morton, *kb = L.keys_tmp;
-    uint32_t *va = L.sorted, *vb = L.sorted_tmp;
-    for (int shift = 0; shift < 64; shift += 8) {
-        k_radix_count<<<L.hist_blocks, RB, 0, st>>>(ka, n, shift, L.hist, L.hist_blocks);
-        k_radix_scan<<<1, 1024, 0, st>>>(L.hist, 256 * L.hist_blocks);
-        k_radix_scatter<<<L.hist_blocks, RB, 0, st>>>(ka, va, kb, vb, n, shift, L.hist, L.hist_blocks);
-        count_launch(c, 3);
-        std::swap(ka, kb);
-        std::swap(va, vb);
-    }
-    // 8 passes: the sorted keys/values end in the original buffers, but the
-    // original codes were overwritten, so keep the sorted codes and restore the
-    // per-primitive codes by a scatter through the sorted order.
-    // (ka == L.morton holds sorted keys, va == L.sorted holds sorted indices.)
-    cudaMemsetAsync(L.parent, 0xFF, sizeof(uint32_t) * nn, st);
-    cudaMemsetAsync(L.visited, 0, sizeof(uint32_t) * nn, st);
-    cudaMemsetAsync(L.pair_count, 0, sizeof(uint32_t), st);
-    if (n > 1) {
-        k_karras<<<nb(n - 1, 256), 256, 0, st>>>(L, ka, L.range);
+    count_launch(c);
+    // the sorted codes and order end in L.morton and L.sorted
+    if (n <= RANK_SORT_MAX) {
+        k_sort_tiles<<<nb(n, SORT_TILE), SORT_TILE, 0, st>>>(L, box);
+        k_rank_tiles<<<nb(8 * n, 256), 256, 0, st>>>(L);
+        count_launch(c, 2);
+    } else {
+        k_morton<<<nb(n, 256), 256, 0, st>>>(L, box);
         count_launch(c);
+        uint64_t *ka = L.morton, *kb = L.keys_tmp;
+        uint32_t *va = L.sorted, *vb = L.sorted_tmp;
+        for (int shift = 0; shift < 64; shift += 8) {  // 8 passes: back in the original buffers
+            k_radix_count<<<L.hist_blocks, RB, 0, st>>>(ka, n, shift, L.hist, L.hist_blocks);
+            k_radix_scan<<<1, 1024, 0, st>>>(L.hist, 256 * L.hist_blocks);
+            k_radix_scatter<<<L.hist_blocks, RB, 0, st>>>(ka, va, kb, vb, n, shift, L.hist, L.hist_blocks);
+            count_launch(c, 3);
+            std::swap(ka, kb);
+            std::swap(va, vb);
+        }
     }
-    k_refit<<<nb(n, 256), 256, 0, st>>>(L);
-    k_traverse<<<nb(n, 128), 128, 0, st>>>(L, L.range, n > 1 ? n : 0, c->d_error);
+    if (n > 1) {
+        k_karras<<<nb(n - 1, 256), 256, 0, st>>>(L, L.morton, L.range);
+        count_launch(c);
+    } else {
+        cudaMemsetAsync(L.parent, 0xFF, sizeof(uint32_t) * nn, st);
+        cudaMemsetAsync(L.pair_count, 0, sizeof(uint32_t), st);
+    }
+    // (sets an attribute, no launch: also fine while the step is captured)
+    cudaFuncSetAttribute(k_refit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RefitShared));
+    k_refit<<<nb(n, REFIT_LEAVES), REFIT_LEAVES, sizeof(RefitShared), st>>>(L);
+    k_traverse<<<nb(n, 64), 64, 0, st>>>(L, c->d_error);
     count_launch(c, 2);
     launch_narrow<R>(c, s, st);
 }
@@ -652,25 +881,9 @@ __global__ void __launch_bounds__(256) k_box_of_aabbs(const double* __restrict__
 #pragma unroll
     for (int a = 0; a < 3; a++) {
         e[a] = valid ? ord_enc(aabb[6ull * i + a]) : ~0ull;
-        e[3 + a] = valid ? ord_enc(aabb[6ull * i + 3 + a]) : 0ull;
+        e[3 + a] = valid ? ~ord_enc(aabb[6ull * i + 3 + a]) : ~0ull;
     }
-#pragma unroll
-    for (int m = 16; m >= 1; m >>= 1) {
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            unsigned long long o = __shfl_xor_sync(0xffffffffu, e[a], m);
-            e[a] = o < e[a] ? o : e[a];
-            o = __shfl_xor_sync(0xffffffffu, e[3 + a], m);
-            e[3 + a] = o > e[3 + a] ? o : e[3 + a];
-        }
-    }
-    if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            atomicMin(box + a, e[a]);
-            atomicMax(box + 3 + a, e[3 + a]);
-        }
-    }
+    box_reduce(e, box);
 }
 
 }  // namespace
@@ -713,8 +926,7 @@ extern "C" int avbd_lbvh_morton_sort_noalloc(const double* aabb6, unsigned n, ui
     L.aabb = const_cast<double*>(aabb6);
     L.morton = morton;          // per-primitive codes (output)
     L.sorted = sorted_order;    // identity, sorted in place below
-    ok(cudaMemsetAsync(S.box, 0xFF, 3 * sizeof(unsigned long long), st)) &&
-        ok(cudaMemsetAsync(S.box + 3, 0x00, 3 * sizeof(unsigned long long), st)) &&
+    ok(cudaMemsetAsync(S.box, 0xFF, 6 * sizeof(unsigned long long), st)) &&
         launch(k_box_of_aabbs, (n + 255) / 256, 256, (const double*)aabb6, n, S.box) &&
         launch(k_morton, (n + 255) / 256, 256, L, (const unsigned long long*)S.box) &&
         ok(cudaMemcpyAsync(S.keys_a, morton, sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, st));
