@@ -154,6 +154,12 @@ int avbd_create(avbd_ctx** out, int device, unsigned particles_capacity, unsigne
         return fail(AVBD_ERR_CUDA, std::string("cudaStreamCreate: ") + cudaGetErrorString(e));
     }
     c->stream = c->own_stream;
+    e = cudaMallocHost((void**)&c->h_error, sizeof(int));
+    if (e != cudaSuccess) {
+        cudaStreamDestroy(c->own_stream);
+        delete c;
+        return fail(AVBD_ERR_CUDA, std::string("cudaMallocHost: ") + cudaGetErrorString(e));
+    }
     if (const char* g = getenv("AVBD_GRAPH")) c->use_graph = atoi(g) != 0;  // 0: no CUDA graphs
     // condition threshold above which a block is re-solved in FP64 (0: always)
     if (const char* km = getenv("AVBD_KAPPA_MAX")) c->kappa_max = atof(km);
@@ -172,6 +178,7 @@ int avbd_destroy(avbd_ctx* c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     free_device(c);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
+    if (c->h_error) cudaFreeHost(c->h_error);
     delete c;
     return AVBD_OK;
 }
@@ -1617,11 +1624,16 @@ static int autotune(avbd_ctx* c) {
 
 namespace {
 
-int device_error(avbd_ctx* c) {
-    int h = 0;
+// The device-side status: copied behind a call's results on its stream, so
+// that one wait serves both (device_error_queue), then examined.
+int device_error_queue(avbd_ctx* c) {
     if (!c->d_error) return AVBD_OK;
-    CUDA_OR_FAIL(cudaMemcpyAsync(&h, c->d_error, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    CUDA_OR_FAIL(cudaStreamSynchronize(c->stream));
+    CUDA_OR_FAIL(cudaMemcpyAsync(c->h_error, c->d_error, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    return AVBD_OK;
+}
+
+int device_error_check(avbd_ctx* c) {  // after the wait
+    const int h = c->d_error ? *c->h_error : 0;
     if (h == AVBD_ERR_NAN) return fail(h, "non-finite particle state");
     if (h == AVBD_ERR_UNSUPPORTED_PAIR) return fail(h, "Unsupported collision!");
     if (h == AVBD_ERR_CAPACITY)
@@ -1639,6 +1651,12 @@ int device_error(avbd_ctx* c) {
     return AVBD_OK;
 }
 
+int device_error(avbd_ctx* c) {
+    if (int r = device_error_queue(c)) return r;
+    CUDA_OR_FAIL(cudaStreamSynchronize(c->stream));
+    return device_error_check(c);
+}
+
 }  // namespace
 
 extern "C" {
@@ -1652,8 +1670,9 @@ int avbd_step(avbd_ctx* c, unsigned n_steps) {
 
 int avbd_synchronize(avbd_ctx* c) {
     if (int r = check_ctx(c)) return r;
+    if (int r = device_error_queue(c)) return r;
     CUDA_OR_FAIL(cudaStreamSynchronize(c->stream));
-    return device_error(c);
+    return device_error_check(c);
 }
 
 int avbd_collision_stage(avbd_ctx* c) {
@@ -1789,7 +1808,6 @@ static int get_vec(avbd_ctx* c, int which, unsigned first, unsigned n, double* o
     else launch_store_vec<float>(c->f, which, c->d_h2d, c->d_inv + first, n, c->stream);
     CUDA_OR_FAIL(cudaGetLastError());
     CUDA_OR_FAIL(cudaMemcpyAsync(out, c->d_h2d, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, c->stream));
-    CUDA_OR_FAIL(cudaStreamSynchronize(c->stream));
     return device_error(c);
 }
 
@@ -1817,7 +1835,6 @@ static int get_rot(avbd_ctx* c, int which, unsigned first, unsigned n, double* o
     else launch_store_rot<float>(c->f, which, c->d_h2d, c->d_inv + first, n, c->stream);
     CUDA_OR_FAIL(cudaGetLastError());
     CUDA_OR_FAIL(cudaMemcpyAsync(out, c->d_h2d, sizeof(double) * stride * n, cudaMemcpyDeviceToHost, c->stream));
-    CUDA_OR_FAIL(cudaStreamSynchronize(c->stream));
     return device_error(c);
 }
 

@@ -305,6 +305,7 @@ struct avbd_ctx {
     uint32_t* d_perm = nullptr;         // internal -> external
     uint32_t* d_inv = nullptr;          // external -> internal
     int* d_error = nullptr;             // device-side status
+    int* h_error = nullptr;             // pinned copy, read with a call's results
     unsigned long long launches_per_step = 0;
     // per-scene run-to-tolerance state (num_scenes entries, scene ids per vertex)
     unsigned num_scenes = 1;
