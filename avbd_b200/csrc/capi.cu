@@ -1318,7 +1318,13 @@ int autotune_impl(avbd_ctx* c, DevState<R>& s) {
     // (59,000 vertices a color: 3.16 ms with 4, 3.59 with 1, 5.42 with 8)
     std::vector<int> choices = {2, 4, 8, 16};
     if (!c->star_nb) choices = {2, 8};
-    else if (whole) choices = c->max_color_solve < 20000 ? std::vector<int>{4, 8} : std::vector<int>{1, 4};
+    else if (whole) choices = c->max_color_solve < 4000    ? std::vector<int>{8}
+                            : c->max_color_solve < 20000 ? std::vector<int>{4, 8}
+                                                         : std::vector<int>{1, 4};
+    if (choices.size() == 1) {
+        c->lanes = choices[0];
+        return layout_pieces<R>(c, s, st);
+    }
     using V4 = typename Vec4Of<R>::T;
     V4* snap = nullptr;
     CUDA_OR_FAIL(cudaMalloc(&snap, sizeof(V4) * s.n));

@@ -61,6 +61,43 @@ def test_fused_mlp_matches_fp64_reference(n):
     assert np.abs(Y[:, 3:]).max() == 0.0  # padding outputs
 
 
+@pytest.mark.parametrize("n", [127, 129, 128 * 148, 128 * 148 + 1, 3 * 128 * 148 + 5])
+def test_fused_mlp_tile_edges(n):
+    """Rows around a tile (128), one tile for every SM (148) and one for every
+    thread group (3 per SM): each row's output is that of the row alone in the
+    first tile (the rows are computed independently, so it is the same number)."""
+    from avbd_b200 import warmstart
+    m = warmstart.MLP(random_params(5))
+    base = np.zeros((64, 32), dtype=np.float32)
+    base[:, :27] = np.random.default_rng(6).normal(size=(64, 27))
+    F = bf(base)
+    ref = m.forward(F)
+    idx = torch.arange(n, device="cuda") % 64
+    out = m.forward(F[idx].contiguous())
+    m.close()
+    assert torch.equal(out, ref[idx])
+
+
+@pytest.mark.parametrize("B", [128, 128 * 149])
+def test_trainer_gradient_over_several_tiles(B):
+    """One tile, and more tiles than blocks; tolerance as below."""
+    from avbd_b200 import warmstart
+    p = random_params(8)
+    rng = np.random.default_rng(B)
+    X = np.zeros((B, 32), dtype=np.float32)
+    X[:, :27] = rng.normal(size=(B, 27))
+    T = rng.normal(size=(B, 4)).astype(np.float32)
+    T[:, 3] = rng.uniform(0.5, 2.0, size=B)
+    tr = warmstart.Trainer(B, p)
+    loss, g = tr.grad(bf(X), torch.tensor(T, device="cuda"))
+    tr.close()
+    lr_, gr = omlp.loss_and_grad(p, omlp.to_bf16(X), T, bf16=True)
+    assert abs(loss - lr_) <= 1e-3 * lr_
+    for name in ("W1", "b1", "W2", "b2", "W3", "b3", "W4", "b4"):
+        a, b = warmstart.view(g, name).astype(np.float64), omlp.view(gr, name)
+        assert np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-30) < 3e-2, name
+
+
 def test_trainer_gradient_matches_fp64_reference():
     from avbd_b200 import warmstart
     p = random_params(3)

@@ -1,0 +1,106 @@
+"""The star form of the tet solve and the iteration launch at their edges,
+against the FP64 oracle: every lane count of the launch, scenes that stop in
+different iterations, vertices with more neighbours than a piece prefetches
+(16) or the star form takes (64: the context falls back to the records),
+particles without any tet.
+
+Tolerances are those of the parity tests: the FP64 engine differs from the
+oracle by summation order (1e-9 of the bounding-box diagonal), the mixed one
+by its FP32 element constants (1e-6), FP32 without contact by 1e-5.
+"""
+import numpy as np
+import pytest
+
+from avbd_b200 import Context, scenes
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"fp64": 1e-9, "mixed": 1e-6, "fp32": 1e-5}
+
+
+def _pair(oracle_lib, sc, precision, **kw):
+    e = Context()
+    sc.load(e, precision=precision, **kw)
+    e.finalize()
+    o = oracle_lib.Oracle()
+    sc.load(o, **kw)
+    o.finalize()
+    return e, o
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("lanes", [1, 2, 4, 8, 16])
+def test_lane_counts_to_tolerance(oracle_lib, monkeypatch, lanes, precision):
+    """Uneven scenes of odd sizes; they stop in different iterations, so the
+    launch changes from contiguous to dealt pieces on the way."""
+    monkeypatch.setenv("AVBD_LANES", str(lanes))
+    sc = scenes.batched_cubes(num_scenes=7, seed=9, n_min=2, n_max=7)
+    e, o = _pair(oracle_lib, sc, precision, residual_tolerance=1e-4, max_iters=120)
+    stopped = set()
+    for step in range(4):
+        e.step(1)
+        o.step(1)
+        ie, io = e.scene_iterations().astype(int), o.scene_iterations().astype(int)
+        assert np.abs(ie - io).max() <= 2, (step, ie, io)
+        stopped |= set(io.tolist())
+        err = np.abs(e.positions() - o.positions()).max() / sc.bbox_diagonal()
+        assert err <= TOL[precision], (step, err)
+    assert len(stopped) > 2  # the scenes did stop at different times
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "fp32"])
+@pytest.mark.parametrize("lanes", [1, 4, 8, 16])
+def test_lane_counts_fixed_iterations(oracle_lib, monkeypatch, lanes, precision):
+    monkeypatch.setenv("AVBD_LANES", str(lanes))
+    sc = scenes.cube_fixed_bottom(5, iters=7)
+    e, o = _pair(oracle_lib, sc, precision)
+    e.step(6)
+    o.step(6)
+    assert np.abs(e.positions() - o.positions()).max() / sc.bbox_diagonal() <= TOL[precision]
+
+
+def fan(k: int) -> scenes.Scene:
+    """k tets around one edge: its ends have k + 1 neighbours."""
+    sc = scenes.Scene(name=f"fan{k}", dt=1.0 / 60.0, solver_iters=10)
+    a = np.arange(k) * 2 * np.pi / k
+    X = np.concatenate([[[0.0, 0.5, 0.0], [0.0, 1.1, 0.0]],
+                        np.stack([np.cos(a), 0.6 + 0.05 * np.sin(3 * a), np.sin(a)], axis=1)])
+    i = np.arange(k)
+    T = np.stack([np.zeros(k, int), np.ones(k, int), 2 + i, 2 + (i + 1) % k], axis=1)
+    Q, V, lam, mu, m = scenes.tet_setup(X, T, 1e5, 0.4, 1000.0)
+    sc.record("add_particles", X, m)
+    sc.record("add_neo_hookean", T, np.full(k, lam), np.full(k, mu), np.zeros(k), Q.reshape(-1, 9), V)
+    sc.record("set_fixed", [2, 3], np.ones(2, np.uint8))
+    sc.meta["bbox_diagonal"] = 2.9
+    return sc
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "fp32"])
+@pytest.mark.parametrize("k", [15, 16, 40, 63, 64, 90])
+def test_many_neighbours(oracle_lib, k, precision):
+    sc = fan(k)
+    e, o = _pair(oracle_lib, sc, precision)
+    e.step(3)
+    o.step(3)
+    assert np.abs(e.positions() - o.positions()).max() / sc.bbox_diagonal() <= TOL[precision]
+    # the blocks of the edge's ends and of a ring vertex
+    tol = 2e-4 if precision == "fp32" else 1e-5 if precision == "mixed" else 1e-7
+    o.set_positions_raw(0, e.positions())
+    for p in (0, 1, 4):
+        G, H = e.debug_block(p)
+        Go, Ho = o.debug_block(p)[:2]
+        assert np.abs(H - Ho).max() <= tol * np.abs(Ho).max()
+        if precision == "fp64":
+            assert np.abs(G - Go).max() <= 1e-6 * max(1.0, np.abs(Go).max())
+
+
+def test_particles_without_tets(oracle_lib):
+    sc = scenes.Scene(name="free", dt=1.0 / 60.0, solver_iters=5)
+    X = np.random.default_rng(3).uniform(0.01, 1.0, size=(37, 3))
+    m = np.linspace(0.5, 2.0, 37)
+    sc.record("add_particles", X, m)
+    sc.record("add_ground_collision", np.arange(37), m / sc.dt ** 2, np.full(37, 0.4), np.full(37, 0.2))
+    e, o = _pair(oracle_lib, sc, "fp64")
+    e.step(30)
+    o.step(30)
+    assert np.abs(e.positions() - o.positions()).max() <= 1e-9
