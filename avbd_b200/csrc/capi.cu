@@ -163,8 +163,8 @@ int avbd_create(avbd_ctx** out, int device, unsigned particles_capacity, unsigne
     if (const char* g = getenv("AVBD_GRAPH")) c->use_graph = atoi(g) != 0;  // 0: no CUDA graphs
     // condition threshold above which a block is re-solved in FP64 (0: always)
     if (const char* km = getenv("AVBD_KAPPA_MAX")) c->kappa_max = atof(km);
-    // the sweeps of run-to-tolerance steps as one persistent cooperative launch
-    // per iteration (default; 0 launches each color separately)
+    // the iterations of tetrahedral contexts in cooperative launches (default;
+    // 0 launches each color separately)
     if (const char* ps = getenv("AVBD_PERSISTENT")) c->persistent = atoi(ps) != 0;
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess) c->num_sms = (unsigned)sms;
@@ -1542,7 +1542,7 @@ int step_impl(avbd_ctx* c, DevState<R>& s, unsigned n_steps) {
                 cudaGetLastError();
                 c->use_graph = false;
                 capturable = false;
-                trace("persistent sweep: step graph not built, host-driven iteration loop");
+                trace("iteration launch: step graph not built, host-driven iteration loop");
             } else if (gr != AVBD_OK) {
                 return gr;
             }
@@ -1650,7 +1650,7 @@ int device_error_check(avbd_ctx* c) {  // after the wait
         // step's results are invalid, the context stays usable
         CUDA_OR_FAIL(cudaMemsetAsync(c->d_error, 0, sizeof(int), c->stream));
         CUDA_OR_FAIL(cudaStreamSynchronize(c->stream));
-        return fail(h, "a grid-barrier wait of the persistent sweep gave up");
+        return fail(h, "a grid-barrier wait gave up");
     }
     if (h) return fail(h, "device-side error");
     if (c->ws_mlp) return mlp_device_error(c->ws_mlp, c->stream);

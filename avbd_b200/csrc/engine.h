@@ -453,7 +453,7 @@ bool launch_iterate(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaStream
 // to do without the star form or at 2 lanes)
 template <typename R>
 int layout_pieces(avbd_ctx* c, DevState<R>& s, cudaStream_t st);
-// poll limit of the persistent sweep's grid barriers (avbd_debug_set_wait_limit)
+// poll limit of k_iterate's grid barriers (avbd_debug_set_wait_limit)
 int solve_set_wait_limit(unsigned polls);
 // poll limit of the recoloring's grid barriers (avbd_debug_set_wait_limit)
 int contacts_set_wait_limit(unsigned polls);

@@ -239,7 +239,7 @@ AVBD_D void accumulate_tet_e(const DevState<P>& s, const RD& r, unsigned tet, V3
     }
 }
 
-// COH: neighbour positions by coherent loads (the persistent sweep, whose own
+// COH: neighbour positions by coherent loads (k_iterate, whose own
 // launch writes them); otherwise through the read-only path.
 template <typename P, typename RS, typename HT, bool DAMP, bool COH = false>
 AVBD_D void accumulate_tet(const DevState<P>& s, const IncRec<RS>& r, V3<P> xi, P dt, Block3<P, HT>& B) {
@@ -761,7 +761,7 @@ __global__ void __launch_bounds__(256, (SolveMinBlocks<P, RS, FORM>::value)) k_s
                                                           out, T, aux, list);
 }
 
-// Polls a grid-barrier wait of the persistent sweep may take before it gives
+// Polls a grid-barrier wait of k_iterate may take before it gives
 // up (avbd_debug_set_wait_limit lowers it so that tests can make it run out).
 __device__ uint32_t g_sweep_wait_polls = AVBD_DEFAULT_WAIT_POLLS;
 

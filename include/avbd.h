@@ -382,10 +382,11 @@ AVBD_API int avbd_profile_solve(avbd_ctx* ctx, unsigned iterations, double* solv
                                 unsigned* launches);
 
 /* Measurement entry point (no counterpart in the reference): advances one
- * run-to-tolerance step with exactly the launches a timed step uses (the
- * per-scene pieces of each color slab, scenes that have converged gated
- * out), driven from the host, with CUDA events around every color's
- * vertex-solve launch.  Returns their summed time, the algorithmic bytes of
+ * run-to-tolerance step driven from the host, scenes that have converged gated
+ * out, with CUDA events around its solve launches: one launch of the timed
+ * step's kernel per iteration (Chebyshev, ground duals and decisions included,
+ * their bytes counted) for tetrahedral contexts, else the per-scene pieces of
+ * each color slab.  Returns their summed time, the algorithmic bytes of
  * the scenes still iterating when each launch started (per solved vertex as
  * for avbd_profile_solve), the launches and the iterations the step ran.
  * Contexts with dynamic contacts are refused (AVBD_ERR_STATE). */
@@ -432,10 +433,10 @@ AVBD_API int avbd_mlp_destroy(avbd_mlp* m);
  * bounded wait may take on `device` before it gives up
  * (AVBD_DEFAULT_WAIT_POLLS unless changed; 0 gives up at once): the
  * tensor-core barrier waits of the MLP and GEMM kernels, and the grid-barrier
- * waits of the persistent sweep (unless AVBD_PERSISTENT=0 is in the
- * environment when a context is created, each run-to-tolerance sweep of a
- * tetrahedral context runs as one cooperative launch whose blocks meet at a
- * grid barrier between colors), and of the dynamic contacts' recoloring
+ * waits of the iteration launches (unless AVBD_PERSISTENT=0 is in the
+ * environment when a context is created, the iterations of a tetrahedral
+ * context's step run in cooperative launches whose blocks meet at a grid
+ * barrier between colors), and of the dynamic contacts' recoloring
  * (its rounds run as one cooperative launch per step).  A wait that gives up
  * sets AVBD_ERR_BARRIER_TIMEOUT, which the launching call (avbd_step for the
  * sweep and the recoloring) returns; every result of that launch is then
