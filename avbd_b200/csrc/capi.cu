@@ -1310,7 +1310,7 @@ int autotune_impl(avbd_ctx* c, DevState<R>& s) {
     unsigned long long solved = 0;
     for (unsigned v : c->color_solve) solved += v;
     c->lanes = 8;
-    const bool whole = c->persistent && s.no == 0 && !c->dyn && solved > 0;  // iterations are one launch
+    const bool whole = s.no == 0 && whole_iterations(c);  // iterations are one launch
     if (!whole && solved < 50000) return AVBD_OK;
     // with the iterations in one launch, more threads a vertex shorten the
     // chain between two barriers of a small color (8: 17^3 638 against 655 us a
@@ -1625,6 +1625,7 @@ int step_impl(avbd_ctx* c, DevState<R>& s, unsigned n_steps) {
 }  // namespace
 
 static int autotune(avbd_ctx* c) {
+    c->color_launches = colors_fill_launches(c);
     return use64(c) ? autotune_impl<double>(c, c->d) : autotune_impl<float>(c, c->f);
 }
 

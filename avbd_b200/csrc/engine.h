@@ -341,6 +341,7 @@ struct avbd_ctx {
     // iterations of tetrahedral contexts in one cooperative launch with grid
     // barriers (default; AVBD_PERSISTENT=0 turns it off)
     bool persistent = true;
+    bool color_launches = false;  // colors_fill_launches at finalize, for which the lanes were chosen
     uint4* d_slabs = nullptr;           // per color: first internal vertex, solved positional vertices, first piece
     std::vector<uint2> star_off;        // host copy of TetElems::star, during finalize
     std::vector<void*> piece_alloc;     // the laid-out lists (TetElems::piece ...), replaced by each lane choice
@@ -445,6 +446,11 @@ struct IterLaunch {
     const cudaGraphConditionalHandle* loop = nullptr;
     bool sweep_only = false;            // the colors' solves alone (timing of the lane choice)
 };
+// whether a context of these colors and solver settings is better served by
+// launches per color than by k_iterate
+bool colors_fill_launches(const avbd_ctx* c);
+// whether this context's tet iterations run as launches of k_iterate
+bool whole_iterations(const avbd_ctx* c);
 // iterations of one launch of a run-to-tolerance loop
 constexpr unsigned TOL_ITERS_PER_LAUNCH = 32;
 template <typename R>

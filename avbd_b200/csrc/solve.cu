@@ -1989,9 +1989,24 @@ static bool iterate(avbd_ctx* c, DevState<double>& s, const StepConsts& k, cudaS
     return iterate_t<double, double, double>(c, s, s.el, k, st, A);
 }
 
+// k_iterate's 12 to 16 warps an SM save launches and passes over small colors;
+// k_solve_tet's 24 stream large ones better.  Per step, this launch against
+// launches per color: to 1e-4, MIXED, 84,000 vertices a color 11.2 and 21.7 ms,
+// 175,000 24.2 and 29.0, 326,000 45.5 and 39.0, 1,230,000 165 and 125; FP64,
+// 175,000 38.1 and 33.7.  Fixed iterations: MIXED 654,000 10.1 and 10.5, FP32
+// 175,000 equal, FP64 175,000 4.17 and 3.66.
+bool colors_fill_launches(const avbd_ctx* c) {
+    if (c->solver.precision == AVBD_PRECISION_FP64) return c->max_color_solve >= 130000;
+    return c->solver.residual_tolerance > 0 && c->max_color_solve >= 250000;
+}
+
+bool whole_iterations(const avbd_ctx* c) {
+    return c->persistent && !c->color_launches && !c->dyn && c->num_sms != 0 && c->max_color_solve != 0;
+}
+
 template <typename R>
 bool launch_iterate(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaStream_t st, const IterLaunch& L) {
-    if (!c->persistent || s.no != 0 || c->dyn || c->num_sms == 0 || c->max_color_solve == 0) return false;
+    if (s.no != 0 || !whole_iterations(c)) return false;
     IterArgs A = {};
     if (L.tol > 0) {
         A = tol_args(c, L.tol, L.max_it);

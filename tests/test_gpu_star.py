@@ -30,9 +30,12 @@ def _pair(oracle_lib, sc, precision, **kw):
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("lanes", [1, 2, 4, 8, 16])
-def test_lane_counts_to_tolerance(oracle_lib, monkeypatch, lanes, precision):
+@pytest.mark.parametrize("whole", [1, 0])
+def test_lane_counts_to_tolerance(oracle_lib, monkeypatch, whole, lanes, precision):
     """Uneven scenes of odd sizes; they stop in different iterations, so the
-    launch changes from contiguous to dealt pieces on the way."""
+    launch changes from contiguous to dealt pieces on the way.  whole 0: the
+    launches per color that large colors take."""
+    monkeypatch.setenv("AVBD_PERSISTENT", str(whole))
     monkeypatch.setenv("AVBD_LANES", str(lanes))
     sc = scenes.batched_cubes(num_scenes=7, seed=9, n_min=2, n_max=7)
     e, o = _pair(oracle_lib, sc, precision, residual_tolerance=1e-4, max_iters=120)
