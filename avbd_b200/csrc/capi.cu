@@ -495,14 +495,20 @@ struct HostStar {
     unsigned max_nb = 0;
 };
 
-// False when the context needs the records: a vertex with more than
-// STAR_MAX_NB neighbours, or element constants outside RS's comfortable range
-// (rest volumes far from any mesh's, or values that are not finite).
+// False when the context needs the records: a tet that names a vertex twice
+// (the vertex is no neighbour of its own: such an edge has no place in the
+// lists), a vertex with more than STAR_MAX_NB neighbours, or element constants
+// outside RS's comfortable range (rest volumes far from any mesh's, or values
+// that are not finite).
 template <typename RS>
 bool build_star(const avbd_ctx* c, const std::vector<uint32_t>& begin, const std::vector<unsigned>& inc_off,
                 const std::vector<uint32_t>& inc_tet, const std::vector<uint16_t>& inc_local,
                 const std::vector<unsigned>& p_off, const std::vector<unsigned>& p_nbr, HostStar<RS>& S) {
     const unsigned n = (unsigned)c->mass.size();
+    for (const HostNH& h : c->nh)
+        for (int j = 1; j < 4; j++)
+            for (int k = 0; k < j; k++)
+                if (h.idx[j] == h.idx[k]) return false;
     S.off.assign(n + 1, make_uint2(0, 0));
     std::atomic<bool> ok{true};
     // a positional vertex's neighbours (external ids, ascending) are those of its tets

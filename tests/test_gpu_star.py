@@ -107,3 +107,26 @@ def test_particles_without_tets(oracle_lib):
     e.step(30)
     o.step(30)
     assert np.abs(e.positions() - o.positions()).max() <= 1e-9
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "fp32"])
+@pytest.mark.parametrize("twice", [(9, 9, 2, 5), (2, 9, 9, 0), (7, 3, 6, 7), (1, 4, 1, 8)])
+def test_tet_with_a_repeated_vertex(oracle_lib, twice, precision):
+    """Accepted by the entry points: the edge between the two is zero.  The
+    repeated vertex is the largest, the smallest or one between its
+    neighbours.  Blocks as in test_many_neighbours."""
+    sc = fan(8)
+    Q = np.array([[1.1, 0.2, -0.3, 0.1, 0.9, 0.2, -0.2, 0.3, 1.3]])
+    sc.record("add_neo_hookean", np.array([twice]), np.array([1e5]), np.array([4e4]), np.zeros(1), Q, np.array([0.02]))
+    e, o = _pair(oracle_lib, sc, precision)
+    e.step(2)
+    X = e.positions()
+    assert np.isfinite(X).all()
+    o.set_positions_raw(0, X)
+    tol = 2e-4 if precision == "fp32" else 1e-5 if precision == "mixed" else 1e-7
+    for p in sorted({0, 1} | set(twice) - {2, 3}):
+        G, H = e.debug_block(p)
+        Go, Ho = o.debug_block(p)[:2]
+        assert np.abs(H - Ho).max() <= tol * np.abs(Ho).max()
+        if precision == "fp64":
+            assert np.abs(G - Go).max() <= 1e-6 * max(1.0, np.abs(Go).max())
