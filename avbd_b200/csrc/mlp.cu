@@ -217,6 +217,7 @@ struct MlpSink {
     P scale;
     float kappa;           // relative error assumed by the acceptance test
     unsigned long long* applied;  // count of accepted corrections (may be null)
+    bool out_16;           // out is 16-byte aligned (the caller's pointer need not be)
 };
 
 // Thread groups of the fused inference: each takes its own tile through the
@@ -382,11 +383,17 @@ __global__ void __launch_bounds__(GROUPS * GTHREADS, 1) k_mlp_apply(MlpW w, cons
             if (row < n) {
                 const float* b4 = bias + 3 * HID;
                 if (sink.out) {
-                    float4* o = reinterpret_cast<float4*>(sink.out + (size_t)row * OUT);
+                    float* o = sink.out + (size_t)row * OUT;
 #pragma unroll
-                    for (int j = 0; j < 4; j++)
-                        o[j] = make_float4(v[4 * j] + b4[4 * j], v[4 * j + 1] + b4[4 * j + 1],
-                                           v[4 * j + 2] + b4[4 * j + 2], v[4 * j + 3] + b4[4 * j + 3]);
+                    for (int j = 0; j < (int)OUT; j++) v[j] += b4[j];
+                    if (sink.out_16) {
+#pragma unroll
+                        for (int j = 0; j < (int)OUT; j += 4)
+                            *reinterpret_cast<float4*>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < (int)OUT; j++) o[j] = v[j];
+                    }
                 } else if (!(sink.flags[row] & (VF_FIXED | VF_ORIENTED))) {
                     const float y[3] = {v[0] + b4[0], v[1] + b4[1], v[2] + b4[2]};
                     if (accept(Xs, warp * 32 + lane, y, sink.kappa)) {
@@ -780,7 +787,7 @@ template <typename P>
 int mlp_apply_state(const MlpDevice& m, const void* feat, unsigned n, typename Vec4Of<P>::T* x,
                     typename Vec4Of<P>::T* xl, typename Vec4Of<P>::T* xll, const uint8_t* flags, double scale,
                     float kappa, unsigned long long* applied, cudaStream_t st) {
-    MlpSink<P> s{nullptr, x, xl, xll, flags, (P)scale, kappa, applied};
+    MlpSink<P> s{nullptr, x, xl, xll, flags, (P)scale, kappa, applied, false};
     return mlp_launch<P>(m, (const bf16*)feat, n, s, st);
 }
 template int mlp_apply_state<float>(const MlpDevice&, const void*, unsigned, float4*, float4*, float4*,
@@ -888,7 +895,7 @@ int avbd_mlp_forward(avbd_mlp* m, const void* features, unsigned n, float* out, 
     if (!m || !features || !out) return set_error(AVBD_ERR_INVALID_ARG, "null argument");
     if ((uintptr_t)features & 15) return set_error(AVBD_ERR_INVALID_ARG, "features must be 16-byte aligned");
     cudaStream_t st = stream ? (cudaStream_t)stream : m->st;
-    MlpSink<float> s{out, nullptr, nullptr, nullptr, nullptr, 0.f, 0.f, nullptr};
+    MlpSink<float> s{out, nullptr, nullptr, nullptr, nullptr, 0.f, 0.f, nullptr, ((uintptr_t)out & 15) == 0};
     if (int rc = mlp_launch<float>(*m->m, (const bf16*)features, n, s, st)) return rc;
     return mlp_device_error(m->m, st);
 }

@@ -2,6 +2,8 @@
 FP32 matmul of the same BF16 inputs, the fused MLP against the FP64 oracle
 MLP with the engine's BF16 rounding points, the trainer's gradient against
 the oracle's, and the warm-start hooks of a context."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -96,6 +98,27 @@ def test_trainer_gradient_over_several_tiles(B):
     for name in ("W1", "b1", "W2", "b2", "W3", "b3", "W4", "b4"):
         a, b = warmstart.view(g, name).astype(np.float64), omlp.view(gr, name)
         assert np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-30) < 3e-2, name
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3, 4])
+@pytest.mark.parametrize("n", [1, 129])
+def test_fused_mlp_output_of_any_float_alignment(n, offset):
+    """The entry point states no alignment of its output: an array that starts
+    `offset` floats behind a 256-byte boundary receives the same rows, and
+    nothing is written around it."""
+    from avbd_b200 import _lib, warmstart
+    X = bf(np.random.default_rng(n).normal(size=(n, 32)))
+    torch.cuda.synchronize()
+    m = warmstart.MLP(random_params(n))
+    want = m.forward(X)
+    buf = torch.full((n * 16 + 8,), 7.0, device="cuda")
+    torch.cuda.synchronize()
+    rc = m.L.avbd_mlp_forward(m.h, C.c_void_p(X.data_ptr()), n, C.c_void_p(buf.data_ptr() + 4 * offset), None)
+    assert rc == _lib.AVBD_OK
+    torch.cuda.synchronize()
+    m.close()
+    assert torch.equal(buf[offset:offset + n * 16].view(n, 16), want)
+    assert (buf[:offset] == 7).all() and (buf[offset + n * 16:] == 7).all()
 
 
 def test_trainer_gradient_matches_fp64_reference():
