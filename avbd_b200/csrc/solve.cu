@@ -1041,12 +1041,12 @@ __device__ __noinline__ unsigned iterate_candidates(const IterArgs& A, SceneBits
     for (unsigned i = threadIdx.x; i < (A.S + 31) / 32; i += blockDim.x) cand.w[i] = 0;
     if (threadIdx.x == 0) *red = 0;
     __syncthreads();
-    const double t2 = A.tol * A.tol * A.g2 * (1 + 1e-9);  // a cheap bound first, then the exact comparison
+    const double t2 = A.tol * A.tol * (1 + 1e-9);  // a cheap bound first, then the exact comparison
     unsigned n = 0;
     for (unsigned q = threadIdx.x; q < A.S; q += blockDim.x)
         if (on.get(q)) {
-            const double r = __ldcg(r2 + q), m = A.m2[q];
-            if ((r <= t2 * m || !(m > 0)) && scene_R(r, m * A.g2) <= A.tol) {
+            const double r = __ldcg(r2 + q), mg2 = A.m2[q] * A.g2;  // 0 without gravity: the residual is absolute
+            if ((r <= t2 * mg2 || !(mg2 > 0)) && scene_R(r, mg2) <= A.tol) {
                 atomicOr(cand.w + (q >> 5), 1u << (q & 31u));
                 n++;
             }

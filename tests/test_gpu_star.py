@@ -130,3 +130,22 @@ def test_tet_with_a_repeated_vertex(oracle_lib, twice, precision):
         assert np.abs(H - Ho).max() <= tol * np.abs(Ho).max()
         if precision == "fp64":
             assert np.abs(G - Go).max() <= 1e-6 * max(1.0, np.abs(Go).max())
+
+
+@pytest.mark.parametrize("whole", [1, 0])
+def test_tolerance_without_gravity(oracle_lib, monkeypatch, whole):
+    """The residual is then the absolute force (its scale, the weight, is 0):
+    scenes stop where the oracle's do, not at the cap."""
+    monkeypatch.setenv("AVBD_PERSISTENT", str(whole))
+    sc = scenes.batched_cubes(num_scenes=5, seed=9, n_min=2, n_max=5)
+    sc.g_accel = 0.0
+    e, o = _pair(oracle_lib, sc, "fp64", residual_tolerance=1e-2, max_iters=120)
+    V = np.random.default_rng(3).uniform(-0.2, 0.2, size=e.positions().shape)
+    e.set_velocities(0, V)
+    o.set_velocities(0, V)
+    for step in range(3):
+        e.step(1)
+        o.step(1)
+        ie, io = e.scene_iterations().astype(int), o.scene_iterations().astype(int)
+        assert io.max() < 100 and np.abs(ie - io).max() <= 2, (step, ie, io)
+        assert np.abs(e.positions() - o.positions()).max() / sc.bbox_diagonal() <= TOL["fp64"]
