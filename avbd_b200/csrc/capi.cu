@@ -1242,6 +1242,14 @@ int enqueue_step_fixed(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaStr
 
 int ensure_omega_table(avbd_ctx* c, unsigned n, cudaStream_t st);
 
+// Ends the recording of st.  A launch that was refused is missing from the
+// graph, which must not be kept then: a step would silently leave out its
+// iterations, and a loop whose body lost the launch that ends it would not end.
+cudaError_t end_capture(cudaStream_t st, cudaGraph_t* g) {
+    const cudaError_t launch = cudaGetLastError(), e = cudaStreamEndCapture(st, g);
+    return launch != cudaSuccess ? launch : e;
+}
+
 // A fixed-iteration step with dynamic contacts: the step start runs the
 // host contact management (so the step as a whole cannot be one graph), then
 // one iteration -- the sweep over the step's colors and contact lists,
@@ -1266,10 +1274,13 @@ int step_fixed_dyn_graph(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaS
         enqueue_sweep<R>(c, s, k, st, SceneTol());
         enqueue_chebyshev<R>(c, s, k, 1.0, 0, st, T);
         launch_iter_next(c, n, st);
-        cudaError_t e = cudaStreamEndCapture(st, &g);
+        cudaError_t e = end_capture(st, &g);
         const unsigned long long per_iter = c->stats.kernel_launches - before;
         c->stats.kernel_launches = before;
-        if (e != cudaSuccess) return fail(AVBD_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
+        if (e != cudaSuccess) {
+            if (g) cudaGraphDestroy(g);
+            return fail(AVBD_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
+        }
         if (c->dyn_graph) {
             cudaGraphExecUpdateResultInfo info;
             if (cudaGraphExecUpdate(c->dyn_graph, g, &info) != cudaSuccess) {
@@ -1454,7 +1465,7 @@ int build_tol_graph(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaStream
     e = cudaStreamGetCaptureInfo(st, &cs, nullptr, nullptr, &deps, &ndeps);
     if (e != cudaSuccess) return abandon("graph capture: ", e);
     std::vector<cudaGraphNode_t> tail(deps, deps + ndeps);
-    e = cudaStreamEndCapture(st, &g);
+    e = end_capture(st, &g);
     if (e != cudaSuccess) return abandon("graph capture: ", e);
     // the iteration loop
     cudaGraphConditionalHandle h;
@@ -1489,13 +1500,13 @@ int build_tol_graph(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaStream
         body_launches = (unsigned)(c->stats.kernel_launches - body0);
         launch_tol_loop_next(c, h, max_it, body_launches, st);
     }
-    e = cudaStreamEndCapture(st, &body);
+    e = end_capture(st, &body);
     if (e != cudaSuccess) return abandon("graph capture: ", e);
     // step end
     e = cudaStreamBeginCaptureToGraph(st, g, &loop, nullptr, 1, mode);
     if (e != cudaSuccess) return abandon("graph capture: ", e);
     enqueue_velocity<R>(c, s, k, st);
-    e = cudaStreamEndCapture(st, &g);
+    e = end_capture(st, &g);
     if (e != cudaSuccess) return abandon("graph capture: ", e);
     e = cudaGraphInstantiate(&c->graph, g, 0);
     cudaGraphDestroy(g);
@@ -1596,11 +1607,15 @@ int step_impl(avbd_ctx* c, DevState<R>& s, unsigned n_steps) {
     if (int r = ensure_omega_table(c, c->solver.solver_iters, st)) return r;
     if (capturable && !c->graph) {
         unsigned long long before = c->stats.kernel_launches;
-        cudaGraph_t g;
+        cudaGraph_t g = nullptr;
         CUDA_OR_FAIL(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         enqueue_step_fixed<R>(c, s, k, st);  // no host step without dynamic contacts: cannot fail
-        cudaError_t e = cudaStreamEndCapture(st, &g);
-        if (e != cudaSuccess) return fail(AVBD_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
+        cudaError_t e = end_capture(st, &g);
+        if (e != cudaSuccess) {
+            c->stats.kernel_launches = before;
+            if (g) cudaGraphDestroy(g);
+            return fail(AVBD_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
+        }
         e = cudaGraphInstantiate(&c->graph, g, 0);
         cudaGraphDestroy(g);
         if (e != cudaSuccess) return fail(AVBD_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));

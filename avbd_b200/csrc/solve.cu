@@ -1589,12 +1589,18 @@ void launch_tet_eprev(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaStre
     count_launch(c);
 }
 
-// Dynamic shared memory of a kernel's neighbour staging; above 48 KB, with
-// the static part (under 8 KB), the kernel has to opt in.
+// Dynamic shared memory a kernel's neighbour staging may take: what a block can
+// have (227 KB) less the static part of these kernels (under 8 KB).
+constexpr unsigned STAGE_SMEM_MAX = (227 - 8) * 1024;
+// Above 48 KB with the static part a kernel has to opt in.  The limit belongs to
+// the kernel, which all contexts and host threads of the process share, so it
+// is only ever set to this one value: set to a context's own size, a smaller
+// context could lower it between a larger one's setting and its launch.
 template <typename K>
 static bool stage_smem(K kern, unsigned bytes) {
     return bytes <= 40 * 1024 ||
-           cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+           (bytes <= STAGE_SMEM_MAX &&
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STAGE_SMEM_MAX) == cudaSuccess);
 }
 
 template <typename P, typename RS, typename HT, int LANES, int FORM, int MODE, bool DYN>

@@ -8,6 +8,8 @@ Tolerances are those of the parity tests: the FP64 engine differs from the
 oracle by summation order (1e-9 of the bounding-box diagonal), the mixed one
 by its FP32 element constants (1e-6), FP32 without contact by 1e-5.
 """
+import threading
+
 import numpy as np
 import pytest
 
@@ -149,3 +151,49 @@ def test_tolerance_without_gravity(oracle_lib, monkeypatch, whole):
         ie, io = e.scene_iterations().astype(int), o.scene_iterations().astype(int)
         assert io.max() < 100 and np.abs(ie - io).max() <= 2, (step, ie, io)
         assert np.abs(e.positions() - o.positions()).max() / sc.bbox_diagonal() <= TOL["fp64"]
+
+
+@pytest.mark.parametrize("whole", [1, 0])
+def test_contexts_of_different_valence_on_two_threads(monkeypatch, whole):
+    """Contexts are independent: while one host thread steps a context, another
+    steps one whose staging of neighbours takes less shared memory (both more
+    than the 48 KB a kernel has without opting in).  Every launch is a call of
+    its own (no graph), so that the two meet often; fixed iterations are
+    deterministic, so each ends where it ends alone."""
+    monkeypatch.setenv("AVBD_PERSISTENT", str(whole))
+    monkeypatch.setenv("AVBD_GRAPH", "0")
+    sizes, steps = (60, 52), 400
+
+    def context(k):
+        e = Context()
+        fan(k).load(e, precision="fp64")
+        e.finalize()
+        return e
+
+    def run(e, errors):
+        try:
+            for _ in range(steps):
+                e.step(1)
+            e.synchronize()
+        except Exception as ex:
+            errors.append(repr(ex))
+
+    alone = []
+    for k in sizes:
+        e = context(k)
+        errors = []
+        run(e, errors)
+        assert not errors
+        alone.append(e.positions())
+        e.close()
+    both = [context(k) for k in sizes]
+    errors = []
+    threads = [threading.Thread(target=run, args=(e, errors)) for e in both]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for e, X in zip(both, alone):
+        assert np.array_equal(e.positions(), X)
+        e.close()
