@@ -1308,39 +1308,43 @@ int step_fixed_dyn_graph(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaS
 
 StepConsts consts(avbd_ctx* c) { return StepConsts{c->params.dt, c->params.g_accel, c->kappa_max}; }
 
-// Picks the threads-per-vertex of the tet solve (1, 2, 4, 8 or 16; 2 or 8 with
-// the records) by timing sweeps with each choice on the context's own data,
+// Picks the threads-per-vertex of the tet solve (2, 4, 8 or 16; in k_iterate 4 or
+// 8 with the star form, 2 or 8 with the records), where sizes do not settle it
+// by timing equal numbers of sweeps with each choice on the context's own data,
 // in the launches a step will use.  Positions are snapshotted and restored,
 // so the state is untouched.  AVBD_LANES=<n> in the environment forces a
 // choice.
 template <typename R>
 int autotune_impl(avbd_ctx* c, DevState<R>& s) {
     cudaStream_t st = c->stream;
-    const char* env = getenv("AVBD_LANES");
-    if (env) {
-        int l = atoi(env);
-        if (l == 1 || l == 2 || l == 4 || l == 8 || l == 16 || l == 32) c->lanes = std::min(l, 16);
-        if (!c->star_nb && c->lanes > 2) c->lanes = 8;
-        if (!c->star_nb && c->lanes < 2) c->lanes = 2;
-        return layout_pieces<R>(c, s, st);
+    const bool whole = s.no == 0 && whole_iterations(c);  // iterations are one launch
+    c->lanes = 8;
+    if (const char* env = getenv("AVBD_LANES")) {
+        const int l = atoi(env);
+        if (l == 1 || l == 2 || l == 4 || l == 8 || l == 16 || l == 32) c->lanes = std::max(2, std::min(l, whole ? 8 : 16));
+        return whole ? layout_pieces<R>(c, s, st) : AVBD_OK;
     }
     unsigned long long solved = 0;
     for (unsigned v : c->color_solve) solved += v;
-    c->lanes = 8;
-    const bool whole = s.no == 0 && whole_iterations(c);  // iterations are one launch
-    if (!whole && solved < 50000) return AVBD_OK;
-    // with the iterations in one launch, more threads a vertex shorten the
-    // chain between two barriers of a small color (8: 17^3 638 against 655 us a
-    // pass with 4, 662 with 16) and fewer take less instructions of a large one
-    // (59,000 vertices a color: 3.16 ms with 4, 3.59 with 1, 5.42 with 8)
-    std::vector<int> choices = {2, 4, 8, 16};
-    if (!c->star_nb) choices = {2, 8};
-    else if (whole) choices = c->max_color_solve < 4000    ? std::vector<int>{8}
-                            : c->max_color_solve < 20000 ? std::vector<int>{4, 8}
-                                                         : std::vector<int>{1, 4};
+    // In k_iterate more threads a vertex shorten the chain between two barriers of
+    // a small color and fewer take less instructions of a large one.  Star form,
+    // us a step of 15 iterations with 4 and 8 threads: grids FP32 1,459 vertices
+    // a color 243 and 212, 8,985 equal, 17,231 318 and 398; MIXED 3,907 equal,
+    // 8,985 298 and 415; FP64 8,985 359 and 420, 17,231 667 and 630; tetrahedra
+    // of random points (15 to 40 neighbours) FP64 13,308 1,459 and 1,201, to
+    // 1e-4 66,540 37.8 and 27.9 ms.  Records, 2 and 8 threads: FP32 17,231 950
+    // and 852; to 1e-4 30,523 8.5 and 10.1 ms, MIXED 11.5 and 13.4, FP64 equal,
+    // random points MIXED 44,360 63.5 and 44.9.
+    std::vector<int> choices = {8};
+    if (whole && c->star_nb && c->max_color_solve >= 4000)
+        choices = c->max_color_solve < 20000 ? std::vector<int>{4, 8} : std::vector<int>{8, 4};
+    else if (whole && !c->star_nb && c->max_color_solve >= 20000)
+        choices = {2, 8};
+    else if (!whole && solved >= 50000)
+        choices = {2, 4, 8, 16};
     if (choices.size() == 1) {
         c->lanes = choices[0];
-        return layout_pieces<R>(c, s, st);
+        return whole ? layout_pieces<R>(c, s, st) : AVBD_OK;
     }
     using V4 = typename Vec4Of<R>::T;
     V4* snap = nullptr;
@@ -1351,19 +1355,25 @@ int autotune_impl(avbd_ctx* c, DevState<R>& s) {
     CUDA_OR_FAIL(cudaEventCreate(&a));
     CUDA_OR_FAIL(cudaEventCreate(&b));
     const unsigned long long launches0 = c->stats.kernel_launches;
+    const unsigned sweeps = solved < 50000 ? 16 : 2;
     int best = 8;
     float best_ms = 1e30f;
     for (int l : choices) {
         c->lanes = l;
         if (whole)
             if (int r = layout_pieces<R>(c, s, st)) return r;
-        for (int rep = 0; rep < 2; rep++) {  // rep 0 warms up, rep 1 is timed
+        bool refused = false;  // k_iterate cannot run with this choice
+        for (unsigned rep = 0; rep < 2 && !refused; rep++) {  // rep 0 warms up, rep 1 is timed
             if (rep == 1) CUDA_OR_FAIL(cudaEventRecord(a, st));
-            IterLaunch L;
-            L.n = solved < 50000 ? 16 : 2;
-            L.sweep_only = true;
-            if (launch_iterate<R>(c, s, k, st, L)) continue;
-            for (unsigned col = 0; col < c->num_colors; col++) {
+            if (whole) {
+                IterLaunch L;
+                L.n = sweeps;
+                L.sweep_only = true;
+                refused = !launch_iterate<R>(c, s, k, st, L);
+                continue;
+            }
+            for (unsigned q = 0; q < sweeps * c->num_colors; q++) {
+                const unsigned col = q % c->num_colors;
                 if (!c->color_solve[col]) continue;
                 if (c->solver.residual_tolerance > 0 && c->d_solve_ranges) {  // the launches a step will use
                     const unsigned r0 = c->solve_range_off[col], r1 = c->solve_range_off[col + 1];
@@ -1373,10 +1383,12 @@ int autotune_impl(avbd_ctx* c, DevState<R>& s) {
                 }
             }
         }
+        if (refused) continue;
         CUDA_OR_FAIL(cudaEventRecord(b, st));
         CUDA_OR_FAIL(cudaEventSynchronize(b));
         float ms = 0;
         CUDA_OR_FAIL(cudaEventElapsedTime(&ms, a, b));
+        ms /= (float)sweeps;
         if (getenv("AVBD_TRACE")) fprintf(stderr, "[avbd] autotune: %d threads per vertex: %.3f ms per sweep\n", l, ms);
         if (ms < best_ms) {
             best_ms = ms;

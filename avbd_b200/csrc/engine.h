@@ -347,7 +347,7 @@ struct avbd_ctx {
     std::vector<void*> piece_alloc;     // the laid-out lists (TetElems::piece ...), replaced by each lane choice
     uint32_t* d_sweep_sync = nullptr;   // IterArgs::sync
     unsigned num_sms = 0;
-    int8_t iterate_fits[2][5] = {};     // [run to tolerance][lanes 2, 4, 8, 16, 1]: 0 not queried, 1 yes, -1 no
+    int8_t iterate_fits[2][3] = {};     // [run to tolerance][lanes 2, 4, 8]: 0 not queried, 1 yes, -1 no
     unsigned long long host_iterations = 0;  // scene-iterations of fixed-iteration steps
 
     // CUDA graph of one full step: fixed iterations, or (graph_tol) the

@@ -886,10 +886,10 @@ struct IterThreads {
 
 // A piece of 32 / LANES vertices of the star form whose constant data are on
 // their way into registers: this thread's entries of the first rounds (16
-// neighbours and 24 or 32 tets a vertex; the rest is read when its turn comes).
+// neighbours and 24 tets a vertex; the rest is read when its turn comes).
 template <typename RS, int LANES>
 struct StarPiece {
-    static constexpr int UN = 16 / LANES, UT = LANES == 16 ? 2 : 24 / LANES;
+    static constexpr int UN = 16 / LANES, UT = 24 / LANES;
     uint4 h;  // TetElems::piece
     StarNb<RS> nb[UN];
     StarTet<RS> tet[UT];
@@ -1150,96 +1150,6 @@ AVBD_D void finish_ground(const DevState<P>& s, unsigned p, typename Vec4Of<P>::
     if (gf != g0) s.gflag[p] = gf;
 }
 
-// The pieces of one color at one thread a vertex: no lane idles in the solve
-// and nothing is reduced, so a vertex takes a third of the instructions of 4
-// threads; for colors that fill the SMs' warps this way.
-template <typename P, typename RS, bool GROUND, bool TOL>
-AVBD_D void color_wide(const DevState<P>& s, const TetElems<RS>& el, const Consts<P>& c, const IterArgs& A,
-                       unsigned long long* counters, const uint32_t* scene, uint4 sl, SceneBits on, bool spread, P om,
-                       typename Vec4Of<P>::T* hist, double* r2, P* es) {
-    using V4 = typename Vec4Of<P>::T;
-    constexpr int THREADS = IterThreads<P, FORM_STAR, 1>::value;
-    constexpr unsigned WARPS = THREADS / 32, ST = StarStage<P, 1, THREADS>::STRIDE, U = 4;
-    const unsigned warp = threadIdx.x >> 5, wl = threadIdx.x & 31u, K = el.max_nb;
-    const unsigned B = gridDim.x, b = blockIdx.x;
-    const unsigned nch = (sl.y + 31) / 32, per = (nch + B - 1) / B;
-    const unsigned end = spread ? nch : min(nch, (b + 1) * per), step = spread ? B * WARPS : WARPS;
-    SceneSum sum(r2);
-    for (unsigned k = spread ? b * WARPS + warp : b * per + warp; k < end; k += step) {
-        const unsigned gi = k * 32 + wl, p = sl.x + min(gi, sl.y - 1);
-        bool live = gi < sl.y;
-        unsigned sc = 0;
-        if constexpr (TOL) {
-            sc = scene[p];
-            live = live && on.get(sc);
-            if (!__any_sync(0xffffffffu, live)) continue;
-        }
-        const uint4 h = el.piece[sl.z + k];
-        const V3<P> xi = xyz(ld_vec(s.x + p));
-        Block3<P, P> Bk;
-        for (unsigned u0 = 0; u0 < h.y; u0 += U) {
-            StarNb<RS> q[U];
-            V3<P> xo[U];
-#pragma unroll
-            for (unsigned u = 0; u < U; u++)
-                if (u0 + u < h.y) q[u] = ld_once(el.pnb + h.x + (u0 + u) * 32 + wl);
-#pragma unroll
-            for (unsigned u = 0; u < U; u++)
-                if (u0 + u < h.y) xo[u] = xyz(ld_vec(s.x + q[u].idx));
-#pragma unroll
-            for (unsigned u = 0; u < U; u++)
-                if (u0 + u < h.y) star_edge<P, RS, P, ST>(q[u].w, xo[u] - xi, es + (u0 + u) * ST, K, Bk);
-        }
-        StarTet<RS> q[U];
-        uint32_t l[U];
-#pragma unroll
-        for (unsigned u = 0; u < U; u++)
-            if (u < h.w) {
-                q[u] = ld_once(el.ptet + h.z + u * 32 + wl);
-                l[u] = ld_once(el.ploc + h.z + u * 32 + wl);
-            }
-        for (unsigned u0 = 0; u0 < h.w; u0 += U) {
-#pragma unroll
-            for (unsigned u = 0; u < U; u++)
-                if (u0 + u < h.w) {
-                    star_tet<P, RS, P, ST>(q[u], l[u], es, K, Bk);
-                    if (u0 + u + U < h.w) {  // a group ahead
-                        q[u] = ld_once(el.ptet + h.z + (u0 + u + U) * 32 + wl);
-                        l[u] = ld_once(el.ploc + h.z + (u0 + u + U) * 32 + wl);
-                    }
-                }
-        }
-        const P hd = (P)el.hd[p];
-        Bk.h00 += hd;
-        Bk.h11 += hd;
-        Bk.h22 += hd;
-        V4 gk, gl, cp;
-        uint8_t fl = 0, gf = 0;
-        if constexpr (GROUND) {
-            fl = live ? s.flags[p] : (uint8_t)0;
-            cp = ld_vec(s.gcp + p);
-            gk = ld_vec(s.gk + p);
-            gl = ld_vec(s.glam + p);
-            gf = s.gflag[p];
-            if (fl & VF_GROUND) accumulate_ground<P, P>(gk, gl, cp, gf, xi, Bk);
-        }
-        double acc = 0.0;
-        if (live) {
-            const V4 y4 = ld_vec(s.y + p);
-            const V3<P> rhs = block_rhs(Bk, xi, y4, c.inv_dt2);
-            if (TOL) acc = sum_sq(rhs);
-            const V3<P> xa = finish_vertex<P, P>(s, c, A, counters, Bk, rhs, xi, p, y4.w, xyz(ld_vec(hist + p)), om, hist);
-            if constexpr (GROUND)
-                if ((fl & VF_GROUND) && !A.sweep_only) finish_ground<P>(s, p, gk, gl, cp, gf, xa);
-        }
-        if constexpr (TOL) {
-            __syncwarp();
-            sum.add(sc, acc);
-        }
-    }
-    if constexpr (TOL) sum.flush();
-}
-
 // The iterations of a step in one cooperative launch of a block per SM, with a
 // grid barrier between colors (about 1 us, against about 3 us for a launch of
 // a graph).  Small scenes are bounded by these phases, not by their bytes: what
@@ -1249,16 +1159,16 @@ AVBD_D void color_wide(const DevState<P>& s, const TetElems<RS>& el, const Const
 // vertex's own solved position, so they follow its solve instead of taking a
 // pass and a barrier of their own: the solved position goes to the second half
 // of x, where the later colors of this iteration read it (tagged ids, StarNb),
-// the accelerated one to x itself, for the next iteration.  At 4 or more lanes
-// (PIPE) a warp's pieces (32 / LANES consecutive vertices) run as one sequence
-// over the colors: the next piece's header is loaded while the current one
+// the accelerated one to x itself, for the next iteration.  A warp's pieces
+// (32 / LANES consecutive vertices) run as one sequence over the colors: the next piece's header is loaded while the current one
 // gathers, its lists while the current one reduces and solves -- also across
 // the barrier, since they are constant -- so a phase is one round trip for the
 // positions and the arithmetic.  Measured: a barrier with the release and the
 // first read behind it 1.9 us, a color of an 8^3 cube 2.9 us (4.6 with the
 // loads of the lists behind the barrier, 3.7 as a launch of a graph).
-// Records, and the star form at 2 lanes (AVBD_LANES): every color is a pass of
-// tet_vertex and the acceleration another.
+// Records: every color is a pass of tet_vertex and the acceleration another.  So
+// does the star form at 2 lanes, which only AVBD_LANES=2 takes: it solves as
+// k_solve_tet does, operation for operation, so that the two can be compared.
 //
 // While every scene iterates, the blocks own contiguous parts of a color
 // (neighbouring vertices share their neighbours in L1); once scenes have
@@ -1275,8 +1185,7 @@ __global__ void __launch_bounds__((IterThreads<P, FORM, LANES>::value), 1)
     using V4 = typename Vec4Of<P>::T;
     constexpr int THREADS = IterThreads<P, FORM, LANES>::value;
     constexpr unsigned WARPS = THREADS / 32, V = 32 / LANES;
-    constexpr bool STAR = FORM == FORM_STAR && LANES != 2;  // accelerates as it solves
-    constexpr bool PIPE = STAR && LANES > 1;
+    constexpr bool PIPE = FORM == FORM_STAR && LANES > 2;  // accelerates as it solves
     constexpr unsigned ST = StarStage<P, LANES, THREADS>::STRIDE;
     using Piece = StarPiece<RS, PIPE ? LANES : 4>;
     __shared__ unsigned red;
@@ -1359,15 +1268,7 @@ __global__ void __launch_bounds__((IterThreads<P, FORM, LANES>::value), 1)
         double* const r2 = TOL ? A.r2 + (size_t)(it % 3u) * A.S : nullptr;
         if constexpr (TOL) done_it += na;
         const P om = A.sweep_only ? P(1) : (P)A.omega[it];
-        if constexpr (STAR && !PIPE) {
-            for (unsigned col = 0; col < A.ncolors; col++) {
-                const uint4 sl = slabs[col];
-                if (sl.y == 0) continue;
-                color_wide<P, RS, GROUND, TOL>(s, el, c, A, counters, scene, sl, on, spread, om, (it & 1u) ? s.xll : s.xl,
-                                               r2, es);
-                if (!iterate_barrier(A.sync, ++bar, s.err)) return;
-            }
-        } else if constexpr (PIPE) {
+        if constexpr (PIPE) {
             V4* const hist = (it & 1u) ? s.xll : s.xl;
             SceneSum sum(r2);
             for (unsigned col = 0; col < A.ncolors; col++) {
@@ -1625,19 +1526,16 @@ static void solve_dispatch(avbd_ctx* c, DevState<P>& s, const TetElems<RS>& el, 
                            const uint4* ranges = nullptr, unsigned nranges = 0) {
     if (el.star)
         solve_dispatch_form<P, RS, HT, LANES, FORM_STAR, MODE, DYN>(c, s, el, k, begin, count, st, out, T, list, ranges, nranges);
-    else if constexpr (LANES == 2 || LANES == 8) {
-        if (c->damping)
-            solve_dispatch_form<P, RS, HT, LANES, FORM_DAMP, MODE, DYN>(c, s, el, k, begin, count, st, out, T, list, ranges, nranges);
-        else
-            solve_dispatch_form<P, RS, HT, LANES, FORM_REC, MODE, DYN>(c, s, el, k, begin, count, st, out, T, list, ranges, nranges);
-    }
+    else if (c->damping)
+        solve_dispatch_form<P, RS, HT, LANES, FORM_DAMP, MODE, DYN>(c, s, el, k, begin, count, st, out, T, list, ranges, nranges);
+    else
+        solve_dispatch_form<P, RS, HT, LANES, FORM_REC, MODE, DYN>(c, s, el, k, begin, count, st, out, T, list, ranges, nranges);
 }
 
 // The solve, residual and features passes run with the context's lane count
 // (the residual pass spans every vertex every iteration, so its thread count
 // matters even when few scenes are candidates); the one-vertex debug pass
 // uses 8.
-// Lane counts: 2, 4, 8 and 16 with the star form, 2 and 8 with the records.
 template <typename P, typename RS, typename HT, int MODE>
 static void solve_lanes_t(avbd_ctx* c, DevState<P>& s, const TetElems<RS>& el, const StepConsts& k, unsigned begin,
                           unsigned count, cudaStream_t st, double* out, const SceneTol& T, const uint32_t* list,
@@ -1656,7 +1554,6 @@ static void solve_lanes_t(avbd_ctx* c, DevState<P>& s, const TetElems<RS>& el, c
             solve_dispatch<P, RS, HT, 8, MODE, true>(c, s, el, k, begin, count, st, out, T, list);
     } else {
         switch (c->lanes) {
-            case 1:  // one thread a vertex only in k_iterate
             case 2: solve_dispatch<P, RS, HT, 2, MODE>(c, s, el, k, begin, count, st, out, T, list, ranges, nranges); break;
             case 4: solve_dispatch<P, RS, HT, 4, MODE>(c, s, el, k, begin, count, st, out, T, list, ranges, nranges); break;
             case 16: solve_dispatch<P, RS, HT, 16, MODE>(c, s, el, k, begin, count, st, out, T, list, ranges, nranges); break;
@@ -1929,10 +1826,10 @@ static bool iterate_launch(avbd_ctx* c, DevState<P>& s, const TetElems<RS>& el, 
     const bool ground = !c->ground.empty(), tol = A.max_it != 0;
     auto kern = tol ? (ground ? k_iterate<P, RS, HT, LANES, FORM, true, true> : k_iterate<P, RS, HT, LANES, FORM, false, true>)
                     : (ground ? k_iterate<P, RS, HT, LANES, FORM, true, false> : k_iterate<P, RS, HT, LANES, FORM, false, false>);
-    constexpr bool STAR = FORM == FORM_STAR && LANES != 2;
-    if (STAR && !el.piece) return false;
+    constexpr bool PIPE = FORM == FORM_STAR && LANES > 2;
+    if (PIPE && !el.piece) return false;
     unsigned smem = FORM == FORM_STAR
-                        ? StarStage<P, LANES, THREADS>::bytes(STAR ? star_rows(el.max_nb, LANES) : el.max_nb)
+                        ? StarStage<P, LANES, THREADS>::bytes(PIPE ? star_rows(el.max_nb, LANES) : el.max_nb)
                         : 0;
     if (tol) smem += 2 * nblocks(A.S, 32) * (unsigned)sizeof(uint32_t);
     if (!stage_smem(kern, smem)) {
@@ -1941,7 +1838,7 @@ static bool iterate_launch(avbd_ctx* c, DevState<P>& s, const TetElems<RS>& el, 
     }
     // whether one block per SM is resident (the grid barrier needs all of
     // them), queried once per lane count and kind of step
-    int8_t& fits = c->iterate_fits[tol][LANES == 1 ? 4 : LANES == 2 ? 0 : LANES == 4 ? 1 : LANES == 8 ? 2 : 3];
+    int8_t& fits = c->iterate_fits[tol][LANES == 2 ? 0 : LANES == 4 ? 1 : 2];
     if (fits == 0) {
         int per_sm = 0, coop = 0;
         fits = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device) == cudaSuccess && coop &&
@@ -1974,11 +1871,10 @@ static bool iterate_t(avbd_ctx* c, DevState<P>& s, const TetElems<RS>& el, const
                       const IterArgs& A) {
     if (el.star) {
         switch (c->lanes) {
-            case 1: return iterate_launch<P, RS, P, 1, FORM_STAR>(c, s, el, k, st, A);
             case 2: return iterate_launch<P, RS, HT, 2, FORM_STAR>(c, s, el, k, st, A);
             case 4: return iterate_launch<P, RS, P, 4, FORM_STAR>(c, s, el, k, st, A);
-            case 16: return iterate_launch<P, RS, P, 16, FORM_STAR>(c, s, el, k, st, A);
-            default: return iterate_launch<P, RS, P, 8, FORM_STAR>(c, s, el, k, st, A);
+            case 8: return iterate_launch<P, RS, P, 8, FORM_STAR>(c, s, el, k, st, A);
+            default: return false;  // not laid out for k_iterate
         }
     }
     if (c->damping)

@@ -197,3 +197,49 @@ def test_contexts_of_different_valence_on_two_threads(monkeypatch, whole):
     for e, X in zip(both, alone):
         assert np.array_equal(e.positions(), X)
         e.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "fp32"])
+@pytest.mark.parametrize("lanes", [2, 4, 8, 16])
+@pytest.mark.parametrize("whole", [1, 0])
+def test_record_lane_counts(oracle_lib, monkeypatch, whole, lanes, precision):
+    """Damped tets (records) with each lane count of the launches per color; the
+    iteration launch takes 2 or 8."""
+    monkeypatch.setenv("AVBD_PERSISTENT", str(whole))
+    monkeypatch.setenv("AVBD_LANES", str(lanes))
+    sc = scenes.Scene(name="damped", dt=1.0 / 60.0, solver_iters=7)
+    scenes.add_tet_cube(sc, 5, E=1e5, nu=0.45, density=1000.0, fix_bottom=True, kd=5.0)
+    e, o = _pair(oracle_lib, sc, precision)
+    e.step(6)
+    o.step(6)
+    assert np.abs(e.positions() - o.positions()).max() / sc.bbox_diagonal() <= TOL[precision]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "fp32"])
+def test_lane_choice_of_large_colors_with_many_neighbours(precision):
+    """21,600 vertices a color (their lane count is timed), hubs of 21
+    neighbours: whatever is chosen, the iterations stay one launch, and every
+    scene does what it does alone (other lane counts: other sums)."""
+    k, copies = 20, 2400
+    one = fan(k)
+    (_, (X, m), _), (_, (T, lam, mu, kd, Q, V), _), (_, (held, flags), _) = one.calls
+    many = scenes.Scene(name="fans", dt=one.dt, solver_iters=one.solver_iters)
+    for s in range(copies):
+        if s:
+            many.record("begin_scene")
+        many.record("add_particles", X, m)
+        many.record("add_neo_hookean", T + s * len(X), lam, mu, kd, Q, V)
+        many.record("set_fixed", np.asarray(held) + s * len(X), flags)
+    e = Context()
+    many.load(e, precision=precision)
+    e.finalize()
+    before = e.stats()["kernel_launches"]
+    e.step(1)
+    assert e.stats()["kernel_launches"] - before <= 4
+    e.step(2)
+    a = Context()
+    one.load(a, precision=precision)
+    a.finalize()
+    a.step(3)
+    P, A = e.positions().reshape(copies, len(X), 3), a.positions()
+    assert np.abs(P - A).max() / one.bbox_diagonal() <= TOL[precision]
