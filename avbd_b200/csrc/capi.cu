@@ -1658,7 +1658,7 @@ int step_impl(avbd_ctx* c, DevState<R>& s, unsigned n_steps) {
 }  // namespace
 
 static int autotune(avbd_ctx* c) {
-    c->color_launches = colors_fill_launches(c);
+    c->color_lists = c->star_nb != 0 && colors_fill_launches(c);
     return use64(c) ? autotune_impl<double>(c, c->d) : autotune_impl<float>(c, c->f);
 }
 

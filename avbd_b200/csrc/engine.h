@@ -341,7 +341,7 @@ struct avbd_ctx {
     // iterations of tetrahedral contexts in one cooperative launch with grid
     // barriers (default; AVBD_PERSISTENT=0 turns it off)
     bool persistent = true;
-    bool color_launches = false;  // colors_fill_launches at finalize, for which the lanes were chosen
+    bool color_lists = false;     // star form finalized for launches per color: not laid out for k_iterate
     uint4* d_slabs = nullptr;           // per color: first internal vertex, solved positional vertices, first piece
     std::vector<uint2> star_off;        // host copy of TetElems::star, during finalize
     std::vector<void*> piece_alloc;     // the laid-out lists (TetElems::piece ...), replaced by each lane choice

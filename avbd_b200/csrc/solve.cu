@@ -879,9 +879,14 @@ AVBD_D bool iterate_barrier(unsigned* sync, unsigned number, int* err) {
 // Threads of an iteration block (one per SM): the prefetching sweeps of the
 // star form with a double state take 168 registers (with 128 they spilled and
 // a batch of 24 scenes ran 10.3 instead of 7.3 ms a pass), the others 128.
+// FP32 records at 2 lanes, which large colors take, stream better at twice the
+// warps, 64 registers and some 100 bytes of spill (to 1e-4 241,611 vertices a
+// color 57.9 with 512 threads and 51.9 ms a step, 481,124 106.9 and 91.8); MIXED
+// ones did not (24 scenes 11.5 ms, 15.6 with 768 threads).
 template <typename P, int FORM, int LANES = 8>
 struct IterThreads {
-    static constexpr int value = FORM == FORM_STAR && sizeof(P) == 8 && LANES > 2 ? 384 : 512;
+    static constexpr int value = FORM == FORM_STAR && sizeof(P) == 8 && LANES > 2 ? 384
+                                 : FORM != FORM_STAR && sizeof(P) == 4 && LANES == 2 ? 1024 : 512;
 };
 
 // A piece of 32 / LANES vertices of the star form whose constant data are on
@@ -1892,18 +1897,29 @@ static bool iterate(avbd_ctx* c, DevState<double>& s, const StepConsts& k, cudaS
 }
 
 // k_iterate's 12 to 16 warps an SM save launches and passes over small colors;
-// k_solve_tet's 24 stream large ones better.  Per step, this launch against
-// launches per color: to 1e-4, MIXED, 84,000 vertices a color 11.2 and 21.7 ms,
-// 175,000 24.2 and 29.0, 326,000 45.5 and 39.0, 1,230,000 165 and 125; FP64,
-// 175,000 38.1 and 33.7.  Fixed iterations: MIXED 654,000 10.1 and 10.5, FP32
-// 175,000 equal, FP64 175,000 4.17 and 3.66.
+// k_solve_tet's 24 and more stream large ones better.  ms a step, this launch
+// against launches per color, by the vertices of the largest color:
+// Star form, to 1e-4, MIXED: 84,000 11.2 and 21.7, 175,000 24.2 and 29.0,
+// 326,000 45.5 and 39.0, 1,230,000 165 and 125; FP64: 175,000 38.1 and 33.7;
+// FP32: 481,000 46.2 and 49.6, 754,000 68.4 and 73.3.  Fixed iterations: MIXED
+// 654,000 10.1 and 10.5, FP32 175,000 equal, FP64 175,000 4.17 and 3.66.
+// Records, fixed iterations, FP32: 1,459 0.341 and 0.353, 3,907 0.387 and 0.383,
+// 8,985 0.531 and 0.499, 17,231 0.852 and 0.721, 120,691 4.75 and 3.66; random
+// points MIXED: 4,436 1.77 and 1.74, 17,744 3.17 and 2.86, 41,228 5.72 and 3.48;
+// FP64: 4,436 1.69 and 1.79, 44,360 7.54 and 7.27 (grids 30,523 2.19 and 2.25,
+// 241,611 14.7 and 14.0).  Records to tolerance, where a launch per color also
+// pays for the decisions: MIXED 481,124 143 and 158, FP64 241,611 103 and 119,
+// FP32 481,124 92 and 111.
 bool colors_fill_launches(const avbd_ctx* c) {
+    const bool tol = c->solver.residual_tolerance > 0;
+    if (c->star_nb == 0) return !tol && c->max_color_solve >= (c->solver.precision == AVBD_PRECISION_FP32 ? 4000u : 10000u);
     if (c->solver.precision == AVBD_PRECISION_FP64) return c->max_color_solve >= 130000;
-    return c->solver.residual_tolerance > 0 && c->max_color_solve >= 250000;
+    return tol && c->solver.precision == AVBD_PRECISION_MIXED && c->max_color_solve >= 250000;
 }
 
 bool whole_iterations(const avbd_ctx* c) {
-    return c->persistent && !c->color_launches && !c->dyn && c->num_sms != 0 && c->max_color_solve != 0;
+    return c->persistent && !c->color_lists && !colors_fill_launches(c) && !c->dyn && c->num_sms != 0 &&
+           c->max_color_solve != 0;
 }
 
 template <typename R>

@@ -243,3 +243,29 @@ def test_lane_choice_of_large_colors_with_many_neighbours(precision):
     a.step(3)
     P, A = e.positions().reshape(copies, len(X), 3), a.positions()
     assert np.abs(P - A).max() / one.bbox_diagonal() <= TOL[precision]
+
+
+def test_route_of_large_record_contexts_follows_the_solver():
+    """Damped FP32 colors of some 4,900 vertices: launches per color for a fixed
+    number of iterations, the iteration launch to a tolerance, also when the
+    solver is set after finalize."""
+    sc = scenes.Scene(name="damped", dt=1.0 / 60.0, solver_iters=6)
+    scenes.add_tet_cube(sc, 26, E=1e5, nu=0.45, density=1000.0, fix_bottom=True, kd=5.0)
+    e = Context()
+    sc.load(e, precision="fp32")
+    e.finalize()
+    colors = e.stats()["num_colors"]
+
+    def launches():
+        before = e.stats()["kernel_launches"]
+        e.step(1)
+        e.synchronize()
+        return e.stats()["kernel_launches"] - before
+
+    fixed = launches()
+    assert fixed >= 6 * colors
+    e.set_solver(6, sc.iter_acceleration, 1e-12, 32, "fp32")  # not reached: 32 iterations
+    assert launches() < 32
+    e.set_solver(6, sc.iter_acceleration, 0.0, 0, "fp32")
+    assert launches() == fixed
+    assert np.isfinite(e.positions()).all()
