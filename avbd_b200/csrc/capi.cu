@@ -1347,13 +1347,22 @@ int autotune_impl(avbd_ctx* c, DevState<R>& s) {
         return whole ? layout_pieces<R>(c, s, st) : AVBD_OK;
     }
     using V4 = typename Vec4Of<R>::T;
-    V4* snap = nullptr;
-    CUDA_OR_FAIL(cudaMalloc(&snap, sizeof(V4) * s.n));
+    struct Trial {  // released on every way out
+        V4* snap = nullptr;
+        cudaEvent_t a = nullptr, b = nullptr;
+        ~Trial() {
+            if (a) cudaEventDestroy(a);
+            if (b) cudaEventDestroy(b);
+            cudaFree(snap);
+        }
+    } trial;
+    CUDA_OR_FAIL(cudaMalloc(&trial.snap, sizeof(V4) * s.n));
+    CUDA_OR_FAIL(cudaEventCreate(&trial.a));
+    CUDA_OR_FAIL(cudaEventCreate(&trial.b));
+    V4* const snap = trial.snap;
+    const cudaEvent_t a = trial.a, b = trial.b;
     CUDA_OR_FAIL(cudaMemcpyAsync(snap, s.x, sizeof(V4) * s.n, cudaMemcpyDeviceToDevice, st));
     StepConsts k = consts(c);
-    cudaEvent_t a, b;
-    CUDA_OR_FAIL(cudaEventCreate(&a));
-    CUDA_OR_FAIL(cudaEventCreate(&b));
     const unsigned long long launches0 = c->stats.kernel_launches;
     const unsigned sweeps = solved < 50000 ? 16 : 2;
     int best = 8;
@@ -1398,9 +1407,6 @@ int autotune_impl(avbd_ctx* c, DevState<R>& s) {
     }
     CUDA_OR_FAIL(cudaMemsetAsync(c->d_counters, 0, sizeof(unsigned long long), st));
     CUDA_OR_FAIL(cudaStreamSynchronize(st));
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-    cudaFree(snap);
     if (c->lanes != best) {
         c->lanes = best;
         if (whole)

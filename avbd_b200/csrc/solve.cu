@@ -1762,8 +1762,11 @@ __global__ void k_layout_pieces(TetElems<RS> el, const uint4* slabs, unsigned nc
 
 template <typename R, typename RS>
 static int layout_pieces_t(avbd_ctx* c, TetElems<RS>& el, cudaStream_t st) {
-    for (void* p : c->piece_alloc) cudaFree(p);
-    c->piece_alloc.clear();
+    auto release = [c] {
+        for (void* p : c->piece_alloc) cudaFree(p);
+        c->piece_alloc.clear();
+    };
+    release();
     el.piece = nullptr;
     const unsigned lanes = (unsigned)c->lanes;
     if (!el.star || lanes == 2 || c->star_off.empty()) return AVBD_OK;
@@ -1797,7 +1800,9 @@ static int layout_pieces_t(avbd_ctx* c, TetElems<RS>& el, cudaStream_t st) {
     };
     if (!al(&dp, sizeof(uint4) * piece.size()) || !al(&dn, sizeof(StarNb<RS>) * nn) ||
         !al(&dt, sizeof(StarTet<RS>) * nt) || !al(&dl, sizeof(uint32_t) * nt)) {
-        return set_error(AVBD_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(cudaGetLastError()));
+        release();  // no room for a second copy of the lists: not laid out either
+        cudaGetLastError();
+        return AVBD_OK;
     }
     cudaMemcpyAsync(dp, piece.data(), sizeof(uint4) * piece.size(), cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(c->d_slabs, slabs.data(), sizeof(uint4) * slabs.size(), cudaMemcpyHostToDevice, st);

@@ -123,3 +123,34 @@ def test_barrier_wait_gives_up_with_a_status():
     again = m.forward(feat).cpu().numpy()
     assert np.array_equal(again, ref)
     m.close()
+
+
+def test_finalize_without_room_for_the_streamed_lists(monkeypatch):
+    """The iteration launch streams a second copy of the element lists.  With no
+    device memory left for it, finalize succeeds and the step takes launches
+    per color, with the same results (other lane counts: other sums)."""
+    torch = pytest.importorskip("torch")
+    sc = scenes.batched_cubes(num_scenes=48, seed=2, n_min=16, n_max=18)
+    X = []
+    ballast = None
+    try:
+        for persistent in (0, 1):
+            monkeypatch.setenv("AVBD_PERSISTENT", str(persistent))
+            torch.cuda.synchronize()
+            free = torch.cuda.mem_get_info()[0]
+            if persistent:  # what the context took without the second copy, and a quarter of that copy
+                ballast = torch.empty(free - used - 32 * 2 ** 20, dtype=torch.uint8, device="cuda")
+            e = Context()
+            sc.load(e, precision="mixed")
+            e.finalize()
+            before = e.stats()["kernel_launches"]
+            e.step(1)
+            e.synchronize()
+            assert e.stats()["kernel_launches"] - before > 20
+            X.append(e.positions())
+            used = free - torch.cuda.mem_get_info()[0]
+            e.close()
+    finally:
+        del ballast
+        torch.cuda.empty_cache()
+    assert np.abs(X[0] - X[1]).max() / sc.bbox_diagonal() <= 1e-6
