@@ -1949,9 +1949,18 @@ int profile_step_impl(avbd_ctx* c, DevState<R>& s, double* solve_ms, double* sol
     std::vector<uint8_t> act(S);
     std::vector<unsigned> sb = c->scene_begin;
     if (sb.back() != s.n) sb.push_back(s.n);
-    // Chebyshev and ground duals of one vertex, inside the whole-iteration launch
+    // what the whole-iteration launch moves beyond the sweep's bytes, by scene.  In
+    // the streamed star form the acceleration and the duals follow a vertex's
+    // solve: its history read, the history and the second position written (duals
+    // are written only where they change).  Else a pass of their own over every
+    // vertex.
     const double V4B = sizeof(typename Vec4Of<R>::T);
-    const double cheb_b = 4 * V4B + 6 + (c->ground.empty() ? 0.0 : 5 * V4B + 2);
+    const bool fused = c->star_nb != 0 && c->lanes > 2;
+    const double accel_b = fused ? 3 * V4B : 4 * V4B + 6 + (c->ground.empty() ? 0.0 : 5 * V4B + 2);
+    std::vector<double> accel(S, 0.0);
+    for (unsigned sc = 0; sc < S; sc++)
+        for (unsigned e = sb[sc]; e < sb[sc + 1]; e++)
+            if (!fused || !c->fixed[e]) accel[sc] += accel_b;
     IterLaunch L;
     L.n = 1;
     L.tol = tol;
@@ -1982,7 +1991,7 @@ int profile_step_impl(avbd_ctx* c, DevState<R>& s, double* solve_ms, double* sol
         if (whole) {
             nl++;
             for (unsigned sc = 0; sc < S; sc++)
-                if (act[sc]) bytes += cheb_b * (sb[sc + 1] - sb[sc]);
+                if (act[sc]) bytes += accel[sc];
         } else {
             for (unsigned col = 0; col < nc; col++) {
                 cudaEventRecord(ev[2 * col], st);

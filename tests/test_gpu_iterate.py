@@ -75,3 +75,20 @@ def test_barrier_timeout_is_reported(monkeypatch, precision, tol, lanes, graph):
     e.synchronize()
     assert np.isfinite(e.positions()).all()
     e.close()
+
+
+def test_profiled_bytes_of_the_fused_iteration():
+    """Beyond the sweep an iteration of the streamed star form moves a history
+    read, a history write and a second position (32 bytes each in MIXED) per
+    solved vertex; fixed ones have none, ground duals change in place."""
+    sc = scenes.Scene(name="cube", dt=1.0 / 60.0, solver_iters=5)
+    scenes.add_tet_cube(sc, 6, fix_bottom=True, ground=True)
+    e = Context()
+    sc.load(e, precision="mixed", residual_tolerance=1e-12, max_iters=1)
+    e.finalize()
+    sweep = e.profile_solve(1)[1]
+    _, step, launches, iterations = e.profile_step()
+    assert (launches, iterations) == (1, 1)
+    solved = 7 ** 3 - 7 ** 2
+    assert step - sweep == pytest.approx(3 * 32 * solved)
+    e.close()
