@@ -1475,7 +1475,8 @@ int build_tol_graph(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaStream
     cudaError_t e = cudaStreamBeginCaptureToGraph(st, g, nullptr, nullptr, 0, mode);
     if (e != cudaSuccess) return abandon("graph capture: ", e);
     enqueue_begin<R>(c, s, k, st);  // no host step without dynamic contacts: cannot fail
-    launch_tol_init(c, st);  // also the iteration index and its weight
+    launch_tol_init(c, st);
+    launch_iter_set(c, st);
     cudaStreamCaptureStatus cs;
     const cudaGraphNode_t* deps = nullptr;
     size_t ndeps = 0;

@@ -269,24 +269,3 @@ def test_route_of_large_record_contexts_follows_the_solver():
     e.set_solver(6, sc.iter_acceleration, 0.0, 0, "fp32")
     assert launches() == fixed
     assert np.isfinite(e.positions()).all()
-
-
-def test_graph_and_host_loop_to_tolerance_launch_the_same(monkeypatch):
-    """A step to tolerance launches the same kernels from its graph as from the
-    host-driven loop."""
-    sc = scenes.batched_cubes(num_scenes=3, seed=4, n_min=3, n_max=4)
-    counts, iterations = [], []
-    for graph in (1, 0):
-        monkeypatch.setenv("AVBD_GRAPH", str(graph))
-        e = Context()
-        sc.load(e, precision="fp64", residual_tolerance=1e-4, max_iters=100)
-        e.finalize()
-        e.step(1)
-        before = e.stats()["kernel_launches"]
-        e.step(2)
-        e.synchronize()
-        counts.append(e.stats()["kernel_launches"] - before)
-        iterations.append(e.scene_iterations().tolist())
-        e.close()
-    assert iterations[0] == iterations[1]
-    assert counts[0] == counts[1]
