@@ -1887,10 +1887,11 @@ static bool iterate_t(avbd_ctx* c, DevState<P>& s, const TetElems<RS>& el, const
             default: return false;  // not laid out for k_iterate
         }
     }
+    // 2 or 8 lanes, the nearer of the context's (launches per color have 4 and 16 too)
     if (c->damping)
-        return c->lanes == 2 ? iterate_launch<P, RS, HT, 2, FORM_DAMP>(c, s, el, k, st, A)
+        return c->lanes <= 4 ? iterate_launch<P, RS, HT, 2, FORM_DAMP>(c, s, el, k, st, A)
                              : iterate_launch<P, RS, HT, 8, FORM_DAMP>(c, s, el, k, st, A);
-    return c->lanes == 2 ? iterate_launch<P, RS, HT, 2, FORM_REC>(c, s, el, k, st, A)
+    return c->lanes <= 4 ? iterate_launch<P, RS, HT, 2, FORM_REC>(c, s, el, k, st, A)
                          : iterate_launch<P, RS, HT, 8, FORM_REC>(c, s, el, k, st, A);
 }
 static bool iterate(avbd_ctx* c, DevState<float>& s, const StepConsts& k, cudaStream_t st, const IterArgs& A) {
