@@ -438,7 +438,8 @@ void launch_solve_color(avbd_ctx* c, DevState<R>& s, const StepConsts& k, unsign
 // iteration cap max_it, in a graph's while loop when `loop` is given (the
 // first iteration is then d_tol_it's).  False, having launched nothing, when
 // the context does not qualify: oriented particles, dynamic contacts,
-// AVBD_PERSISTENT=0, no cooperative launches.
+// AVBD_PERSISTENT=0, colors that launches fill, lists that are not laid out, no
+// cooperative launches.
 struct IterLaunch {
     unsigned it0 = 0, n = 0;
     double tol = 0;
@@ -456,7 +457,8 @@ constexpr unsigned TOL_ITERS_PER_LAUNCH = 32;
 template <typename R>
 bool launch_iterate(avbd_ctx* c, DevState<R>& s, const StepConsts& k, cudaStream_t st, const IterLaunch& L);
 // lays the star form out for k_iterate at c->lanes threads a vertex (nothing
-// to do without the star form or at 2 lanes)
+// to do without the star form or at 2 lanes; where the lists do not fit the
+// device they are not laid out)
 template <typename R>
 int layout_pieces(avbd_ctx* c, DevState<R>& s, cudaStream_t st);
 // poll limit of k_iterate's grid barriers (avbd_debug_set_wait_limit)
