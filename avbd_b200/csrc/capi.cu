@@ -1570,6 +1570,7 @@ int step_impl(avbd_ctx* c, DevState<R>& s, unsigned n_steps) {
         SceneTol resT{c->d_scene, nullptr, c->d_scene_cand, nullptr, c->d_scene_ex};
         int gr = AVBD_OK;
         if (capturable && !c->graph) {
+            CUDA_OR_FAIL(cudaGetLastError());  // an earlier call's error is not the recording's
             gr = build_tol_graph<R>(c, s, k, st, max_it, tol, solveT, resT);
             if (gr != AVBD_OK && c->persistent) {
                 // a graph that cannot hold the cooperative launch: the
